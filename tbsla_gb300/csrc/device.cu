@@ -141,7 +141,8 @@ struct DeviceMatrix {
                     (void*)bcoef})
       if (p) cudaFree(p);
     for (SellPlan& p : sell)
-      for (void* q : {(void*)p.slice, (void*)p.lane, (void*)p.lane_len})
+      for (void* q : {(void*)p.slice, (void*)p.lane, (void*)p.lane_len, (void*)p.piece_cut, (void*)p.piece_at,
+                      (void*)p.cut_first, (void*)p.piece_sum, (void*)p.cut_done, (void*)p.cut_terms})
         if (q) cudaFree(q);
     for (cudaEvent_t e : xready)
       if (e) cudaEventDestroy(e);
@@ -355,11 +356,20 @@ int build_sell(const tbsla_matrix* m, DeviceMatrix* d) {
     SellPlan& dp = d->sell[k];
     dp = hp;
     dp.slice = nullptr;
-    dp.lane = nullptr;
-    dp.lane_len = nullptr;
+    dp.lane = dp.lane_len = dp.piece_cut = dp.piece_at = dp.cut_first = nullptr;
     st = upload_array(d, &dp.slice, hp.slice, (size_t)hp.nslices);
     if (!st) st = upload_array(d, &dp.lane, hp.lane, 32 * (size_t)hp.nslices);
     if (!st) st = upload_array(d, &dp.lane_len, hp.lane_len, 32 * (size_t)hp.nwide);
+    if (!st && hp.ncut > 0) {
+      st = upload_array(d, &dp.piece_cut, hp.piece_cut, (size_t)hp.npieces);
+      if (!st) st = upload_array(d, &dp.piece_at, hp.piece_at, (size_t)hp.npieces);
+      if (!st) st = upload_array(d, &dp.cut_first, hp.cut_first, (size_t)hp.ncut + 1);
+      if (!st) st = dalloc(&dp.piece_sum, (size_t)hp.npieces);
+      if (!st) st = dalloc(&dp.cut_done, (size_t)hp.ncut);
+      if (!st) st = dalloc(&dp.cut_terms, 3 * (size_t)hp.ncut);
+      if (!st) st = status_of(cudaMemsetAsync(dp.cut_done, 0, (size_t)hp.ncut * sizeof(unsigned), d->stream));
+      d->bytes += (size_t)hp.npieces * 8 + (size_t)hp.ncut * 28;
+    }
     if (!st) st = status_of(cudaStreamSynchronize(d->stream));  // host plan arrays are freed next
     sell_plan_free(&hp);
     steps += dp.sell_len / 32;

@@ -108,9 +108,11 @@ __device__ __forceinline__ int next_block(Ctl ctl, Smem& sm) {
 }
 
 // Per-CTA partials, then the last CTA to finish sums them in CTA order
-// (deterministic), calls epi.finalize(result) and resets the counters.
+// (deterministic), then the `nextra` groups of NRED terms left in `extra` by
+// any CTA before this call, calls fin(result) and resets the counters.
 template <int NRED, class Fin>
-__device__ __forceinline__ void reduce_and_finish(Ctl ctl, double* red, Smem& sm, Fin fin) {
+__device__ __forceinline__ void reduce_and_finish(Ctl ctl, double* red, Smem& sm, Fin fin,
+                                                  const double* extra = nullptr, int nextra = 0) {
   for (int k = 0; k < NRED; k++) {
     double v = block_sum<NT>(red[k], sm.red);
     if (threadIdx.x == 0) ctl.partials[(size_t)blockIdx.x * NRED + k] = v;
@@ -128,6 +130,7 @@ __device__ __forceinline__ void reduce_and_finish(Ctl ctl, double* red, Smem& sm
     double acc = 0;
     for (int i = threadIdx.x; i < (int)gridDim.x; i += NT)
       acc = add_rn(acc, __ldcg(ctl.partials + (size_t)i * NRED + k));
+    for (int i = threadIdx.x; i < nextra; i += NT) acc = add_rn(acc, __ldcg(extra + (size_t)i * NRED + k));
     acc = block_sum<NT>(acc, sm.red);
     if (threadIdx.x == 0) ctl.result[k] = acc;
   }

@@ -66,9 +66,12 @@ cudaError_t csr_merge_spmv_noalloc(const double* vals, const int* rowptr, const 
 // most short_thr entries take one lane each and are sorted by length within
 // windows of `sigma` consecutive rows; longer rows take the fewest lanes (up
 // to 32) that keep their slice at most long_thr steps wide and are sorted by
-// length over the whole block.  One warp per slice, fetched dynamically,
-// widest slices first; lanes past their row's end issue no loads, so
-// padding costs no traffic.
+// length over the whole block.  A row that 32 lanes cannot hold in long_thr
+// steps is cut into pieces of at most 32 * long_thr consecutive entries, a
+// slice each; the warp that finishes a row's last piece adds the pieces'
+// sums in piece order.  One warp per slice, fetched dynamically, widest
+// slices first; lanes past their row's end issue no loads, so padding costs
+// no traffic.
 //
 // The columns are split into blocks small enough for their part of x to
 // stay in L2 while the block runs (x beyond ~60 MB misses L2 for most
@@ -82,8 +85,21 @@ struct SellPlan {
   long sell_len = 0;           // elements of the block's slices
   int4* slice = nullptr;       // [nslices]: {step offset, width in steps, g, base}
   int* lane = nullptr;         // [32 * nslices]: base >= 0: (row - base) << 8 | len;
-                               // base = -1: row; -1 for an unused lane
-  int* lane_len = nullptr;     // [32 * nwide]: the row's entries in the block
+                               // base < 0: row; -1 for an unused lane
+  int* lane_len = nullptr;     // [32 * nwide]: the row's entries in the block (base = -1)
+                               // or in the piece (base = -2 - piece)
+  // rows cut into pieces: piece k belongs to cut row piece_cut[k], whose
+  // pieces are cut_first[c] .. cut_first[c + 1) in entry order
+  int npieces = 0, ncut = 0;
+  int* piece_cut = nullptr;    // [npieces]: index of the cut row
+  int* piece_at = nullptr;     // [npieces]: the row's entries in the block before the piece
+  int* cut_first = nullptr;    // [ncut + 1]
+  // device scratch of a launch: the pieces' sums, the pieces finished per cut
+  // row (zeroed once; the warp that adds a row up resets its count), and the
+  // PageRank terms of the cut rows (3 per row)
+  double* piece_sum = nullptr;
+  unsigned* cut_done = nullptr;
+  double* cut_terms = nullptr;
   int row_lo = 0, row_hi = 0;  // rows the plan may hold (a part of the last block: its rows)
 };
 // Parts by rows of the last column block (when there are several blocks).

@@ -19,6 +19,14 @@
 // consecutive words (256-byte coalesced loads) and no work item takes much
 // longer than another: one warp per slice, fetched dynamically, widest first.
 //
+// A row too long for 32 lanes in long_thr steps is cut into pieces, a slice
+// each, because a hub row on one warp was the critical path of the whole
+// launch: PageRank on a 2^22-node graph whose longest row holds 89,090 entries
+// went from 37.4 to 12.5 ms (36 steps), an SpMV of 10^6 power-law rows of up
+// to 7,400 entries (FP32 values) from 103.6 to 92.5 us.  long_thr is where
+// the cut lies because a slice of that width is the widest item the other
+// rows make, so a piece never takes longer than they do.
+//
 // Each lane sums its entries in entry order with fused multiply-adds; G > 1
 // lanes of a row are combined by a fixed butterfly of additions.
 #include <algorithm>
@@ -130,8 +138,8 @@ struct Lane {
 
 // Decodes lane `lane` of slice k with descriptor d = {step offset, width, g,
 // base}: a window slice (base >= 0) packs (row - base) << 8 | length per
-// lane; a slice sorted over the whole block (base = -1) holds the row, with
-// its length in lane_len.
+// lane; a slice sorted over the whole block (base < 0) holds the row, with
+// its length (of the piece, base < -1) in lane_len.
 __device__ __forceinline__ Lane slice_lane(const SellPlan& p, const int4& d, int meta, long k, int lane) {
   Lane l{-1, 0, 0};
   if (meta < 0) return l;
@@ -172,6 +180,29 @@ struct Claims {
     return it;
   }
 };
+
+// A finished piece of a cut row (its sum on every lane).  The warp whose
+// piece completes the row gets true and the row's sum in acc: lane l adds
+// pieces l, l + 32, ... in that order, then the fixed butterfly, so the sum
+// does not depend on which warp was last.  Lane 0 publishes its piece before
+// it counts itself in (the fence), and the last warp reads after the count.
+__device__ __forceinline__ bool cut_row_done(const SellPlan& p, int piece, int lane, double& acc) {
+  const int c = __ldg(p.piece_cut + piece);
+  const int first = __ldg(p.cut_first + c), n = __ldg(p.cut_first + c + 1) - first;
+  int last = 0;
+  if (lane == 0) {
+    __stcg(p.piece_sum + piece, acc);
+    __threadfence();
+    last = atomicAdd(p.cut_done + c, 1u) == (unsigned)n - 1;
+  }
+  if (!__shfl_sync(FULL, last, 0)) return false;
+  __threadfence();
+  double t = 0;
+  for (int k = lane; k < n; k += 32) t = add_rn(t, __ldcg(p.piece_sum + first + k));
+  acc = warp_sum(t);
+  if (lane == 0) p.cut_done[c] = 0;  // for the next launch
+  return true;
+}
 
 // One column block: y = A_block x (block 0) or y += A_block x (later blocks,
 // whose plans leave out the rows without entries in the block).
@@ -237,10 +268,25 @@ __global__ void __launch_bounds__(NT) k_sell(SellPlan p, const V* __restrict__ s
       mn = __ldg(p.lane + (long)nxt * 32 + lane);
     }
     const Lane l = slice_lane(p, d, meta, cur, lane);
-    const bool head = l.row >= 0 && (lane & ((1 << d.z) - 1)) == 0;
+    bool head = l.row >= 0 && (lane & ((1 << d.z) - 1)) == 0;
     const double y0 = (!PR && accumulate && head) ? y[l.row] : 0.0;  // issued before the sum
     double acc = slice_rows<V, U>(sv, sc, (long)d.x * 32 + lane, l.steps, d.y, x, f_col, pol);
     for (int o = (1 << d.z) >> 1; o > 0; o >>= 1) acc = add_rn(acc, __shfl_xor_sync(FULL, acc, o));
+    if (d.w < -1) {  // a piece of a cut row
+      const int piece = -2 - d.w;
+      head = cut_row_done(p, piece, lane, acc) && lane == 0;
+      if constexpr (PR) {
+        // any warp may be the last one: the row's terms go to slots of their
+        // own, which the last CTA adds in cut-row order
+        if (head) {
+          double terms[3] = {0, 0, 0};
+          epi.emit(l.row, acc, terms);
+          double* t = p.cut_terms + 3 * (size_t)__ldg(p.piece_cut + piece);
+          for (int k = 0; k < 3; k++) t[k] = terms[k];
+        }
+        head = false;
+      }
+    }
     if constexpr (PR) {
       if (head) epi.emit(l.row, acc, red);
       cur = nxt;
@@ -256,7 +302,7 @@ __global__ void __launch_bounds__(NT) k_sell(SellPlan p, const V* __restrict__ s
   }
   if constexpr (PR) {
     __shared__ csr::Smem sm;
-    csr::reduce_and_finish<3>(ctl, red, sm, csr::PageRankFinish::of(pr));
+    csr::reduce_and_finish<3>(ctl, red, sm, csr::PageRankFinish::of(pr), p.cut_terms, p.ncut);
     return;
   }
   // The last warp to finish resets the work counters for the next launch:
@@ -288,14 +334,14 @@ __global__ void __launch_bounds__(NT) k_sell_fill(SellPlan p, const V* __restric
     const int s = l.row >= 0 ? rowptr[l.row] : 0;
     const int e = l.row >= 0 ? rowptr[l.row + 1] : 0;
     const int span = __reduce_max_sync(FULL, e - s);
-    int placed = 0;  // entries of this lane's row placed so far
-    for (int base = 0; base < span; base += G) {
+    int placed = d.w < -1 ? -p.piece_at[-2 - d.w] : 0;  // entries of this lane's row placed so far
+    for (int base = 0; base < span && (d.w >= -1 || placed < l.len); base += G) {
       const int j = s + base + sub;
       const int col = j < e ? colidx[j] - f_col : -1;
       const bool in = col >= p.col_lo && col < p.col_hi;
       const unsigned m = (__ballot_sync(FULL, in) >> group) & (G == 32 ? FULL : (1u << G) - 1);
-      if (in) {
-        const int q = placed + __popc(m & ((1u << sub) - 1));
+      const int q = placed + __popc(m & ((1u << sub) - 1));
+      if (in && q >= 0 && q < l.len) {
         const long o = off + (long)(q >> d.z) * 32 + group + (q & (G - 1));
         sv[o] = vals[j];
         sc[o] = colidx[j];
@@ -426,19 +472,37 @@ void sell_plan_build(const int* L, int n, int sthr, int lthr, int sigma, bool sk
   struct Slice {
     int width, g;
     long first;  // index into wide_rows of its first row
+    int piece;   // of a cut row (-1: whole rows)
   };
   std::vector<int4> desc;
   std::vector<int> meta, meta_len;
   std::vector<std::pair<int, int>> order;  // (width, slice) of the wide slices
   std::vector<Slice> wide;
   std::vector<int> wide_rows;
+  std::vector<int> piece_cut, piece_at, piece_len, cut_first;
   auto by_len = [&](int a, int b) { return len(a) > len(b); };
   for (int g = 0; g <= 5; g++) {
     auto& v = lng[g];
     std::stable_sort(v.begin(), v.end(), by_len);
     const int per = 32 >> g;
-    for (size_t q = 0; q < v.size(); q += per) {
-      Slice s{(len(v[q]) + (1 << g) - 1) >> g, g, (long)wide_rows.size()};
+    // a row past 32 * long_thr entries: equal pieces, whole steps each
+    size_t q0 = 0;
+    for (; g == 5 && q0 < v.size() && (len(v[q0]) + 31) >> 5 > lthr; q0++) {
+      const int l = len(v[q0]), steps = (l + 31) >> 5, np = (steps + lthr - 1) / lthr;
+      const int size = 32 * ((steps + np - 1) / np);
+      cut_first.push_back((int)piece_at.size());
+      for (int at = 0; at < l; at += size) {
+        Slice s{(std::min(size, l - at) + 31) >> 5, 5, (long)wide_rows.size(), (int)piece_at.size()};
+        piece_cut.push_back((int)cut_first.size() - 1);
+        piece_at.push_back(at);
+        piece_len.push_back(std::min(size, l - at));
+        wide_rows.push_back(v[q0]);
+        order.push_back({s.width, (int)wide.size()});
+        wide.push_back(s);
+      }
+    }
+    for (size_t q = q0; q < v.size(); q += per) {
+      Slice s{(len(v[q]) + (1 << g) - 1) >> g, g, (long)wide_rows.size(), -1};
       for (int r = 0; r < per; r++) wide_rows.push_back(q + r < v.size() ? v[q + r] : -1);
       order.push_back({s.width, (int)wide.size()});
       wide.push_back(s);
@@ -448,11 +512,11 @@ void sell_plan_build(const int* L, int n, int sthr, int lthr, int sigma, bool sk
   long off = step0;  // in steps of 32 entries
   for (auto& o : order) {
     const Slice& s = wide[o.second];
-    desc.push_back(make_int4((int)off, s.width, s.g, -1));
+    desc.push_back(make_int4((int)off, s.width, s.g, s.piece >= 0 ? -2 - s.piece : -1));
     for (int l = 0; l < 32; l++) {
       const int row = wide_rows[s.first + (l >> s.g)];
       meta.push_back(row);
-      meta_len.push_back(row >= 0 ? len(row) : 0);
+      meta_len.push_back(s.piece >= 0 ? piece_len[s.piece] : row >= 0 ? len(row) : 0);
     }
     off += s.width;
   }
@@ -506,12 +570,24 @@ void sell_plan_build(const int* L, int n, int sthr, int lthr, int sigma, bool sk
   std::copy(meta.begin(), meta.end(), p->lane);
   p->lane_len = new int[std::max<size_t>(meta_len.size(), 1)];
   std::copy(meta_len.begin(), meta_len.end(), p->lane_len);
+  p->npieces = (int)piece_at.size();
+  p->ncut = (int)cut_first.size();
+  cut_first.push_back(p->npieces);
+  p->piece_cut = new int[std::max<size_t>(piece_cut.size(), 1)];
+  std::copy(piece_cut.begin(), piece_cut.end(), p->piece_cut);
+  p->piece_at = new int[std::max<size_t>(piece_at.size(), 1)];
+  std::copy(piece_at.begin(), piece_at.end(), p->piece_at);
+  p->cut_first = new int[cut_first.size()];
+  std::copy(cut_first.begin(), cut_first.end(), p->cut_first);
 }
 
 void sell_plan_free(SellPlan* p) {
   delete[] p->slice;
   delete[] p->lane;
   delete[] p->lane_len;
+  delete[] p->piece_cut;
+  delete[] p->piece_at;
+  delete[] p->cut_first;
   *p = SellPlan{};
 }
 
