@@ -114,6 +114,8 @@ struct DeviceMatrix {
   // double-float column sums (n), coefficients and flags, kept between solves
   double *bx0 = nullptr, *bx1 = nullptr, *btele = nullptr, *bw = nullptr, *bcoef = nullptr;
   size_t bx0_len = 0, bx1_len = 0, btele_len = 0, bw_len = 0, bcoef_len = 0;
+  BatchPlan bplan;        // its work items, built at the first batched solve
+  int bplan_budget = 0;
   double* x = nullptr;
   size_t x_len = 0;
   double* y = nullptr;
@@ -138,7 +140,9 @@ struct DeviceMatrix {
                     (void*)counter, (void*)partials, (void*)result, (void*)coord, (void*)carry_row,
                     (void*)carry_val, svals, (void*)scols, (void*)sell_counter, (void*)colw, (void*)xdf,
                     (void*)df_flag, (void*)coo_carry, (void*)bx0, (void*)bx1, (void*)btele, (void*)bw,
-                    (void*)bcoef})
+                    (void*)bcoef, (void*)bplan.item, (void*)bplan.piece_cut, (void*)bplan.cut_first,
+                    (void*)bplan.piece_sum,
+                    (void*)bplan.cut_done})
       if (p) cudaFree(p);
     for (SellPlan& p : sell)
       for (void* q : {(void*)p.slice, (void*)p.lane, (void*)p.lane_len, (void*)p.piece_cut, (void*)p.piece_at,
@@ -1114,6 +1118,41 @@ int dev_page_rank(tbsla_matrix* m, double beta, double eps, int max_it, double* 
   return hflags[0] ? TBSLA_OK : TBSLA_ERR_NOT_CONVERGED;
 }
 
+namespace {
+// The work items of the batched step for a grid of `grid` CTAs, kept with the
+// device copy until another grid wants another item size.
+int batch_plan(const tbsla_matrix* m, DeviceMatrix* d, int grid) {
+  const int n = m->info.n_row;
+  const int* rp = m->idx0.data();
+  const int budget = batch_plan_budget((long)rp[n] - rp[0], n, 8 * grid);
+  if (d->bplan.item && d->bplan_budget == budget) return TBSLA_OK;
+  std::vector<int4> items;
+  std::vector<int> cut, first;
+  batch_plan_build(rp, n, budget, &items, &cut, &first);
+  BatchPlan& b = d->bplan;
+  TRY(cudaStreamSynchronize(d->stream));
+  for (void* q : {(void*)b.item, (void*)b.piece_cut, (void*)b.cut_first, (void*)b.piece_sum, (void*)b.cut_done})
+    if (q) cudaFree(q);
+  b = BatchPlan{};
+  int st = upload_array(d, &b.item, items.data(), items.size());
+  if (!st) st = upload_array(d, &b.piece_cut, cut.data(), cut.size());
+  if (!st) st = upload_array(d, &b.cut_first, first.data(), first.size());
+  if (!st) st = dalloc(&b.piece_sum, 32 * cut.size());
+  if (!st) st = dalloc(&b.cut_done, first.size());
+  if (!st) st = status_of(cudaMemsetAsync(b.cut_done, 0, first.size() * sizeof(unsigned), d->stream));
+  if (!st) st = status_of(cudaStreamSynchronize(d->stream));
+  if (st) {  // no plan: the next call builds it again
+    if (b.item) cudaFree(b.item);
+    b.item = nullptr;
+    return st;
+  }
+  b.nitems = (int)items.size();
+  b.npieces = (int)cut.size();
+  d->bplan_budget = budget;
+  return TBSLA_OK;
+}
+}  // namespace
+
 int dev_page_rank_batched(tbsla_matrix* m, int nvec, const double* tele, double beta, double eps,
                           int max_it, double* result, int* iterations) {
   if (m->format != TBSLA_CSR) return TBSLA_ERR_UNSUPPORTED;
@@ -1132,14 +1171,15 @@ int dev_page_rank_batched(tbsla_matrix* m, int nvec, const double* tele, double 
   // FP32 pipe; FP64 values keep FP64 arithmetic
   const bool df = d->prec != TBSLA_F64;
   const int gather = m->pr_gather == 16 ? 16 : 8;
-  // the row-block stream form keeps X row offsets in 32 bits
-  const int stream = m->pr_stream && (long)I.n_col * nvec <= 0x7fffffffL ? 1 : 0;
+  // the entry-stream form; in double-float it keeps X row offsets in 32 bits
+  const int stream = !df || (m->pr_stream && (long)I.n_col * nvec <= 0x7fffffffL) ? 1 : 0;
   int grid = csr_pagerank_batched_grid(d->prec, gather, stream);
   // the buffers stay with the device copy: repeated solves allocate (and
   // synchronise on frees) nothing
   if ((st = d->vec(&d->bx0, &d->bx0_len, nn)) || (st = d->vec(&d->bx1, &d->bx1_len, nn)) ||
       (st = d->vec(&d->btele, &d->btele_len, nn)) || (st = d->vec(&d->bcoef, &d->bcoef_len, 130)) ||
-      (st = d->ctl(96, grid)) || (st = column_weights(m, d)) || (df && (st = d->vec(&d->bw, &d->bw_len, (size_t)n))))
+      (st = d->ctl(96, grid)) || (st = column_weights(m, d)) || (df && (st = d->vec(&d->bw, &d->bw_len, (size_t)n))) ||
+      (stream && (st = batch_plan(m, d, grid))))
     return st;
   double *X0 = d->bx0, *X1 = d->bx1, *T = d->btele, *coef = d->bcoef, *W = d->bw;
   int* flags = reinterpret_cast<int*>(d->bcoef + 128);
@@ -1168,9 +1208,8 @@ int dev_page_rank_batched(tbsla_matrix* m, int nvec, const double* tele, double 
       const bool even = (launched % 2) == 0;
       p.coef_in = coef + (even ? 0 : 64);
       p.coef_out = coef + (even ? 64 : 0);
-      cudaError_t e = df ? csr_pagerank_batched_df_step(a, nvec, even ? X0 : X1, even ? X1 : X0, T, W, p, ctl, grid,
-                                                        gather, stream, s)
-                         : csr_pagerank_batched_step(a, n, nvec, even ? X0 : X1, even ? X1 : X0, T, p, ctl, grid, s);
+      const cudaError_t e = csr_pagerank_batched_step(a, d->bplan, nvec, even ? X0 : X1, even ? X1 : X0, T,
+                                                      df ? W : d->colw, p, ctl, grid, gather, stream, s);
       if (e != cudaSuccess) return status_of(e);
     }
     if (cudaMemcpyAsync(hflags, flags, 2 * sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess ||

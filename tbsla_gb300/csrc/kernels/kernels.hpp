@@ -5,6 +5,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <vector>
+
 namespace tbsla_gpu {
 
 enum Prec { kF64 = 0, kF32 = 1, kBF16 = 2 };
@@ -177,29 +179,48 @@ cudaError_t csr_pagerank_step(const CsrArgs& a, const double* x, double* y,
 // to 8 CTAs per SM.  cudaErrorInvalidValue for a plan of several blocks.
 cudaError_t sell_pagerank(const SellArgs& a, const double* x, double* y, const PageRankArgs& p, Ctl ctl,
                           cudaStream_t s);
+// Work items of the batched step's entry-stream form, of about `budget`
+// entries (a row counts 4 more): runs of rows {r0, r1, first entry, end}.  A
+// row of more entries than that is cut into pieces; the pieces are items
+// [0, npieces) (so they are claimed first), piece k belongs to cut row
+// piece_cut[k], whose pieces are cut_first[c] .. cut_first[c + 1) in entry
+// order.  piece_sum: 32 FP64 sums per piece; cut_done: a zeroed
+// count per cut row, reset by each launch.
+struct BatchPlan {
+  int nitems = 0, npieces = 0;
+  int4* item = nullptr;
+  int* piece_cut = nullptr;
+  int* cut_first = nullptr;
+  double* piece_sum = nullptr;
+  unsigned* cut_done = nullptr;
+};
+// Entries per item: six items for each of the grid's warps, so that the last
+// wave is a small part of the step, at least 64 (below that the start of an
+// item, three dependent loads, is most of it) and at most 1024.  32 vectors,
+// FP32 values, us a step with items of 64 / 256 / 512 / 1024 / 2048 entries:
+// 1,220 / 911 / 796 / 785 / 791 at 2^20 nodes (14.8 M entries), 66 / 65 / 96 /
+// 141 / 241 at 20,000; this rule: 780 and 66.
+int batch_plan_budget(long nnz, int n, int warps);
+void batch_plan_build(const int* rowptr, int n, int budget, std::vector<int4>* items, std::vector<int>* piece_cut,
+                      std::vector<int>* cut_first);
 // Batched personalised PageRank step: X, Y, T are n x nvec row-major
 // (nvec <= 32); column k as above with s_k = coef_in[k], t_k =
 // coef_in[32 + k] and c_i = t_k * T[i, k].  Reductions per column k:
 // result[k] = L1 change, result[nvec + k] = S', result[2 nvec + k] = M';
 // the last CTA writes coef_out[k], coef_out[32 + k] and sets *done when
-// every column's change is < eps.
-// The same in double-float (pairs of floats h + l, about 46 bits) for FP32 /
-// BF16 values: X, Y, T (n x nvec) and W (the column sums, n) are float2
-// arrays of the same byte size as FP64 ones; reductions are FP64.  gather:
-// X-row gathers in flight per warp (8 or 16); stream: 0 a warp per row (the
-// CTA's warps take a block's rows in turn), 1 a warp per row block, its
-// entries walked as one stream across row boundaries.
-cudaError_t csr_pagerank_batched_df_step(const CsrArgs& a, int nvec, const void* X, void* Y, const void* T,
-                                         const void* W, const PageRankArgs& p, Ctl ctl, int grid, int gather,
-                                         int stream, cudaStream_t s);
+// every column's change is < eps.  FP64 values: X, Y, T and W (the column
+// sums, n) are FP64 and the entry-stream form runs.  FP32 / BF16 values:
+// they are float2 arrays of the same byte size in double-float (pairs of
+// floats h + l, about 46 bits); reductions are FP64.  gather: X-row gathers
+// in flight per warp (8 or 16); stream: 0 a warp per row (the CTA's warps
+// take a block's rows in turn), 1 the entry-stream form.
+cudaError_t csr_pagerank_batched_step(const CsrArgs& a, const BatchPlan& plan, int nvec, const void* X, void* Y,
+                                      const void* T, const void* W, const PageRankArgs& p, Ctl ctl, int grid,
+                                      int gather, int stream, cudaStream_t s);
 // FP64 <-> double-float (float2) conversions, element by element (the
 // destination may be the source's own storage).
 cudaError_t f64_to_df(const double* src, void* dst, long n, cudaStream_t s);
 cudaError_t df_to_f64(const void* src, double* dst, long n, cudaStream_t s);
-cudaError_t csr_pagerank_batched_step(const CsrArgs& a, int n_row, int nvec, const double* X,
-                                      double* Y, const double* T, const PageRankArgs& p,
-                                      Ctl ctl, int grid, cudaStream_t s);
-
 // PageRank step after a separate SpMV t = A x (the sliced-ELL path): the
 // same y, reductions and coefficients as csr_pagerank_step, over n rows, in
 // `grid` CTAs (ctl sized for grid x 3 partials).

@@ -78,3 +78,36 @@ def test_pagerank_with_hub_rows(gpu, prec):
     v = a["values"] if prec == "f64" else a["values"].astype(np.float32).astype(np.float64)
     xr, _, _ = oracle.pagerank(a["rowptr"], a["colidx"], v, 0.85, 1e-10, out[0][1], stop_early=False)
     assert np.abs(out[0][0] - xr).sum() <= 1e-10
+
+
+@pytest.mark.parametrize("prec,nvec", [("f64", 1), ("f64", 32), ("f32", 32), ("bf16", 5)])
+def test_batched_pagerank_with_hub_rows(gpu, prec, nvec):
+    """The entry-stream form with rows around and past an item's length (64
+    entries at this size) and hub rows of many pieces, empty rows before,
+    between and after: each vector within 1e-10 in L1 of the oracle, and the
+    double-float forms within 1e-13 of the warp-per-row form."""
+    T = gpu
+    n = 6000
+    m, lens = ragged(T, n, [60, 63, 64, 65, 127, 128, 129, 3000, 20_000, 0, 0, 0], 11)
+    a = m.arrays()
+    m = T.MatrixCSR.from_arrays(n, n, a["rowptr"], a["colidx"], np.ones(len(a["values"])))
+    m.make_stochastic(np.zeros(n))
+    m.set_precision({"f64": T.F64, "f32": T.F32, "bf16": T.BF16}[prec])
+    rng = np.random.default_rng(12)
+    tele = np.zeros((n, nvec))
+    for k in range(nvec):
+        tele[rng.choice(n, 30, replace=False), k] = 1.0 / 30
+    X, it, ok = m.page_rank_batched(tele, 0.85, 1e-10, 500)
+    Y, it2, _ = m.page_rank_batched(tele, 0.85, 1e-10, 500)
+    assert ok and it == it2 and np.abs(X - Y).sum(axis=0).max() <= 1e-13
+    if prec != "f64":
+        m.set_pagerank_stream(False)
+        Z, it3, _ = m.page_rank_batched(tele, 0.85, 1e-10, 500)
+        assert it3 == it and np.abs(X - Z).sum(axis=0).max() <= 1e-13
+    a = m.arrays()
+    v = a["values"]
+    v = v.astype(np.float32).astype(np.float64) if prec == "f32" else oracle.bf16_round(v) if prec == "bf16" else v
+    for k in {0, nvec // 2, nvec - 1}:
+        xr, _, _ = oracle.pagerank(a["rowptr"], a["colidx"], v, 0.85, 1e-10, it, stop_early=False,
+                                   teleport=np.ascontiguousarray(tele[:, k]))
+        assert np.abs(X[:, k] - xr).sum() <= 1e-10, k
