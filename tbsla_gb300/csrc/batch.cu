@@ -289,7 +289,7 @@ int build_dia(tbsla_batch* B, const std::vector<int>& delta, int K) {
   CK(alloc(&B->fallback_d, nsys));
   CK(alloc(&B->relres_d, nsys));
   CK(alloc(&B->acc, (size_t)12 * nsys));
-  CK(alloc(&B->bar, 4));
+  CK(alloc(&B->bar, 64 + kClaimWords));
   B->vec4 = B->prec != TBSLA_F64;
   for (int s = 0; s <= nsys; s++) B->vec4 = B->vec4 && B->off[s] % 4 == 0;
   B->adelta_h = delta;
@@ -520,6 +520,15 @@ int dia_solve(tbsla_batch* B, const double* rhs, double* x, int max_iterations, 
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, B->device);
     grid = std::min(grid, B->ctas_per_sm * sms);
   }
+  // no more CTAs than the batch has warp units to hand out, a unit per warp:
+  // every further CTA only arrives at the barriers.  With that, one atomic
+  // per CTA in the sums and the shorter barrier, one system takes, us an
+  // iteration: 16^3 12.0 -> 9.0, 48^3 15.8 -> 9.6, 64^3 20.1 -> 10.5, 96^3
+  // 31.1 -> 17.5 (A kept in L2 too).
+  long units = 0;
+  const long urows = vec4 ? 128 : 32;
+  for (int k = 0; k < ns; k++) units += (B->off[k + 1] - B->off[k] + urows - 1) / urows;
+  grid = (int)std::max<long>(1, std::min<long>(grid, (units + 7) / 8));
   DiaCg c;
   std::memset(&c, 0, sizeof c);  // padding too: the struct is the graph's cache key
   c.nsys = ns;
@@ -552,12 +561,21 @@ int dia_solve(tbsla_batch* B, const double* rhs, double* x, int max_iterations, 
   c.relres = B->relres_d;
   c.acc = B->acc;
   c.bar = B->bar;
+  c.claims = B->bar + 64;
   c.tol2 = rel_tol * rel_tol;
   c.max_it = max_iterations;
   c.refresh = B->prec != TBSLA_F64 ? refresh : 0;
   c.wait_ns = B->wait_ns;
   c.vec4 = vec4 ? 1 : 0;
   c.st7 = st7 ? 1 : 0;
+  {
+    // bytes per row of an iteration: A, and d, r and p of two parities, q, z,
+    // D^-1 (factored: L and t instead of z and D^-1); 64 MiB is about what
+    // GB300's 129 MB L2 keeps of data read by every SM
+    const long ev = B->prec == TBSLA_F64 ? 8 : 4, ea = B->prec == TBSLA_F64 ? 8 : B->prec == TBSLA_F32 ? 4 : 2;
+    const long row = B->K * ea + 7 * ev + (precond == 2 ? B->KL * (lprec == TBSLA_BF16 ? 2 : 4) : 4);
+    c.keep_rows = (64L << 20) / row;
+  }
   std::vector<int> mode(ns, precond);
   CK(cudaMemcpyAsync(B->b, rhs, n * 8, cudaMemcpyHostToDevice, s));
   CK(cudaMemcpyAsync(B->x, x, n * 8, cudaMemcpyHostToDevice, s));
@@ -570,11 +588,11 @@ int dia_solve(tbsla_batch* B, const double* rhs, double* x, int max_iterations, 
     if (precond == 1) e = dia_dinv(B->a64_dia, B->row_sys, B->adelta, B->K, n, B->dinv_f, st);
     if (e == cudaSuccess) e = cudaMemsetAsync(B->dv, 0, (size_t)n * es, st);
     if (e == cudaSuccess) e = cudaMemsetAsync(B->acc, 0, (size_t)12 * ns * 8, st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(B->bar, 0, 4 * sizeof(unsigned), st);
+    if (e == cudaSuccess) e = cudaMemsetAsync(B->bar, 0, (64 + kClaimWords) * sizeof(unsigned), st);
     if (e == cudaSuccess) e = cg_dia_solve(c, grid, st);
     return e;
   };
-  if (!B->pgraph || std::memcmp(&B->pkey, &c, sizeof c) != 0 || B->pkey_pre != precond) {
+  if (!B->pgraph || std::memcmp(&B->pkey, &c, sizeof c) != 0 || B->pkey_pre != precond || B->pgrid != grid) {
     if (B->pgraph) cudaGraphExecDestroy(B->pgraph);
     B->pgraph = nullptr;
     cudaGraph_t g = nullptr;
@@ -593,6 +611,7 @@ int dia_solve(tbsla_batch* B, const double* rhs, double* x, int max_iterations, 
     }
     B->pkey = c;
     B->pkey_pre = precond;
+    B->pgrid = grid;
   }
   if (B->pgraph) CK(cudaGraphLaunch(B->pgraph, s));
   else CK(enqueue(s));

@@ -99,32 +99,39 @@ __device__ __forceinline__ unsigned long long global_ns() {
   return t;
 }
 
-// Grid-wide barrier with a bounded wait.  bar[0] arrival count, bar[1]
-// generation, bar[2] error word.  Returns false when the grid must stop.
+// Grid-wide barrier with a bounded wait.  bar[0] counts arrivals and is never
+// reset (barrier number `gen` is over when it reaches gen * gridDim.x, compared
+// as a difference, so it may wrap), bar[2] is the error word.  One atomic in
+// release order and one polled word, because every L2 round trip of a barrier
+// is about 0.45 us of a small system's iteration (count, reset, generation,
+// error word and fences took five).  Returns false when the grid must stop: a
+// wait that ran out sets the error word and returns, the others find it in
+// their own next wait, which cannot end without that CTA.
 __device__ bool grid_sync(unsigned* bar, unsigned& gen, long long wait_ns, int* s_stop) {
   __syncthreads();
   if (threadIdx.x == 0) {
-    const unsigned target = gen + 1;
-    __threadfence();
-    const unsigned arrived = atomicAdd(&bar[0], 1u);
-    if (arrived == gridDim.x - 1) {
-      atomicExch(&bar[0], 0u);
-      __threadfence();
-      atomicExch(&bar[1], target);
-    } else {
+    gen++;
+    const unsigned target = gen * gridDim.x;
+    unsigned seen;
+    asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(seen) : "l"(bar) : "memory");
+    seen++;
+    int stop = 0;
+    if ((int)(seen - target) < 0) {
       const unsigned long long t0 = global_ns();
-      while (ld_acquire(&bar[1]) != target) {
-        if (ld_acquire(&bar[2]) != 0u) break;
-        if ((long long)(global_ns() - t0) > wait_ns) {
-          atomicExch(&bar[2], 1u);
+      for (int spin = 1; (int)(ld_acquire(bar) - target) < 0; spin++) {
+        if (spin % 32 != 0 && wait_ns > 0) continue;
+        if (ld_acquire(bar + 2) != 0u) {
+          stop = 1;
           break;
         }
-        __nanosleep(32);
+        if ((long long)(global_ns() - t0) > wait_ns) {
+          atomicExch(bar + 2, 1u);
+          stop = 1;
+          break;
+        }
       }
     }
-    gen = target;
-    __threadfence();
-    *s_stop = ld_acquire(&bar[2]) != 0u;
+    *s_stop = stop;
   }
   __syncthreads();
   return !*s_stop;
@@ -189,10 +196,18 @@ __device__ __forceinline__ float dot4(float4 a, float4 b, float acc) {
 }
 
 // Per-warp running sums of up to 3 values for one system at a time: lanes
-// add their rows' terms; when the warp moves to another system (or the phase
-// ends) the warp reduces them and lane 0 adds them to acc[what * ns + sys] in
-// FP64.  No CTA-wide barrier.  Every lane of the warp calls to() / flush()
-// at the same points (a unit belongs to one warp and one system).
+// add their rows' terms; when the warp moves to another system it leaves its
+// sums in the CTA's shared memory, and at the end of a phase the CTA adds one
+// FP64 atomic per system and value to acc[what * ns + sys] (one per warp
+// held up the end of every phase: 3,648 atomics on one address, times the
+// systems that the phase sweeps).  Every lane of the warp calls to() at the
+// same points (a unit belongs to one warp and one system).
+struct SumsSmem {
+  double v[3 * kDiaMaxSys];  // [what * ns + sys]; all zero between phases
+  int touched;               // some warp added to v in this phase
+  int sys[PNT / 32];         // the warps' last systems and their sums
+  double last[3][PNT / 32];
+};
 template <class T, int NV>
 struct WarpSums {
   int sys = -1;
@@ -201,27 +216,67 @@ struct WarpSums {
 #pragma unroll
     for (int k = 0; k < NV; k++) v[k] = (T)0;
   }
-  __device__ __forceinline__ void flush(double* acc, int ns) {
+  __device__ __forceinline__ void reduce() {
+#pragma unroll
+    for (int k = 0; k < NV; k++) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
+    }
+  }
+  __device__ __forceinline__ void to(int s, int ns, SumsSmem& sm) {
+    if (s == sys) return;
     if (sys >= 0) {
-#pragma unroll
-      for (int k = 0; k < NV; k++) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
-      }
+      reduce();
       if ((threadIdx.x & 31) == 0) {
+        sm.touched = 1;
 #pragma unroll
-        for (int k = 0; k < NV; k++) atomicAdd(acc + (size_t)k * ns + sys, (double)v[k]);
+        for (int k = 0; k < NV; k++) atomicAdd(&sm.v[k * ns + sys], (double)v[k]);
       }
 #pragma unroll
       for (int k = 0; k < NV; k++) v[k] = (T)0;
     }
-    sys = -1;
+    sys = s;
   }
-  __device__ __forceinline__ void to(int s, double* acc, int ns) {
-    if (s != sys) {
-      flush(acc, ns);
-      sys = s;
+  // the end of a phase, called by every thread of the CTA (grid_sync follows)
+  __device__ __forceinline__ void finish(double* acc, int ns, SumsSmem& sm) {
+    constexpr int NW = PNT / 32;
+    const int warp = threadIdx.x >> 5;
+    reduce();
+    if ((threadIdx.x & 31) == 0) {
+      sm.sys[warp] = sys;
+#pragma unroll
+      for (int k = 0; k < NV; k++) sm.last[k][warp] = (double)v[k];
     }
+    __syncthreads();
+    if (warp == 0) {
+      const int lane = threadIdx.x;
+      int mine = lane < NW ? sm.sys[lane] : -1;
+      const int any = __reduce_max_sync(0xffffffffu, mine);
+      if (__all_sync(0xffffffffu, mine == any || mine < 0)) {  // one system: a tree over the warps
+        if (any >= 0) {
+#pragma unroll
+          for (int k = 0; k < NV; k++) {
+            double t = mine >= 0 ? sm.last[k][lane] : 0.0;
+#pragma unroll
+            for (int o = NW / 2; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+            if (lane == 0) atomicAdd(acc + (size_t)k * ns + any, t);
+          }
+        }
+      } else if (mine >= 0) {
+#pragma unroll
+        for (int k = 0; k < NV; k++) atomicAdd(acc + (size_t)k * ns + mine, sm.last[k][lane]);
+      }
+    } else if (sm.touched) {
+      for (int t = threadIdx.x - 32; t < NV * ns; t += PNT - 32) {
+        const double x = sm.v[t];
+        if (x != 0) {
+          atomicAdd(acc + t, x);
+          sm.v[t] = 0;
+        }
+      }
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) sm.touched = 0;
   }
 };
 
@@ -233,17 +288,32 @@ struct WarpSums {
 // moment the whole grid works on one compact window of rows, so each
 // array is read as one front sweeping through memory (many streams at
 // scattered places ran at about 45% of the HBM bandwidth, against 98% for
-// the same loads swept grid-stride), and every warp gets an even share
-// whatever systems have finished.
+// the same loads swept in order).  A warp starts on the unit of its index and
+// claims further ones from a counter, one ahead of its work, because the SMs
+// do not run at one speed: with equal shares a CTA waited up to 40% of a phase
+// for the slowest.  8 systems of 96^3: Jacobi 129 -> 105 us an iteration,
+// factored 170 -> 135; 16 systems of 16^3 to 96^3: 46.7 -> 33.3.  Each warp of
+// a CTA has a counter of its own, in a separate 256-byte line, for the units
+// congruent to its index mod 8, so the claims do not queue up on one address.
 #define SELECT(cond)                        \
   select_sys([&](int s_) { return (cond); }); \
+  sel_active = false;                       \
+  const int nsel_ = s_nsel
+// The S_ACTIVE systems: kept from phase to phase and iteration to iteration
+// while no state changes.
+#define SELECT_ACTIVE()                                             \
+  if (!sel_active) {                                                \
+    select_sys([&](int s_) { return s_st[s_] == S_ACTIVE; });       \
+    sel_active = true;                                              \
+  }                                                                 \
   const int nsel_ = s_nsel
 // A warp keeps the system of its last unit and that system's range of
 // selected units [uk0_, uk1_): its next unit (a grid's worth of units on)
 // usually lies in the same system, and then needs no search.
 #define FOR_CHUNKS(ch)                                                                          \
-  for (int ku_ = blockIdx.x * (PNT / 32) + warp_, us_ = -1, uk0_ = 0, uk1_ = 0; ku_ < nsel_; \
-       ku_ += gridDim.x * (PNT / 32))                                                           \
+  for (int ku_ = blockIdx.x * (PNT / 32) + warp_, us_ = -1, uk0_ = 0, uk1_ = 0,               \
+           nx_ = claim(nsel_, ph);                                                              \
+       ku_ < nsel_; ku_ = __shfl_sync(0xffffffffu, nx_, 0), nx_ = claim(nsel_, ph))             \
     for (int ch_sys = (ku_ >= uk0_ && ku_ < uk1_)                                               \
                           ? us_                                                                 \
                           : (us_ = unit_sys(ku_), uk1_ = s_end[us_],                            \
@@ -269,6 +339,7 @@ __global__ void __launch_bounds__(PNT, 3) k_cg_persistent(DiaCg c) {
   __shared__ int s_su[kDiaMaxSys + 1];    // first warp unit of each system, then the unit count
   __shared__ int s_end[kDiaMaxSys];       // selected units of systems 0..s
   __shared__ int s_nsel;
+  __shared__ SumsSmem s_sums;
   __shared__ int s_ad[kDiaMaxSys * KMAX], s_ld[kDiaMaxSys * KMAX];
   const int ns = c.nsys;
   const int tid = threadIdx.x;
@@ -289,9 +360,9 @@ __global__ void __launch_bounds__(PNT, 3) k_cg_persistent(DiaCg c) {
   T* __restrict__ Z = static_cast<T*>(c.z);
   T* __restrict__ Tt = static_cast<T*>(c.t);
   const float* __restrict__ dinv = c.dinv;
-  const uint64_t pol = policy_evict_first();
-
   for (int s = tid; s <= ns; s += PNT) s_off[s] = c.sys_off[s];
+  for (int t = tid; t < 3 * ns; t += PNT) s_sums.v[t] = 0;
+  if (tid == 0) s_sums.touched = 0;
   for (int t = tid; t < ns * KMAX; t += PNT) {
     s_ad[t] = c.adelta[t];
     s_ld[t] = c.ldelta ? c.ldelta[t] : 0;
@@ -321,19 +392,43 @@ __global__ void __launch_bounds__(PNT, 3) k_cg_persistent(DiaCg c) {
   int g = 0;   // iteration parity of the R / P buffers
   bool init = true;
   auto slot = [&](int p) { return c.acc + (size_t)(p % 3) * 4 * ns; };
-  // CTA 0 clears the slot two phases ahead (read at the start of the
-  // previous phase by every CTA, written next in the following phase)
+  // CTA 0 clears the slot and the claim counters two phases ahead (read at
+  // the start of the previous phase by every CTA, written next in the
+  // following phase)
   auto clear_ahead = [&]() {
     if (blockIdx.x == 0) {
       double* a = slot(ph + 1);
       for (int t = tid; t < 4 * ns; t += PNT) a[t] = 0.0;
+      if (tid < PNT / 32) c.claims[((ph + 1) % 3 * (PNT / 32) + tid) * kClaimStride] = 0;
     }
   };
-  auto any_state = [&](int st, int mode) {
-    int f = 0;
-    for (int s = tid; s < ns; s += PNT) f |= s_st[s] == st && (mode < 0 || s_mode[s] == mode);
-    return __syncthreads_or(f) != 0;
+  // the unit after this warp's current one (lane 0 holds it), in the phase
+  // whose counters are those of ph; past the end when the first units are all
+  // there are
+  auto claim = [&](int nsel, int p) {
+    const int nw = gridDim.x * (PNT / 32);
+    int k = nsel;
+    if (nsel > nw && lane_ == 0)
+      k = nw + warp_ + (PNT / 32) * (int)atomicAdd(c.claims + (p % 3 * (PNT / 32) + warp_) * kClaimStride, 1u);
+    return k;
   };
+  // what the systems' states ask for, the same in every thread (each warp
+  // looks the states over itself: no barrier; called after one)
+  enum { ANY_CHECK = 1, ANY_RESTART = 2, ANY_ACTIVE = 4, LIVE_FACT = 8, ACTIVE_PLAIN = 16 };
+  auto states = [&]() {
+    unsigned f = 0;
+    for (int s = lane_; s < ns; s += 32) {
+      const int st = s_st[s];
+      const bool fact = s_mode[s] == 2;
+      f |= st == S_CHECK ? ANY_CHECK : st == S_RESTART_F ? ANY_RESTART : st == S_ACTIVE ? ANY_ACTIVE : 0;
+      // factored systems still iterating, or just stopped by phase B' (which
+      // leaves their d += alpha p to phase D)
+      if (fact && (st == S_ACTIVE || st == S_CHECK)) f |= LIVE_FACT;
+      if (!fact && st == S_ACTIVE) f |= ACTIVE_PLAIN;
+    }
+    return __reduce_or_sync(0xffffffffu, f);
+  };
+  bool sel_active = false;  // s_end / s_nsel hold the selection of the S_ACTIVE systems
   // s_end / s_nsel for the systems where pred(s) holds (warp 0: a scan over
   // the systems, up to 8 per lane)
   auto select_sys = [&](auto pred) {
@@ -378,7 +473,7 @@ __global__ void __launch_bounds__(PNT, 3) k_cg_persistent(DiaCg c) {
 
   for (;;) {
     // ================= refinement: systems in S_CHECK ======================
-    if (any_state(S_CHECK, -1)) {
+    if (states() & ANY_CHECK) {
       // R1: x += d (FP64), d = 0; at the start, check the factors
       clear_ahead();
       {
@@ -390,7 +485,7 @@ __global__ void __launch_bounds__(PNT, 3) k_cg_persistent(DiaCg c) {
           if (s_st[s] != S_CHECK) continue;
           const int r0 = ch_r0, r1 = ch_r1;
           const bool chk = init && s_mode[s] == 2;
-          if (chk) bad.to(s, acc, ns);
+          if (chk) bad.to(s, ns, s_sums);
           for (int i = r0 + lane_; i < r1; i += 32) {
             const double xi = c.x[i] + (double)D[i];
             if (isfinite(xi)) c.x[i] = xi;  // a non-finite correction is dropped
@@ -404,7 +499,7 @@ __global__ void __launch_bounds__(PNT, 3) k_cg_persistent(DiaCg c) {
             }
           }
         }
-        bad.flush(acc, ns);
+        bad.finish(acc, ns, s_sums);
       }
       if (!grid_sync(c.bar, gen, c.wait_ns, &s_stop)) return;
       {
@@ -425,13 +520,14 @@ __global__ void __launch_bounds__(PNT, 3) k_cg_persistent(DiaCg c) {
         double* acc = slot(ph);
         T* __restrict__ Rn = R(g);
         T* __restrict__ Po = P(g);
+        const uint64_t pol = policy_evict_first();
         WarpSums<double, 3> part;
         FOR_CHUNKS(ch) {
           const int s = ch_sys;
           if (s_st[s] != S_CHECK) continue;
-          part.to(s, acc, ns);
+          part.to(s, ns, s_sums);
           const int r0 = ch_r0, r1 = ch_r1;
-          const long lo = c.sys_off[s], hi = c.sys_off[s + 1];
+          const long lo = s_off[s], hi = s_off[s + 1];
           int dd[KMAX];
           load_deltas(c.adelta, s, c.K, dd);
           const bool ident = s_mode[s] == 0;
@@ -457,7 +553,7 @@ __global__ void __launch_bounds__(PNT, 3) k_cg_persistent(DiaCg c) {
             Po[i] = (T)0;
           }
         }
-        part.flush(acc, ns);
+        part.finish(acc, ns, s_sums);
       }
       if (!grid_sync(c.bar, gen, c.wait_ns, &s_stop)) return;
       {
@@ -498,7 +594,7 @@ __global__ void __launch_bounds__(PNT, 3) k_cg_persistent(DiaCg c) {
         init = false;
       }
       __syncthreads();
-      if (any_state(S_RESTART_F, -1)) {
+      if (states() & ANY_RESTART) {
         // R3: t = L^T r (T arithmetic), r.z = t.t
         clear_ahead();
         {
@@ -509,9 +605,9 @@ __global__ void __launch_bounds__(PNT, 3) k_cg_persistent(DiaCg c) {
           FOR_CHUNKS(ch) {
             const int s = ch_sys;
             if (s_st[s] != S_RESTART_F) continue;
-            part.to(s, acc, ns);
+            part.to(s, ns, s_sums);
             const int r0 = ch_r0, r1 = ch_r1;
-            const long hi = c.sys_off[s + 1];
+            const long hi = s_off[s + 1];
             int ld[KMAX];
             load_deltas(c.ldelta, s, c.KL, ld);
             for (int i = r0 + lane_; i < r1; i += 32) {
@@ -527,7 +623,7 @@ __global__ void __launch_bounds__(PNT, 3) k_cg_persistent(DiaCg c) {
               part.v[0] += t * t;
             }
           }
-          part.flush(acc, ns);
+          part.finish(acc, ns, s_sums);
         }
         if (!grid_sync(c.bar, gen, c.wait_ns, &s_stop)) return;
         {
@@ -556,7 +652,7 @@ __global__ void __launch_bounds__(PNT, 3) k_cg_persistent(DiaCg c) {
             const int s = ch_sys;
             if (s_st[s] != S_RESTART_F) continue;
             const int r0 = ch_r0, r1 = ch_r1;
-            const long lo = c.sys_off[s];
+            const long lo = s_off[s];
             int ld[KMAX];
             load_deltas(c.ldelta, s, c.KL, ld);
             for (int i = r0 + lane_; i < r1; i += 32) {
@@ -580,7 +676,7 @@ __global__ void __launch_bounds__(PNT, 3) k_cg_persistent(DiaCg c) {
         __syncthreads();
       }
     }
-    if (!any_state(S_ACTIVE, -1)) break;
+    if (!(states() & ANY_ACTIVE)) break;
 
     // ================= one iteration =======================================
     const T* __restrict__ Pold = P(g);
@@ -588,15 +684,18 @@ __global__ void __launch_bounds__(PNT, 3) k_cg_persistent(DiaCg c) {
     // A: q = A p, p.q
     clear_ahead();
     {
-      SELECT(s_st[s_] == S_ACTIVE);
+      SELECT_ACTIVE();
+      // A's values are read once per iteration: first out of L2, unless all
+      // that the running systems touch in an iteration stays there
+      const uint64_t pol = (long)nsel_ * urows <= c.keep_rows ? policy_evict_normal() : policy_evict_first();
       double* acc = slot(ph);
       WarpSums<T, 1> part;
       FOR_CHUNKS(ch) {
         const int s = ch_sys;
         if (s_st[s] != S_ACTIVE) continue;
-        part.to(s, acc, ns);
+        part.to(s, ns, s_sums);
         const int r0 = ch_r0, r1 = ch_r1;
-        const long lo = c.sys_off[s], hi = c.sys_off[s + 1];
+        const long lo = s_off[s], hi = s_off[s + 1];
         const bool fact = s_mode[s] == 2;
         int dd[KMAX];
         load_deltas(c.adelta, s, c.K, dd);
@@ -664,7 +763,7 @@ __global__ void __launch_bounds__(PNT, 3) k_cg_persistent(DiaCg c) {
           part.v[0] += pi * q;
         }
       }
-      part.flush(acc, ns);
+      part.finish(acc, ns, s_sums);
     }
     if (!grid_sync(c.bar, gen, c.wait_ns, &s_stop)) return;
     {
@@ -681,20 +780,20 @@ __global__ void __launch_bounds__(PNT, 3) k_cg_persistent(DiaCg c) {
     clear_ahead();
     {
       double* acc = slot(ph);
-      SELECT(s_st[s_] == S_ACTIVE);
+      SELECT_ACTIVE();
       const T* __restrict__ Ro = R(g);
       T* __restrict__ Rn = R(g + 1);
       WarpSums<T, 2> part;
       FOR_CHUNKS(ch) {
         const int s = ch_sys;
         if (s_st[s] != S_ACTIVE) continue;
-        part.to(s, acc, ns);
+        part.to(s, ns, s_sums);
         const int r0 = ch_r0, r1 = ch_r1;
         const T alpha = (T)s_alpha[s];
         const int mode = s_mode[s];
         if constexpr (sizeof(T) == 4) {
           if (c.vec4) {
-            const long lo = c.sys_off[s], hi = c.sys_off[s + 1];
+            const long lo = s_off[s], hi = s_off[s + 1];
             float* Df = reinterpret_cast<float*>(D);
             const float* Rof = reinterpret_cast<const float*>(Ro);
             const float* Qf = reinterpret_cast<const float*>(Q);
@@ -753,7 +852,7 @@ __global__ void __launch_bounds__(PNT, 3) k_cg_persistent(DiaCg c) {
           }
         }
         if (mode == 2) {
-          const long hi = c.sys_off[s + 1];
+          const long hi = s_off[s + 1];
           int ld[KMAX];
           load_deltas(c.ldelta, s, c.KL, ld);
           for (int i = r0 + lane_; i < r1; i += 32) {
@@ -784,7 +883,7 @@ __global__ void __launch_bounds__(PNT, 3) k_cg_persistent(DiaCg c) {
           }
         }
       }
-      part.flush(acc, ns);
+      part.finish(acc, ns, s_sums);
     }
     if (!grid_sync(c.bar, gen, c.wait_ns, &s_stop)) return;
     {
@@ -808,26 +907,28 @@ __global__ void __launch_bounds__(PNT, 3) k_cg_persistent(DiaCg c) {
       ph++;
     }
     __syncthreads();
-    // factored systems still iterating, or just stopped by phase B' (which
-    // leaves their d += alpha p to this phase)
-    int fact_ = 0;
-    for (int s = tid; s < ns; s += PNT) fact_ |= s_mode[s] == 2 && (s_st[s] == S_ACTIVE || s_st[s] == S_CHECK);
-    if (__syncthreads_or(fact_)) {
+    const unsigned after = states();
+    if (after & ANY_CHECK) sel_active = false;
+    if (after & LIVE_FACT) {
       // D: d += alpha p; z = L t, p = z + beta p (iterating systems)
       clear_ahead();
-      SELECT(s_mode[s_] == 2 && (s_st[s_] == S_ACTIVE || s_st[s_] == S_CHECK));
+      if (!sel_active || (after & ACTIVE_PLAIN)) {
+        select_sys([&](int s_) { return s_mode[s_] == 2 && (s_st[s_] == S_ACTIVE || s_st[s_] == S_CHECK); });
+        sel_active = false;
+      }
+      const int nsel_ = s_nsel;
       FOR_CHUNKS(ch) {
         const int s = ch_sys;
         const bool act = s_st[s] == S_ACTIVE;
         const int r0 = ch_r0, r1 = ch_r1;
-        const long lo = c.sys_off[s];
+        const long lo = s_off[s];
         const T alpha = (T)s_alpha[s];
         const T beta = (T)s_beta[s];
         int ld[KMAX];
         load_deltas(c.ldelta, s, c.KL, ld);
         if constexpr (sizeof(T) == 4) {
           if (c.vec4) {
-            const long hi = c.sys_off[s + 1];
+            const long hi = s_off[s + 1];
             const float* Tf = reinterpret_cast<const float*>(Tt);
             float* Df = reinterpret_cast<float*>(D);
             for (long i0 = r0 + 4 * lane_; i0 < r1; i0 += 128) {
@@ -889,6 +990,7 @@ __global__ void __launch_bounds__(PNT, 3) k_cg_persistent(DiaCg c) {
   }
 }
 #undef FOR_CHUNKS
+#undef SELECT_ACTIVE
 #undef SELECT
 
 // ---- layout builders ----------------------------------------------------------

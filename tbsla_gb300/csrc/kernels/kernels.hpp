@@ -277,6 +277,8 @@ struct CgBatch {
 // ---- persistent batched CG on diagonal-structured systems (cg_dia.cu) ----------
 constexpr int kDiaMaxDiag = 8;   // diagonals per system (A and L)
 constexpr int kDiaMaxSys = 256;  // systems per batch
+constexpr int kClaimStride = 64;  // words between claim counters (256 bytes)
+constexpr int kClaimWords = 3 * 8 * kClaimStride;  // three phases x a CTA's eight warps
 enum DiaFallback { kFallbackNone = 0, kFallbackBadFactor = 1, kFallbackStagnation = 2 };
 struct DiaCg {
   int nsys;
@@ -300,7 +302,8 @@ struct DiaCg {
   int* fallback;          // [nsys] out: DiaFallback
   double* relres;         // [nsys] out: FP64 true relative residual at exit
   double* acc;            // [3][4][nsys] rotating accumulator slots (zeroed before launch)
-  unsigned* bar;          // [4] grid barrier: count, generation, error (zeroed before launch)
+  unsigned* bar;          // [4] grid barrier: arrivals, unused, error (zeroed before launch)
+  unsigned* claims;       // [kClaimWords] work claims of three phases (zeroed before launch)
   double tol2;
   int max_it;
   int refresh;            // iterations per refinement cycle (narrow storage), 0 = never
@@ -308,6 +311,7 @@ struct DiaCg {
                           // the hot phases take 4 rows per thread with 16-byte loads
   int st7;                // with vec4: every system in the seven-point form (dia_seven_point)
   long long wait_ns;      // bound on one grid-wide wait
+  long keep_rows;         // rows whose iteration stays in L2 (A is then not read evict-first)
 };
 // Co-resident CTAs of the persistent kernel for (prec, lprec, seven-point
 // form) on this device.
