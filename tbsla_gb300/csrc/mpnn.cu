@@ -15,12 +15,19 @@
 //   training loss over Gaussian probes Z (n x P): sum (L L^T A Z - Z)^2 / (nP)
 //
 // GPU mapping: one warp per node with the 32 features on the 32 lanes, so
-// every gather of a neighbour's features is one 128-byte load and every
-// dense layer is 64 shuffles + 64 FMAs per lane against weights in shared
-// memory.  Forward and backward are hand-written kernels in FP32 with the
-// weights rounded to bfloat16 (FP32 master copy in the Adam state);
+// every gather of a neighbour's features is one 128-byte load.  The graph of a
+// system (scaled edge weights, the patterns of L and L^T) is built on the
+// device from the CSR arrays of each call.  Forward and backward are
+// hand-written kernels in FP32 with the weights rounded to bfloat16 (FP32
+// master copy in the Adam state); in the dense layers a lane keeps its
+// output's 64 weights (and, backward, its 64 weight gradients) in registers
+// and the activations of four nodes are read from shared memory by broadcast,
+// so a node costs its 64 (backward 128) multiply-adds and little else;
 // parameter gradients are reduced per CTA in shared memory, then added to
 // global memory once per CTA.
+// 48^3 nodes, 8 probes, loss and gradient from the host arrays: 5.17 -> 0.79 ms
+// (the host's graph 3.9 ms of it, a layer backward 268 -> 35 us, forward 57 ->
+// 28 us without its gather).
 #include <cuda_runtime.h>
 #include <cuda_bf16.h>
 
@@ -35,6 +42,7 @@
 #include "device.hpp"
 #include "host/matrix.hpp"
 #include "kernels/common.cuh"
+#include "kernels/kernels.hpp"
 #include "tbsla_gb300.h"
 
 namespace {
@@ -52,92 +60,121 @@ constexpr unsigned FULL = 0xffffffffu;
 
 __host__ __device__ inline int off_layer(int l) { return OFF_L + (l - 1) * LSZ; }  // l = 1..NL
 
-// ---- host: one system's graph --------------------------------------------------------
+// ---- device kernels: one system's graph ------------------------------------------------
+// L: per row its strictly lower entries (in A's order), then the diagonal;
+// L^T: per column j the L entries of that column, in row order.
 
-struct HostGraph {
-  int n = 0;
-  std::vector<int> rowptr, colidx;
-  std::vector<float> aval, e, s, x;
-  // L: per row its strictly lower entries (in A's order), then the diagonal
-  std::vector<int> lrowptr, lcol, lsrc, lrow;
-  // L^T: per column j the L entries of that column
-  std::vector<int> trowptr, tidx;
+// What the host looks at before the lists are built.
+struct GraphCheck {
+  int bad_col;   // a column outside the matrix
+  int bad_diag;  // a row without a positive diagonal entry
+  int max_col;   // most L entries in a column
 };
+constexpr int kShortCol = 32;  // longest column of L that is ordered in place
 
-// Builds the graph of a square CSR handle; TBSLA_ERR_BAD_MATRIX unless every
-// row holds a positive diagonal entry.
-int build_graph(const tbsla_matrix* m, HostGraph* g) {
-  const tbsla_info& I = m->info;
-  if (m->format != TBSLA_CSR || I.ln_row != I.ln_col || I.f_col != 0) return TBSLA_ERR_INVALID_ARG;
-  const int n = I.ln_row;
-  const int* rp = m->idx0.data();
-  const int* ci = m->idx1.data();
-  const int base = rp[0];
-  g->n = n;
-  g->rowptr.resize(n + 1);
-  for (int i = 0; i <= n; i++) g->rowptr[i] = rp[i] - base;
-  const long nnz = g->rowptr[n];
-  g->colidx.assign(ci + base, ci + base + nnz);
-  g->aval.resize(nnz);
-  std::vector<double> d(n, 0.0);
-  for (int i = 0; i < n; i++)
-    for (long k = g->rowptr[i]; k < g->rowptr[i + 1]; k++) {
-      g->aval[k] = (float)m->values[base + k];
-      if (g->colidx[k] == i) d[i] += m->values[base + k];
+// s_i = a_ii^-1/2 in FP32 (repeated diagonal entries added in FP64), A's
+// values in FP32, and the lengths of L's row and column i.  The FP32
+// operations of s, e and x are those of k_dia_features, so that both give the
+// same bits.
+__global__ void __launch_bounds__(NT) k_graph_rows(int n, int base, const int* __restrict__ rowptr,
+                                                  const int* __restrict__ colidx, const double* __restrict__ a64,
+                                                  float* __restrict__ aval, float* __restrict__ s,
+                                                  unsigned* __restrict__ lcount, unsigned* __restrict__ tcount,
+                                                  GraphCheck* __restrict__ check) {
+  int most = 0;
+  for (long i = blockIdx.x * (long)NT + threadIdx.x; i < n; i += (long)gridDim.x * NT) {
+    const int k0 = rowptr[i] - base, k1 = rowptr[i + 1] - base;
+    double d = 0;
+    unsigned nl = 1;
+    for (int k = k0; k < k1; k++) {
+      const double v = a64[k];
+      const int j = colidx[k];
+      aval[k] = (float)v;
+      if (j < 0 || j >= n) {
+        check->bad_col = 1;
+        continue;
+      }
+      if (j == i) d += v;
+      if (j < i) {
+        nl++;
+        most = max(most, (int)atomicAdd(tcount + j, 1u) + 1);
+      }
     }
-  // s, e and the node inputs in FP32, in the operations the device-side
-  // feature kernel uses (k_dia_features), so that both give the same bits
-  g->s.resize(n);
-  for (int i = 0; i < n; i++) {
-    if (!(d[i] > 0)) return TBSLA_ERR_BAD_MATRIX;
-    g->s[i] = 1.0f / std::sqrt((float)d[i]);
+    if (!(d > 0)) check->bad_diag = 1;
+    s[i] = 1.0f / sqrtf((float)d);
+    lcount[i] = nl;
+    most = max(most, (int)atomicAdd(tcount + i, 1u) + 1);
   }
-  g->e.resize(nnz);
-  g->x.assign((size_t)n * F0, 0.f);
-  g->lrowptr.assign(n + 1, 0);
-  for (int i = 0; i < n; i++) {
+  most = __reduce_max_sync(FULL, most);
+  if ((threadIdx.x & 31) == 0) atomicMax(&check->max_col, most);
+}
+
+// Edge weights and node inputs; L's entries (lsrc: the entry of A, -1 for the
+// diagonal), and into L^T's lists either their places (tnext: the next free
+// place of each column, in any order) or, with tnext null, sort keys.
+__global__ void __launch_bounds__(NT) k_graph_fill(int n, const int* __restrict__ rowptr,
+                                                  const int* __restrict__ colidx, const float* __restrict__ aval,
+                                                  const float* __restrict__ s, const int* __restrict__ lrowptr,
+                                                  float* __restrict__ e, float* __restrict__ x,
+                                                  int* __restrict__ lcol, int* __restrict__ lsrc,
+                                                  int* __restrict__ lrow, unsigned* __restrict__ tnext,
+                                                  uint64_t* __restrict__ keys, int* __restrict__ tidx) {
+  for (long i = blockIdx.x * (long)NT + threadIdx.x; i < n; i += (long)gridDim.x * NT) {
+    const float si = s[i];
     float se = 0.f, se2 = 0.f;
-    int deg = 0, nl = 0;
-    for (long k = g->rowptr[i]; k < g->rowptr[i + 1]; k++) {
-      const int j = g->colidx[k];
-      const float e = (float)m->values[base + k] * g->s[i] * g->s[j];
-      g->e[k] = e;
+    int deg = 0, q = lrowptr[i];
+    auto entry = [&](int col, int src) {
+      lcol[q] = col;
+      lsrc[q] = src;
+      lrow[q] = (int)i;
+      if (tnext) {
+        tidx[atomicAdd(tnext + col, 1u)] = q;
+      } else {
+        keys[q] = (unsigned)col;
+        tidx[q] = q;
+      }
+      q++;
+    };
+    for (int k = rowptr[i]; k < rowptr[i + 1]; k++) {
+      const int j = colidx[k];
+      const float ev = __fmul_rn(__fmul_rn(aval[k], si), s[j]);
+      e[k] = ev;
       if (j != i) {
-        se = se + e;
-        se2 = std::fma(e, e, se2);
+        se = __fadd_rn(se, ev);
+        se2 = fmaf(ev, ev, se2);
         deg++;
       }
-      if (j < i) nl++;
+      if (j < i) entry(j, k);
     }
-    g->x[(size_t)i * F0 + 0] = 1.f;
-    g->x[(size_t)i * F0 + 1] = se;
-    g->x[(size_t)i * F0 + 2] = se2;
-    g->x[(size_t)i * F0 + 3] = deg / 8.f;
-    g->lrowptr[i + 1] = g->lrowptr[i] + nl + 1;
+    entry((int)i, -1);
+    x[i * F0 + 0] = 1.f;
+    x[i * F0 + 1] = se;
+    x[i * F0 + 2] = se2;
+    x[i * F0 + 3] = deg / 8.f;
   }
-  const long nl = g->lrowptr[n];
-  g->lcol.resize(nl);
-  g->lsrc.resize(nl);
-  g->lrow.resize(nl);
-  for (int i = 0; i < n; i++) {
-    long q = g->lrowptr[i];
-    for (long k = g->rowptr[i]; k < g->rowptr[i + 1]; k++)
-      if (g->colidx[k] < i) {
-        g->lcol[q] = g->colidx[k];
-        g->lsrc[q] = (int)k;
-        g->lrow[q++] = i;
-      }
-    g->lcol[q] = i;
-    g->lsrc[q] = -1;
-    g->lrow[q] = i;
+}
+
+// L^T's lists into row order (columns of at most kShortCol entries).
+__global__ void __launch_bounds__(NT) k_order_columns(int n, const int* __restrict__ trowptr,
+                                                     int* __restrict__ tidx) {
+  for (long j = blockIdx.x * (long)NT + threadIdx.x; j < n; j += (long)gridDim.x * NT) {
+    const int t0 = trowptr[j], t1 = trowptr[j + 1];
+    for (int t = t0 + 1; t < t1; t++) {
+      const int q = tidx[t];
+      int u = t;
+      for (; u > t0 && tidx[u - 1] > q; u--) tidx[u] = tidx[u - 1];
+      tidx[u] = q;
+    }
   }
-  g->trowptr.assign(n + 1, 0);
-  for (long q = 0; q < nl; q++) g->trowptr[g->lcol[q] + 1]++;
-  for (int j = 0; j < n; j++) g->trowptr[j + 1] += g->trowptr[j];
-  g->tidx.resize(nl);
-  std::vector<int> fill(g->trowptr.begin(), g->trowptr.end() - 1);
-  for (long q = 0; q < nl; q++) g->tidx[fill[g->lcol[q]]++] = (int)q;
-  return TBSLA_OK;
+}
+
+__global__ void k_shift(int n, int base, int* __restrict__ v) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) v[i] -= base;
+}
+
+__global__ void k_narrow(long len, const double* __restrict__ src, float* __restrict__ dst) {
+  for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < len; t += (long)gridDim.x * blockDim.x)
+    dst[t] = __double2float_rn(src[t]);
 }
 
 // ---- device kernels: forward ---------------------------------------------------------
@@ -154,10 +191,10 @@ __device__ __forceinline__ float sigmoid(float v) { return 1.f / (1.f + expf(-v)
 __device__ __forceinline__ long warp_id() { return ((long)blockIdx.x * NT + threadIdx.x) / kWarp; }
 __device__ __forceinline__ long warp_count() { return (long)gridDim.x * NT / kWarp; }
 
-// h0 = relu(W0 x + b0); lane o is feature o.  z0 (the pre-activation, kept
-// for the backward pass) may be null for inference.
+// h0 = relu(W0 x + b0); lane o is feature o.  mask[i] bit o: the
+// pre-activation is positive (what the backward pass needs of it).
 __global__ void __launch_bounds__(NT) k_layer0(int n, const float* __restrict__ x, const float* __restrict__ w,
-                                              float* __restrict__ z0, float* __restrict__ h0) {
+                                              unsigned* __restrict__ mask, float* __restrict__ h0) {
   const int o = threadIdx.x & 31;
   float wr[F0];
 #pragma unroll
@@ -167,53 +204,189 @@ __global__ void __launch_bounds__(NT) k_layer0(int n, const float* __restrict__ 
     float z = b;
 #pragma unroll
     for (int k = 0; k < F0; k++) z += wr[k] * x[i * F0 + k];
-    if (z0) z0[i * H + o] = z;
+    const unsigned pos = __ballot_sync(FULL, z > 0.f);
+    if (o == 0) mask[i] = pos;
     h0[i * H + o] = relu(z);
   }
 }
 
-// out_i (+)= sum_{j != i} e_ij in_j over A's pattern (e symmetric, so this
-// is also the transpose product the backward pass needs).
-__global__ void __launch_bounds__(NT) k_aggregate(int n, const int* __restrict__ rowptr,
-                                                 const int* __restrict__ colidx, const float* __restrict__ e,
-                                                 const float* __restrict__ in, float* __restrict__ out,
-                                                 int accumulate) {
-  const int f = threadIdx.x & 31;
-  for (long i = warp_id(); i < n; i += warp_count()) {
-    float acc = 0.f;
-    for (int k = rowptr[i]; k < rowptr[i + 1]; k++) {
-      const int j = colidx[k];
-      if (j != i) acc += e[k] * in[(long)j * H + f];
+constexpr int NB = 4;  // nodes that a warp takes together
+
+// The lists ptr[i] .. ptr[i + 1) of nodes i0 .. i0 + 3 when all of them have
+// at most 8 entries (every 7-point stencil): lane 8 u + t holds entry t of node
+// i0 + u, so the four lists are read in one go instead of one after another.
+struct Quad {
+  int k;          // this lane's entry (valid if `live`)
+  bool live;
+  bool all_short; // same on every lane
+  __device__ __forceinline__ Quad(const int* __restrict__ ptr, int drop, long i0, int n) {
+    const int lane = threadIdx.x & 31;
+    const long i = i0 + (lane >> 3);
+    const int b = i < n ? ptr[i] : 0, len = i < n ? ptr[i + 1] - drop - b : 0;
+    k = b + (lane & 7);
+    live = (lane & 7) < len;
+    all_short = !__any_sync(FULL, len > 8);
+  }
+};
+
+// acc[u] += sum_{j != i} e_ij in_j over A's row i = i0 + u (e symmetric, so
+// this is also the transpose product the backward pass needs); lane f is
+// feature f, entries in order, 16 neighbours' features in flight.
+__device__ __forceinline__ void gather_rows(const int* __restrict__ rowptr, const int* __restrict__ colidx,
+                                            const float* __restrict__ e, const float* __restrict__ in, long i0,
+                                            int n, int f, float (&acc)[NB]) {
+  const Quad qd(rowptr, 0, i0, n);
+  if (qd.all_short) {
+    const int cl = qd.live ? colidx[qd.k] : 0;
+    const float el = qd.live ? e[qd.k] : 0.f;
+    const unsigned use = __ballot_sync(FULL, qd.live && cl != i0 + (f >> 3));
+#pragma unroll
+    for (int u = 0; u < NB; u += 2) {
+      float v[16];
+#pragma unroll
+      for (int t = 0; t < 16; t++) {
+        const int c = __shfl_sync(FULL, cl, 8 * u + t);
+        v[t] = use >> (8 * u + t) & 1u ? in[(long)c * H + f] : 0.f;
+      }
+#pragma unroll
+      for (int t = 0; t < 16; t++) {
+        const float ev = __shfl_sync(FULL, el, 8 * u + t);
+        if (use >> (8 * u + t) & 1u) acc[u + (t >> 3)] += ev * v[t];
+      }
     }
-    out[i * H + f] = accumulate ? out[i * H + f] + acc : acc;
+    return;
+  }
+#pragma unroll
+  for (int u = 0; u < NB; u++) {
+    const long i = i0 + u;
+    if (i >= n) break;
+    const int k1 = rowptr[i + 1];
+    for (int k0 = rowptr[i]; k0 < k1; k0 += kWarp) {
+      const int m = min(kWarp, k1 - k0);
+      const int cl = f < m ? colidx[k0 + f] : (int)i;
+      const float el = f < m ? e[k0 + f] : 0.f;
+      for (int t = 0; t < m; t += 8) {
+        int c[8];
+        float v[8];
+#pragma unroll
+        for (int r = 0; r < 8; r++) {
+          c[r] = __shfl_sync(FULL, cl, (t + r) & 31);
+          v[r] = t + r < m ? in[(long)c[r] * H + f] : 0.f;
+        }
+#pragma unroll
+        for (int r = 0; r < 8; r++) {
+          const float ev = __shfl_sync(FULL, el, (t + r) & 31);
+          if (t + r < m && c[r] != i) acc[u] += ev * v[r];
+        }
+      }
+    }
   }
 }
 
-// z = W [h; m] + b, h_out = h + relu(z); W (H x 2H) kept transposed in
-// shared memory so that lane o reads W[o][k] without bank conflicts.
-__global__ void __launch_bounds__(NT) k_layer(int n, const float* __restrict__ w, const float* __restrict__ h,
-                                             const float* __restrict__ m, float* __restrict__ z,
-                                             float* __restrict__ hout) {
-  __shared__ float wt[2 * H][H + 1];
-  __shared__ float bs[H];
-  for (int t = threadIdx.x; t < 2 * H * H; t += NT) wt[t % (2 * H)][t / (2 * H)] = w[t];
-  if (threadIdx.x < H) bs[threadIdx.x] = w[2 * H * H + threadIdx.x];
+// out_i = [out_i +] the gathered neighbours of i.  A kernel of its own: fused
+// into the dense layers, whose weights in registers leave 8 to 16 warps on an
+// SM, the gathers' latency showed (48^3 nodes, caches cold: 70 us forward and
+// 185 us backward per layer, against 24 + 28 and 24 + 35 us).
+__global__ void __launch_bounds__(NT) k_gather(int n, const int* __restrict__ rowptr, const int* __restrict__ colidx,
+                                              const float* __restrict__ e, const float* __restrict__ in,
+                                              float* __restrict__ out, int accumulate) {
+  const int f = threadIdx.x & 31;
+  for (long i0 = warp_id() * NB; i0 < n; i0 += warp_count() * NB) {
+    float old[NB], acc[NB];
+#pragma unroll
+    for (int u = 0; u < NB; u++) {
+      old[u] = accumulate && i0 + u < n ? out[(i0 + u) * H + f] : 0.f;
+      acc[u] = 0.f;
+    }
+    gather_rows(rowptr, colidx, e, in, i0, n, f, acc);
+#pragma unroll
+    for (int u = 0; u < NB; u++)
+      if (i0 + u < n) out[(i0 + u) * H + f] = accumulate ? old[u] + acc[u] : acc[u];
+  }
+}
+
+// z = W [h; m] + b, h_out = h + relu(z).  Lane o holds row o of W (H x 2H) in
+// registers; the next pass's activations are loaded under this one's
+// multiply-adds.
+__global__ void __launch_bounds__(NT, 2) k_layer(int n, const float* __restrict__ w, const float* __restrict__ h,
+                                                 const float* __restrict__ m, unsigned* __restrict__ mask,
+                                                 float* __restrict__ hout) {
+  __shared__ float ws[H][2 * H + 1];
+  __shared__ __align__(16) float in[NT / kWarp][NB][2 * H];
+  for (int t = threadIdx.x; t < 2 * H * H; t += NT) ws[t / (2 * H)][t % (2 * H)] = w[t];
   __syncthreads();
   const int o = threadIdx.x & 31;
-  for (long i = warp_id(); i < n; i += warp_count()) {
-    const float hi = h[i * H + o], mi = m[i * H + o];
-    float acc = bs[o];
+  float wr[2 * H];
 #pragma unroll
-    for (int k = 0; k < H; k++) {
-      acc += wt[k][o] * __shfl_sync(FULL, hi, k);
-      acc += wt[H + k][o] * __shfl_sync(FULL, mi, k);
+  for (int k = 0; k < 2 * H; k++) wr[k] = ws[o][k];
+  const float b = w[2 * H * H + o];
+  auto& st = in[threadIdx.x / kWarp];
+  float hi[NB], mi[NB];
+  auto load = [&](long i0) {
+#pragma unroll
+    for (int u = 0; u < NB; u++) {
+      const bool live = i0 + u < n;
+      hi[u] = live ? h[(i0 + u) * H + o] : 0.f;
+      mi[u] = live ? m[(i0 + u) * H + o] : 0.f;
     }
-    z[i * H + o] = acc;
-    hout[i * H + o] = hi + relu(acc);
+  };
+  const long step = warp_count() * NB;
+  long i0 = warp_id() * NB;
+  load(i0);
+  for (; i0 < n; i0 += step) {
+    float hc[NB], acc[NB];
+#pragma unroll
+    for (int u = 0; u < NB; u++) {
+      st[u][o] = hc[u] = hi[u];
+      st[u][H + o] = mi[u];
+      acc[u] = b;
+    }
+    __syncwarp();
+    load(i0 + step);
+#pragma unroll
+    for (int k = 0; k < H; k += 4) {
+#pragma unroll
+      for (int u = 0; u < NB; u++) {
+        const float4 hv = *reinterpret_cast<const float4*>(&st[u][k]);
+        const float4 mv = *reinterpret_cast<const float4*>(&st[u][H + k]);
+        acc[u] += wr[k] * hv.x;
+        acc[u] += wr[H + k] * mv.x;
+        acc[u] += wr[k + 1] * hv.y;
+        acc[u] += wr[H + k + 1] * mv.y;
+        acc[u] += wr[k + 2] * hv.z;
+        acc[u] += wr[H + k + 2] * mv.z;
+        acc[u] += wr[k + 3] * hv.w;
+        acc[u] += wr[H + k + 3] * mv.w;
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < NB; u++) {
+      const unsigned pos = __ballot_sync(FULL, acc[u] > 0.f);
+      if (i0 + u < n) {
+        if (o == 0) mask[i0 + u] = pos;
+        hout[(i0 + u) * H + o] = hc[u] + relu(acc[u]);
+      }
+    }
+    __syncwarp();
   }
 }
 
-// L values: warp per row; lower entries then the diagonal.  xi (the
+// The warp sums wsum() of v0 .. v3 -- the same pairs in the same order -- on
+// every lane of the quarter q = (lane >> 3) of the warp that belongs to v_q:
+// six shuffles instead of twenty.
+__device__ __forceinline__ float wsum4(float v0, float v1, float v2, float v3) {
+  const int lane = threadIdx.x & 31;
+  const bool hi = lane & 16, mid = lane & 8;
+  // distance 16: the lower half keeps v0 and v1, the upper one v2 and v3
+  const float a = (hi ? v2 : v0) + __shfl_xor_sync(FULL, hi ? v0 : v2, 16);
+  const float b = (hi ? v3 : v1) + __shfl_xor_sync(FULL, hi ? v1 : v3, 16);
+  float r = (mid ? b : a) + __shfl_xor_sync(FULL, mid ? a : b, 8);
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) r += __shfl_xor_sync(FULL, r, o);
+  return r;
+}
+
+// L values: a warp per four rows; lower entries then the diagonal.  xi (the
 // diagonal's pre-activation) is kept for the backward pass.
 __global__ void __launch_bounds__(NT) k_head(int n, const int* __restrict__ lrowptr, const int* __restrict__ lcol,
                                             const int* __restrict__ lsrc, const float* __restrict__ e,
@@ -223,41 +396,71 @@ __global__ void __launch_bounds__(NT) k_head(int n, const int* __restrict__ lrow
   const int f = threadIdx.x & 31;
   const float we = w[OFF_WE + f], wd = w[OFF_WD + f];
   const float ce = w[OFF_CE], be = w[OFF_BE], bd = w[OFF_BD];
-  for (long i = warp_id(); i < n; i += warp_count()) {
-    const float hi = h[i * H + f];
-    const int q0 = lrowptr[i], q1 = lrowptr[i + 1] - 1;  // q1: the diagonal
-    for (int q = q0; q < q1; q++) {
-      const float o = wsum(we * hi * h[(long)lcol[q] * H + f]) + ce * e[lsrc[q]] + be;
-      if (f == 0) lval[q] = s[i] * o;
+  for (long i0 = warp_id() * NB; i0 < n; i0 += warp_count() * NB) {
+    float hi[NB];
+#pragma unroll
+    for (int u = 0; u < NB; u++) hi[u] = i0 + u < n ? h[(i0 + u) * H + f] : 0.f;
+    const Quad qd(lrowptr, 1, i0, n);  // the strictly lower entries
+    if (qd.all_short) {
+      const int cl = qd.live ? lcol[qd.k] : 0;
+      const float el = qd.live ? e[lsrc[qd.k]] : 0.f;
+      const unsigned use = __ballot_sync(FULL, qd.live);
+      float dot = 0.f;  // this lane's entry's sum
+#pragma unroll
+      for (int u = 0; u < NB; u++) {
+#pragma unroll
+        for (int t = 0; t < 8; t += 4) {
+          if ((use >> (8 * u + t) & 0xfu) == 0) continue;
+          float v[4];
+#pragma unroll
+          for (int r = 0; r < 4; r++) {
+            const int j = __shfl_sync(FULL, cl, 8 * u + t + r);
+            v[r] = use >> (8 * u + t + r) & 1u ? h[(long)j * H + f] : 0.f;
+          }
+#pragma unroll
+          for (int r = 0; r < 4; r++) v[r] = we * hi[u] * v[r];
+          // v[r]'s sum from a lane of quarter r to the lane that holds the entry
+          const float q = wsum4(v[0], v[1], v[2], v[3]);
+          const float d = __shfl_sync(FULL, q, (f & 3) * 8);
+          if (f >> 2 == 2 * u + (t >> 2)) dot = d;
+        }
+      }
+      if (qd.live) lval[qd.k] = s[i0 + (f >> 3)] * (dot + ce * el + be);
+    } else {
+#pragma unroll
+      for (int u = 0; u < NB; u++) {
+        const long i = i0 + u;
+        if (i >= n) break;
+        for (int q = lrowptr[i]; q < lrowptr[i + 1] - 1; q++) {
+          const float o = wsum(we * hi[u] * h[(long)lcol[q] * H + f]) + ce * e[lsrc[q]] + be;
+          if (f == 0) lval[q] = s[i] * o;
+        }
+      }
     }
-    const float x = wsum(wd * hi) + bd;
-    if (f == 0) {
+    const float x = wsum4(wd * hi[0], wd * hi[1], wd * hi[2], wd * hi[3]) + bd;
+    const long i = i0 + (f >> 3);
+    if ((f & 7) == 0 && i < n) {
       xi[i] = x;
-      lval[q1] = s[i] * softplus(x);
+      lval[lrowptr[i + 1] - 1] = s[i] * softplus(x);
     }
   }
 }
 
 // ---- device kernels: loss ------------------------------------------------------------
-// Probe blocks are n x P row-major (P <= 16), one thread per row.
+// Probe blocks are n x P row-major (P <= 16), a thread per row and probe: the
+// P threads of a row read consecutive words of every X row.
 
 constexpr int PMAX = 16;
 
 // Y = A X on A's pattern (FP32 values).
 __global__ void k_spmm_a(int n, int P, const int* __restrict__ rowptr, const int* __restrict__ colidx,
                          const float* __restrict__ a, const float* __restrict__ X, float* __restrict__ Y) {
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
-    float acc[PMAX] = {};
-    for (int k = rowptr[i]; k < rowptr[i + 1]; k++) {
-      const float v = a[k];
-      const float* xr = X + (long)colidx[k] * P;
-#pragma unroll
-      for (int p = 0; p < PMAX; p++)
-        if (p < P) acc[p] += v * xr[p];
-    }
-#pragma unroll
-    for (int p = 0; p < PMAX; p++)
-      if (p < P) Y[i * P + p] = acc[p];
+  const long len = (long)n * P;
+  for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < len; t += (long)gridDim.x * blockDim.x) {
+    const int i = (int)((unsigned)t / (unsigned)P), p = (int)(t - (long)i * P);
+    float acc = 0.f;
+    for (int k = rowptr[i]; k < rowptr[i + 1]; k++) acc += a[k] * X[(long)colidx[k] * P + p];
+    Y[t] = acc;
   }
 }
 
@@ -265,19 +468,15 @@ __global__ void k_spmm_a(int n, int P, const int* __restrict__ rowptr, const int
 __global__ void k_spmm_l(int n, int P, const int* __restrict__ ptr, const int* __restrict__ idx,
                          const int* __restrict__ other, const float* __restrict__ lval, int transpose,
                          const float* __restrict__ X, float* __restrict__ Y) {
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
-    float acc[PMAX] = {};
-    for (int t = ptr[i]; t < ptr[i + 1]; t++) {
-      const int q = transpose ? idx[t] : t;    // L entry
-      const int j = other[q];                  // its column (L) or row (L^T)
-      const float v = lval[q];
-#pragma unroll
-      for (int p = 0; p < PMAX; p++)
-        if (p < P) acc[p] += v * X[(long)j * P + p];
+  const long len = (long)n * P;
+  for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < len; t += (long)gridDim.x * blockDim.x) {
+    const int i = (int)((unsigned)t / (unsigned)P), p = (int)(t - (long)i * P);
+    float acc = 0.f;
+    for (int k = ptr[i]; k < ptr[i + 1]; k++) {
+      const int q = transpose ? idx[k] : k;  // L entry; its column (L) or row (L^T):
+      acc += lval[q] * X[(long)other[q] * P + p];
     }
-#pragma unroll
-    for (int p = 0; p < PMAX; p++)
-      if (p < P) Y[i * P + p] = acc[p];
+    Y[t] = acc;
   }
 }
 
@@ -327,35 +526,98 @@ __global__ void k_gauss(long len, unsigned long long seed, float* __restrict__ Z
 
 // ---- device kernels: backward --------------------------------------------------------
 
-// Head, row side: dL -> parameter gradients of the head, and dh_i
-// (written, not added: the first contribution to dh).
+// Head: dL -> parameter gradients of the head, and dh (written, not added: the
+// first contribution to it), a warp per four nodes.  Row side: the row's lower
+// entries and its diagonal; column side: dh_i += sum over the strictly lower
+// entries (r, i) of s_r dL_ri w_e * h_r.
 __global__ void __launch_bounds__(NT) k_head_bwd(int n, const int* __restrict__ lrowptr,
                                                 const int* __restrict__ lcol, const int* __restrict__ lsrc,
-                                                const float* __restrict__ e, const float* __restrict__ s,
-                                                const float* __restrict__ w, const float* __restrict__ h,
-                                                const float* __restrict__ dl, const float* __restrict__ xi,
-                                                float* __restrict__ dh, float* __restrict__ grad) {
+                                                const int* __restrict__ trowptr, const int* __restrict__ tidx,
+                                                const int* __restrict__ lrow, const float* __restrict__ e,
+                                                const float* __restrict__ s, const float* __restrict__ w,
+                                                const float* __restrict__ h, const float* __restrict__ dl,
+                                                const float* __restrict__ xi, float* __restrict__ dh,
+                                                float* __restrict__ grad) {
   __shared__ float part[NT / kWarp][2 * H + 3];
   const int f = threadIdx.x & 31, wi = threadIdx.x / kWarp;
   const float we = w[OFF_WE + f], wd = w[OFF_WD + f];
-  float gwe = 0.f, gwd = 0.f, gce = 0.f, gbe = 0.f, gbd = 0.f;
-  for (long i = warp_id(); i < n; i += warp_count()) {
-    const float hi = h[i * H + f], si = s[i];
-    const int q0 = lrowptr[i], q1 = lrowptr[i + 1] - 1;
-    float d = 0.f;
-    for (int q = q0; q < q1; q++) {
-      const float dO = si * dl[q];
-      const float hj = h[(long)lcol[q] * H + f];
-      gwe += dO * hi * hj;
-      gce += dO * e[lsrc[q]];
-      gbe += dO;
-      d += dO * we * hj;
+  float gwe = 0.f, gwd = 0.f, gce = 0.f, gbe = 0.f, gbd = 0.f;  // gce, gbe, gbd: this lane's entries
+  for (long i0 = warp_id() * NB; i0 < n; i0 += warp_count() * NB) {
+    float hi[NB], d[NB], dc[NB];
+#pragma unroll
+    for (int u = 0; u < NB; u++) {
+      hi[u] = i0 + u < n ? h[(i0 + u) * H + f] : 0.f;
+      d[u] = dc[u] = 0.f;
     }
-    const float dxi = si * dl[q1] * sigmoid(xi[i]);
-    gwd += dxi * hi;
+    const Quad lo(lrowptr, 1, i0, n), up(trowptr, 0, i0, n);
+    if (lo.all_short && up.all_short) {
+      const long i = i0 + (f >> 3);
+      const int cl = lo.live ? lcol[lo.k] : 0, src = lo.live ? lsrc[lo.k] : 0;
+      const int q = up.live ? tidx[up.k] : 0;
+      const float dO = lo.live ? s[i] * dl[lo.k] : 0.f;
+      const int rl = up.live ? lrow[q] : 0;
+      const float cf = up.live ? s[rl] * dl[q] : 0.f;
+      if (lo.live) {
+        gce += dO * e[src];
+        gbe += dO;
+      }
+      const unsigned ul = __ballot_sync(FULL, lo.live), uc = __ballot_sync(FULL, up.live && rl != i);
+#pragma unroll
+      for (int u = 0; u < NB; u++) {
+        float v[8], r[8];
+#pragma unroll
+        for (int t = 0; t < 8; t++) {
+          const int j = __shfl_sync(FULL, cl, 8 * u + t), k = __shfl_sync(FULL, rl, 8 * u + t);
+          v[t] = ul >> (8 * u + t) & 1u ? h[(long)j * H + f] : 0.f;
+          r[t] = uc >> (8 * u + t) & 1u ? h[(long)k * H + f] : 0.f;
+        }
+#pragma unroll
+        for (int t = 0; t < 8; t++) {
+          const float g = __shfl_sync(FULL, dO, 8 * u + t), c = __shfl_sync(FULL, cf, 8 * u + t);
+          if (ul >> (8 * u + t) & 1u) {
+            gwe += g * hi[u] * v[t];
+            d[u] += g * we * v[t];
+          }
+          if (uc >> (8 * u + t) & 1u) dc[u] += c * we * r[t];
+        }
+      }
+    } else {
+#pragma unroll
+      for (int u = 0; u < NB; u++) {
+        const long i = i0 + u;
+        if (i >= n) break;
+        for (int q = lrowptr[i]; q < lrowptr[i + 1] - 1; q++) {
+          const float g = s[i] * dl[q], hj = h[(long)lcol[q] * H + f];
+          gwe += g * hi[u] * hj;
+          d[u] += g * we * hj;
+          if (f == 0) {
+            gce += g * e[lsrc[q]];
+            gbe += g;
+          }
+        }
+        for (int t = trowptr[i]; t < trowptr[i + 1]; t++) {
+          const int q = tidx[t], r = lrow[q];
+          if (r != i) dc[u] += s[r] * dl[q] * we * h[(long)r * H + f];
+        }
+      }
+    }
+    // the diagonals, a lane each, then broadcast
+    float dxi = 0.f;
+    if (f < NB && i0 + f < n) {
+      const long i = i0 + f;
+      dxi = s[i] * dl[lrowptr[i + 1] - 1] * sigmoid(xi[i]);
+    }
     gbd += dxi;
-    dh[i * H + f] = d + dxi * wd;
+#pragma unroll
+    for (int u = 0; u < NB; u++) {
+      const float x = __shfl_sync(FULL, dxi, u);
+      gwd += x * hi[u];
+      if (i0 + u < n) dh[(i0 + u) * H + f] = d[u] + x * wd + dc[u];
+    }
   }
+  gce = wsum(gce);
+  gbe = wsum(gbe);
+  gbd = wsum(gbd);
   part[wi][f] = gwe;
   part[wi][H + f] = gwd;
   if (f == 0) {
@@ -372,86 +634,134 @@ __global__ void __launch_bounds__(NT) k_head_bwd(int n, const int* __restrict__ 
   }
 }
 
-// Head, column side: dh_j += sum over strictly lower entries (i, j) of
-// s_i dL_ij w_e * h_i.
-__global__ void __launch_bounds__(NT) k_head_bwd_cols(int n, const int* __restrict__ trowptr,
-                                                     const int* __restrict__ tidx, const int* __restrict__ lrow,
-                                                     const float* __restrict__ s, const float* __restrict__ w,
-                                                     const float* __restrict__ h, const float* __restrict__ dl,
-                                                     float* __restrict__ dh) {
-  const int f = threadIdx.x & 31;
-  const float we = w[OFF_WE + f];
-  for (long j = warp_id(); j < n; j += warp_count()) {
-    float d = 0.f;
-    for (int t = trowptr[j]; t < trowptr[j + 1]; t++) {
-      const int q = tidx[t];
-      const int i = lrow[q];
-      if (i == j) continue;  // the diagonal was handled on the row side
-      d += s[i] * dl[q] * we * h[(long)i * H + f];
-    }
-    dh[j * H + f] += d;
-  }
-}
-
 // Message layer backward for h_out = h + relu(W [h; m] + b):
-//   dz = dh_out * (z > 0);  dW += dz [h; m]^T;  db += dz;
+//   dz = dh_out where z > 0, else 0;  dW += dz [h; m]^T;  db += dz;
 //   dh_in = dh_out + (W^T dz)[:H] (in place);  dm = (W^T dz)[H:]
-__global__ void __launch_bounds__(NT) k_layer_bwd(int n, const float* __restrict__ w, const float* __restrict__ h,
-                                                 const float* __restrict__ m, const float* __restrict__ z,
-                                                 float* __restrict__ dh, float* __restrict__ dm,
-                                                 float* __restrict__ grad) {
-  __shared__ float wt[2 * H][H + 1];
-  __shared__ float gsum[2 * H * H + H];
-  for (int t = threadIdx.x; t < 2 * H * H; t += NT) wt[t % (2 * H)][t / (2 * H)] = w[t];
-  for (int t = threadIdx.x; t < 2 * H * H + H; t += NT) gsum[t] = 0.f;
+// Lane o holds columns o and H + o of W and row o of dW in registers; the
+// next pass's activations are loaded under this one's multiply-adds.
+__global__ void __launch_bounds__(NT, 1) k_layer_bwd(int n, const float* __restrict__ w, const float* __restrict__ h,
+                                                    const float* __restrict__ m, const unsigned* __restrict__ mask,
+                                                    float* __restrict__ dh, float* __restrict__ dm,
+                                                    float* __restrict__ grad) {
+  constexpr int S = 2 * H + 1;
+  __shared__ float ws[H * S];
+  __shared__ __align__(16) float in[NT / kWarp][NB][2 * H];
+  __shared__ __align__(16) float sdz[NT / kWarp][NB][H];
+  for (int t = threadIdx.x; t < 2 * H * H; t += NT) ws[t / (2 * H) * S + t % (2 * H)] = w[t];
   __syncthreads();
-  const int o = threadIdx.x & 31;
-  float gw[2 * H];
+  const int o = threadIdx.x & 31, wi = threadIdx.x / kWarp;
+  float wh[H], wm[H], gw[2 * H];
+#pragma unroll
+  for (int k = 0; k < H; k++) {
+    wh[k] = ws[k * S + o];
+    wm[k] = ws[k * S + H + o];
+  }
 #pragma unroll
   for (int k = 0; k < 2 * H; k++) gw[k] = 0.f;
   float gb = 0.f;
-  for (long i = warp_id(); i < n; i += warp_count()) {
-    const float dz = z[i * H + o] > 0.f ? dh[i * H + o] : 0.f;
-    const float hi = h[i * H + o], mi = m[i * H + o];
-    float dhin = 0.f, dmin = 0.f;
+  float hi[NB], mi[NB], di[NB];
+  unsigned mk[NB];
+  auto load = [&](long i0) {
 #pragma unroll
-    for (int k = 0; k < H; k++) {
-      gw[k] += dz * __shfl_sync(FULL, hi, k);
-      gw[H + k] += dz * __shfl_sync(FULL, mi, k);
-      const float dzk = __shfl_sync(FULL, dz, k);  // lane o gathers sum_k W[k][o] dz_k
-      dhin += wt[o][k] * dzk;
-      dmin += wt[H + o][k] * dzk;
+    for (int u = 0; u < NB; u++) {
+      const bool live = i0 + u < n;
+      hi[u] = live ? h[(i0 + u) * H + o] : 0.f;
+      mi[u] = live ? m[(i0 + u) * H + o] : 0.f;
+      di[u] = live ? dh[(i0 + u) * H + o] : 0.f;
+      mk[u] = live ? mask[i0 + u] : 0u;
     }
-    gb += dz;
-    dh[i * H + o] += dhin;
-    dm[i * H + o] = dmin;
-  }
+  };
+  const long step = warp_count() * NB;
+  long i0 = warp_id() * NB;
+  load(i0);
+  for (; i0 < n; i0 += step) {
+    float dhi[NB], dz[NB];
 #pragma unroll
-  for (int k = 0; k < 2 * H; k++) atomicAdd(&gsum[o * 2 * H + k], gw[k]);
-  atomicAdd(&gsum[2 * H * H + o], gb);
+    for (int u = 0; u < NB; u++) {
+      dhi[u] = di[u];
+      dz[u] = mk[u] >> o & 1u ? di[u] : 0.f;
+      in[wi][u][o] = hi[u];
+      in[wi][u][H + o] = mi[u];
+      sdz[wi][u][o] = dz[u];
+      gb += dz[u];
+    }
+    __syncwarp();
+    load(i0 + step);
+    float a[NB], c[NB];  // W^T dz
+#pragma unroll
+    for (int u = 0; u < NB; u++) a[u] = c[u] = 0.f;
+#pragma unroll
+    for (int k = 0; k < H; k += 4) {
+#pragma unroll
+      for (int u = 0; u < NB; u++) {
+        const float4 z = *reinterpret_cast<const float4*>(&sdz[wi][u][k]);
+        a[u] += wh[k] * z.x;
+        c[u] += wm[k] * z.x;
+        a[u] += wh[k + 1] * z.y;
+        c[u] += wm[k + 1] * z.y;
+        a[u] += wh[k + 2] * z.z;
+        c[u] += wm[k + 2] * z.z;
+        a[u] += wh[k + 3] * z.w;
+        c[u] += wm[k + 3] * z.w;
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < NB; u++) {
+#pragma unroll
+      for (int k = 0; k < 2 * H; k += 4) {
+        const float4 v = *reinterpret_cast<const float4*>(&in[wi][u][k]);
+        gw[k] += dz[u] * v.x;
+        gw[k + 1] += dz[u] * v.y;
+        gw[k + 2] += dz[u] * v.z;
+        gw[k + 3] += dz[u] * v.w;
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < NB; u++)
+      if (i0 + u < n) {
+        dh[(i0 + u) * H + o] = dhi[u] + a[u];
+        dm[(i0 + u) * H + o] = c[u];
+      }
+    __syncwarp();
+  }
+  // the warps' gradients, added in warp order (row o of dW at stride S: no
+  // bank conflicts), then one addition per CTA
   __syncthreads();
-  for (int t = threadIdx.x; t < 2 * H * H + H; t += NT) atomicAdd(grad + t, gsum[t]);
+  for (int wv = 0; wv < NT / kWarp; wv++) {
+    if (wi == wv) {
+#pragma unroll
+      for (int k = 0; k < 2 * H; k++) ws[o * S + k] = wv ? ws[o * S + k] + gw[k] : gw[k];
+      in[0][0][o] = wv ? in[0][0][o] + gb : gb;
+    }
+    __syncthreads();
+  }
+  for (int t = threadIdx.x; t < 2 * H * H; t += NT) atomicAdd(grad + t, ws[t / (2 * H) * S + t % (2 * H)]);
+  if (threadIdx.x < H) atomicAdd(grad + 2 * H * H + threadIdx.x, in[0][0][threadIdx.x]);
 }
 
 // Input layer backward: dW0 += dz0 x^T, db0 += dz0.
-__global__ void __launch_bounds__(NT) k_layer0_bwd(int n, const float* __restrict__ x, const float* __restrict__ z0,
-                                                  const float* __restrict__ dh, float* __restrict__ grad) {
-  __shared__ float gsum[H * F0 + H];
-  for (int t = threadIdx.x; t < H * F0 + H; t += NT) gsum[t] = 0.f;
-  __syncthreads();
-  const int o = threadIdx.x & 31;
+__global__ void __launch_bounds__(NT) k_layer0_bwd(int n, const float* __restrict__ x,
+                                                  const unsigned* __restrict__ mask, const float* __restrict__ dh,
+                                                  float* __restrict__ grad) {
+  __shared__ float gsum[NT / kWarp][F0 + 1][H];
+  const int o = threadIdx.x & 31, wi = threadIdx.x / kWarp;
   float gw[F0] = {}, gb = 0.f;
   for (long i = warp_id(); i < n; i += warp_count()) {
-    const float dz = z0[i * H + o] > 0.f ? dh[i * H + o] : 0.f;
+    const float dz = mask[i] >> o & 1u ? dh[i * H + o] : 0.f;
 #pragma unroll
     for (int k = 0; k < F0; k++) gw[k] += dz * x[i * F0 + k];
     gb += dz;
   }
 #pragma unroll
-  for (int k = 0; k < F0; k++) atomicAdd(&gsum[o * F0 + k], gw[k]);
-  atomicAdd(&gsum[H * F0 + o], gb);
+  for (int k = 0; k < F0; k++) gsum[wi][k][o] = gw[k];
+  gsum[wi][F0][o] = gb;
   __syncthreads();
-  for (int t = threadIdx.x; t < H * F0 + H; t += NT) atomicAdd(grad + OFF_W0 + t, gsum[t]);
+  for (int t = threadIdx.x; t < (F0 + 1) * H; t += NT) {
+    const int k = t / H, r = t % H;
+    float acc = 0.f;
+    for (int v = 0; v < NT / kWarp; v++) acc += gsum[v][k][r];
+    atomicAdd(grad + (k < F0 ? OFF_W0 + r * F0 + k : OFF_B0 + r), acc);
+  }
 }
 
 // Adam (Kingma & Ba 2015) on the FP32 master parameters; the forward copy is
@@ -696,84 +1006,160 @@ struct Grow {
   }
 };
 
-// Device copy of a graph plus the activations and probe blocks of one pass.
+// One system's graph plus the activations and probe blocks of one pass.
 struct Work {
   int n = 0, P = 0;
   long nnz = 0, nl = 0;
-  Grow<int> rowptr, colidx, lrowptr, lcol, lsrc, lrow, trowptr, tidx;
+  Grow<int> rowptr, colidx, lrowptr, lcol, lsrc, lrow, trowptr, tidx, tidx2;
+  Grow<GraphCheck> check;
+  Grow<uint64_t> keys, keys2;
+  Grow<unsigned> scratch, tnext, mask[NL + 1];
+  Grow<double> a64;
   Grow<float> aval, e, s, x, lval, xi, dl;
-  Grow<float> h[NL + 1], z[NL + 1], m[NL + 1], dh, dm;
+  Grow<float> h[NL + 1], m[NL + 1], dh, dm;
   Grow<float> Z, U, V, W, G, GV;
   void release() {
-    for (auto* g : {&rowptr, &colidx, &lrowptr, &lcol, &lsrc, &lrow, &trowptr, &tidx}) g->release();
+    for (auto* g : {&rowptr, &colidx, &lrowptr, &lcol, &lsrc, &lrow, &trowptr, &tidx, &tidx2}) g->release();
+    for (auto* g : {&keys, &keys2}) g->release();
     for (auto* g : {&aval, &e, &s, &x, &lval, &xi, &dl, &dh, &dm, &Z, &U, &V, &W, &G, &GV}) g->release();
+    check.release();
+    tnext.release();
+    scratch.release();
+    a64.release();
     for (int l = 0; l <= NL; l++) {
       h[l].release();
-      z[l].release();
       m[l].release();
+      mask[l].release();
     }
   }
 };
 
-int upload(const HostGraph& g, int P, Work* w, cudaStream_t s) {
-  int st;
-  w->n = g.n;
-  w->P = P;
-  w->nnz = (long)g.colidx.size();
-  w->nl = (long)g.lcol.size();
-  if ((st = w->rowptr.put(g.rowptr, s)) || (st = w->colidx.put(g.colidx, s)) || (st = w->aval.put(g.aval, s)) ||
-      (st = w->e.put(g.e, s)) || (st = w->s.put(g.s, s)) || (st = w->x.put(g.x, s)) ||
-      (st = w->lrowptr.put(g.lrowptr, s)) || (st = w->lcol.put(g.lcol, s)) || (st = w->lsrc.put(g.lsrc, s)) ||
-      (st = w->lrow.put(g.lrow, s)) || (st = w->trowptr.put(g.trowptr, s)) || (st = w->tidx.put(g.tidx, s)))
-    return st;
-  const size_t nh = (size_t)g.n * H, np = (size_t)g.n * std::max(P, 1);
-  for (int l = 0; l <= NL; l++)
-    if ((st = w->h[l].need(nh)) || (st = w->z[l].need(nh)) || (st = w->m[l].need(nh))) return st;
-  if ((st = w->dh.need(nh)) || (st = w->dm.need(nh)) || (st = w->lval.need(w->nl)) || (st = w->xi.need(g.n)) ||
-      (st = w->dl.need(w->nl)))
-    return st;
-  for (auto* b : {&w->Z, &w->U, &w->V, &w->W, &w->G, &w->GV})
-    if ((st = b->need(np))) return st;
-  return TBSLA_OK;
-}
-
 int warp_grid(long n) { return (int)std::max<long>(1, std::min<long>((n + NT / kWarp - 1) / (NT / kWarp), 152L * 8)); }
 int row_grid(long n) { return (int)std::max<long>(1, std::min<long>((n + NT - 1) / NT, 152L * 16)); }
+// CTAs of the dense-layer kernels: a pass of NB nodes per warp, at most `per`
+// CTAs per SM, which share the loading of the weights among many passes
+int layer_grid(long n, int per) {
+  return (int)std::max<long>(1, std::min<long>((n + NB * (NT / kWarp) - 1) / (NB * (NT / kWarp)), 152L * per));
+}
 
+// The graph of a square CSR handle, built on the device from its arrays, and
+// the buffers of a pass with P probes; TBSLA_ERR_BAD_MATRIX unless every row
+// holds a positive diagonal entry.  Synchronises once (the length of L and
+// the check of the diagonal).
+int build_graph(const tbsla_matrix* mat, int P, Work* w, cudaStream_t st) {
+  const tbsla_info& I = mat->info;
+  if (mat->format != TBSLA_CSR || I.ln_row != I.ln_col || I.f_col != 0) return TBSLA_ERR_INVALID_ARG;
+  const int n = I.ln_row;
+  if (n > 0 && I.nnz == 0) return TBSLA_ERR_BAD_MATRIX;
+  // the row pointer here (as tbsla_impl::validate does), the columns on the device
+  if (n > 0 && mat->idx0.size() != (size_t)n + 1) return TBSLA_ERR_BAD_MATRIX;
+  const int* rp = mat->idx0.data();
+  const int base = n > 0 ? rp[0] : 0;
+  int falls = base < 0;
+  for (int i = 0; i < n; i++) falls |= rp[i + 1] < rp[i];
+  if (falls) return TBSLA_ERR_BAD_MATRIX;
+  const long end = n > 0 ? rp[n] : 0, nnz = end - base;
+  if ((size_t)end > mat->idx1.size() || (size_t)end > mat->values.size()) return TBSLA_ERR_BAD_MATRIX;
+  w->n = n;
+  w->P = P;
+  w->nnz = nnz;
+  w->nl = 0;
+  int r;
+  const size_t nh = (size_t)n * H, np = (size_t)n * std::max(P, 1), n1 = (size_t)n + 1;
+  if ((r = w->rowptr.need(n1)) || (r = w->colidx.need(nnz)) || (r = w->a64.need(nnz)) || (r = w->aval.need(nnz)) ||
+      (r = w->e.need(nnz)) || (r = w->s.need(n)) || (r = w->x.need((size_t)n * F0)) || (r = w->lrowptr.need(n1)) ||
+      (r = w->trowptr.need(n1)) || (r = w->tnext.need(n1)) || (r = w->check.need(1)) ||
+      (r = w->scratch.need(tbsla_gpu::scan_scratch((long)n1))) || (r = w->dh.need(nh)) || (r = w->dm.need(nh)) ||
+      (r = w->xi.need(n)))
+    return r;
+  for (int l = 0; l <= NL; l++)
+    if ((r = w->h[l].need(nh)) || (r = w->m[l].need(nh)) || (r = w->mask[l].need(n))) return r;
+  for (auto* b : {&w->Z, &w->U, &w->V, &w->W, &w->G, &w->GV})
+    if ((r = b->need(np))) return r;
+  if (n == 0) return TBSLA_OK;
+  MCK(cudaMemcpyAsync(w->rowptr.p, rp, n1 * 4, cudaMemcpyHostToDevice, st));
+  MCK(cudaMemcpyAsync(w->colidx.p, mat->idx1.data() + base, nnz * 4, cudaMemcpyHostToDevice, st));
+  MCK(cudaMemcpyAsync(w->a64.p, mat->values.data() + base, nnz * 8, cudaMemcpyHostToDevice, st));
+  const int gr = row_grid(n);
+  unsigned* lcount = reinterpret_cast<unsigned*>(w->lrowptr.p);
+  unsigned* tcount = reinterpret_cast<unsigned*>(w->trowptr.p);
+  MCK(cudaMemsetAsync(w->check.p, 0, sizeof(GraphCheck), st));
+  MCK(cudaMemsetAsync(tcount, 0, n1 * sizeof(unsigned), st));
+  MCK(cudaMemsetAsync(lcount + n, 0, sizeof(unsigned), st));
+  k_graph_rows<<<gr, NT, 0, st>>>(n, base, w->rowptr.p, w->colidx.p, w->a64.p, w->aval.p, w->s.p, lcount, tcount,
+                                  w->check.p);
+  MCK(cudaGetLastError());
+  if (base) k_shift<<<gr, NT, 0, st>>>(n + 1, base, w->rowptr.p);
+  MCK(tbsla_gpu::exclusive_scan(lcount, (long)n1, w->scratch.p, st));
+  MCK(tbsla_gpu::exclusive_scan(tcount, (long)n1, w->scratch.p, st));
+  GraphCheck check{};
+  int nl = 0;
+  MCK(cudaMemcpyAsync(&check, w->check.p, sizeof check, cudaMemcpyDeviceToHost, st));
+  MCK(cudaMemcpyAsync(&nl, w->lrowptr.p + n, sizeof(int), cudaMemcpyDeviceToHost, st));
+  MCK(cudaStreamSynchronize(st));
+  if (check.bad_col || check.bad_diag) return TBSLA_ERR_BAD_MATRIX;
+  w->nl = nl;
+  // L^T's lists, each in L's order: put in place in any order and ordered
+  // there when every column is short (48^3 nodes: 21 us with the fill, against
+  // about 150 us for the stable sort by column that the others take)
+  const bool in_place = check.max_col <= kShortCol;
+  if ((r = w->lcol.need(nl)) || (r = w->lsrc.need(nl)) || (r = w->lrow.need(nl)) || (r = w->tidx.need(nl)) ||
+      (r = w->lval.need(nl)) || (r = w->dl.need(nl)))
+    return r;
+  if (!in_place && ((r = w->tidx2.need(nl)) || (r = w->keys.need(nl)) || (r = w->keys2.need(nl)) ||
+                    (r = w->scratch.need(tbsla_gpu::radix_scratch(nl)))))
+    return r;
+  if (in_place) MCK(cudaMemcpyAsync(w->tnext.p, tcount, n1 * sizeof(unsigned), cudaMemcpyDeviceToDevice, st));
+  k_graph_fill<<<gr, NT, 0, st>>>(n, w->rowptr.p, w->colidx.p, w->aval.p, w->s.p, w->lrowptr.p, w->e.p, w->x.p,
+                                  w->lcol.p, w->lsrc.p, w->lrow.p, in_place ? w->tnext.p : nullptr, w->keys.p,
+                                  w->tidx.p);
+  if (in_place) {
+    k_order_columns<<<gr, NT, 0, st>>>(n, w->trowptr.p, w->tidx.p);
+    MCK(cudaGetLastError());
+    return TBSLA_OK;
+  }
+  MCK(cudaGetLastError());
+  int bits = 1, alt = 0;
+  while (bits < 31 && (1L << bits) < (long)n) bits++;
+  MCK(tbsla_gpu::radix_sort_pairs(w->keys.p, w->keys2.p, w->tidx.p, w->tidx2.p, nl, bits, w->scratch.p, &alt, st));
+  if (alt) std::swap(w->tidx, w->tidx2);
+  return TBSLA_OK;
+}
 // Forward pass: activations and L values.
 int forward(const float* wq, Work& w, cudaStream_t s) {
-  const int n = w.n, gw = warp_grid(n);
-  k_layer0<<<gw, NT, 0, s>>>(n, w.x.p, wq, w.z[0].p, w.h[0].p);
+  const int n = w.n, gw = warp_grid(n), gq = warp_grid(((long)n + NB - 1) / NB);
+  k_layer0<<<gw, NT, 0, s>>>(n, w.x.p, wq, w.mask[0].p, w.h[0].p);
   for (int l = 1; l <= NL; l++) {
-    k_aggregate<<<gw, NT, 0, s>>>(n, w.rowptr.p, w.colidx.p, w.e.p, w.h[l - 1].p, w.m[l].p, 0);
-    k_layer<<<gw, NT, 0, s>>>(n, wq + off_layer(l), w.h[l - 1].p, w.m[l].p, w.z[l].p, w.h[l].p);
+    k_gather<<<gq, NT, 0, s>>>(n, w.rowptr.p, w.colidx.p, w.e.p, w.h[l - 1].p, w.m[l].p, 0);
+    k_layer<<<layer_grid(n, 2), NT, 0, s>>>(n, wq + off_layer(l), w.h[l - 1].p, w.m[l].p, w.mask[l].p, w.h[l].p);
   }
-  k_head<<<gw, NT, 0, s>>>(n, w.lrowptr.p, w.lcol.p, w.lsrc.p, w.e.p, w.s.p, wq, w.h[NL].p, w.lval.p, w.xi.p);
+  k_head<<<gq, NT, 0, s>>>(n, w.lrowptr.p, w.lcol.p, w.lsrc.p, w.e.p, w.s.p, wq, w.h[NL].p, w.lval.p, w.xi.p);
   MCK(cudaGetLastError());
   return TBSLA_OK;
 }
 
 // Loss on the probes in w.Z and the gradient into grad (zeroed here).
 int backward(const float* wq, Work& w, double* dloss, float* grad, cudaStream_t s) {
-  const int n = w.n, P = w.P, gw = warp_grid(n), gr = row_grid(n);
+  const int n = w.n, P = w.P, gw = warp_grid(n), gq = warp_grid(((long)n + NB - 1) / NB);
   const long len = (long)n * P;
-  k_spmm_a<<<gr, NT, 0, s>>>(n, P, w.rowptr.p, w.colidx.p, w.aval.p, w.Z.p, w.U.p);
-  k_spmm_l<<<gr, NT, 0, s>>>(n, P, w.trowptr.p, w.tidx.p, w.lrow.p, w.lval.p, 1, w.U.p, w.V.p);
-  k_spmm_l<<<gr, NT, 0, s>>>(n, P, w.lrowptr.p, nullptr, w.lcol.p, w.lval.p, 0, w.V.p, w.W.p);
+  const int gp = row_grid(len);
+  k_spmm_a<<<gp, NT, 0, s>>>(n, P, w.rowptr.p, w.colidx.p, w.aval.p, w.Z.p, w.U.p);
+  k_spmm_l<<<gp, NT, 0, s>>>(n, P, w.trowptr.p, w.tidx.p, w.lrow.p, w.lval.p, 1, w.U.p, w.V.p);
+  k_spmm_l<<<gp, NT, 0, s>>>(n, P, w.lrowptr.p, nullptr, w.lcol.p, w.lval.p, 0, w.V.p, w.W.p);
   MCK(cudaMemsetAsync(dloss, 0, sizeof(double), s));
-  k_residual<<<row_grid(len), NT, 0, s>>>(len, 1.f / (float)len, w.W.p, w.Z.p, w.G.p, dloss);
-  k_spmm_l<<<gr, NT, 0, s>>>(n, P, w.trowptr.p, w.tidx.p, w.lrow.p, w.lval.p, 1, w.G.p, w.GV.p);
+  k_residual<<<std::min(gp, 152 * 2), NT, 0, s>>>(len, 1.f / (float)len, w.W.p, w.Z.p, w.G.p, dloss);
+  k_spmm_l<<<gp, NT, 0, s>>>(n, P, w.trowptr.p, w.tidx.p, w.lrow.p, w.lval.p, 1, w.G.p, w.GV.p);
   k_dl<<<row_grid(w.nl), NT, 0, s>>>(w.nl, P, w.lrow.p, w.lcol.p, w.G.p, w.V.p, w.U.p, w.GV.p, w.dl.p);
   MCK(cudaMemsetAsync(grad, 0, NPARAMS * sizeof(float), s));
-  k_head_bwd<<<gw, NT, 0, s>>>(n, w.lrowptr.p, w.lcol.p, w.lsrc.p, w.e.p, w.s.p, wq, w.h[NL].p, w.dl.p, w.xi.p,
-                               w.dh.p, grad);
-  k_head_bwd_cols<<<gw, NT, 0, s>>>(n, w.trowptr.p, w.tidx.p, w.lrow.p, w.s.p, wq, w.h[NL].p, w.dl.p, w.dh.p);
+  k_head_bwd<<<std::min(gq, 152 * 6), NT, 0, s>>>(n, w.lrowptr.p, w.lcol.p, w.lsrc.p, w.trowptr.p, w.tidx.p,
+                                                  w.lrow.p, w.e.p, w.s.p, wq, w.h[NL].p, w.dl.p, w.xi.p, w.dh.p,
+                                                  grad);
   for (int l = NL; l >= 1; l--) {
-    k_layer_bwd<<<gw, NT, 0, s>>>(n, wq + off_layer(l), w.h[l - 1].p, w.m[l].p, w.z[l].p, w.dh.p, w.dm.p,
-                                  grad + off_layer(l));
-    k_aggregate<<<gw, NT, 0, s>>>(n, w.rowptr.p, w.colidx.p, w.e.p, w.dm.p, w.dh.p, 1);
+    k_layer_bwd<<<layer_grid(n, 1), NT, 0, s>>>(n, wq + off_layer(l), w.h[l - 1].p, w.m[l].p, w.mask[l].p, w.dh.p,
+                                                w.dm.p, grad + off_layer(l));
+    k_gather<<<gq, NT, 0, s>>>(n, w.rowptr.p, w.colidx.p, w.e.p, w.dm.p, w.dh.p, 1);
   }
-  k_layer0_bwd<<<gw, NT, 0, s>>>(n, w.x.p, w.z[0].p, w.dh.p, grad);
+  k_layer0_bwd<<<std::min(gw, 152 * 4), NT, 0, s>>>(n, w.x.p, w.mask[0].p, w.dh.p, grad);
   MCK(cudaGetLastError());
   return TBSLA_OK;
 }
@@ -936,16 +1322,17 @@ int tbsla_mpnn_set_params(tbsla_mpnn* net, const float* theta, int nparams) try 
 int tbsla_mpnn_loss_grad(tbsla_mpnn* net, const tbsla_matrix* A, int nprobes, const double* Z, double* loss,
                          float* grad) try {
   if (!net || !A || nprobes < 1 || nprobes > PMAX || !Z) return TBSLA_ERR_INVALID_ARG;
-  HostGraph g;
-  int st = build_graph(A, &g);
-  if (st) return st;
   cudaSetDevice(net->device);
   cudaStream_t s = net->stream;
   Work& w = net->work;
-  if ((st = upload(g, nprobes, &w, s))) return st;
-  std::vector<float> zf((size_t)g.n * nprobes);
-  for (size_t k = 0; k < zf.size(); k++) zf[k] = (float)Z[k];
-  MCK(cudaMemcpyAsync(w.Z.p, zf.data(), zf.size() * 4, cudaMemcpyHostToDevice, s));
+  int st = build_graph(A, nprobes, &w, s);
+  if (st) return st;
+  const long len = (long)w.n * nprobes;
+  if (len > 0) {  // the probes in FP32
+    if ((st = w.a64.need(len))) return st;
+    MCK(cudaMemcpyAsync(w.a64.p, Z, len * 8, cudaMemcpyHostToDevice, s));
+    k_narrow<<<row_grid(len), NT, 0, s>>>(len, w.a64.p, w.Z.p);
+  }
   if ((st = forward(net->wq, w, s)) || (st = backward(net->wq, w, net->dloss, net->grad, s))) return st;
   double l = 0;
   MCK(cudaMemcpyAsync(&l, net->dloss, 8, cudaMemcpyDeviceToHost, s));
@@ -958,14 +1345,12 @@ int tbsla_mpnn_loss_grad(tbsla_mpnn* net, const tbsla_matrix* A, int nprobes, co
 int tbsla_mpnn_train_step(tbsla_mpnn* net, const tbsla_matrix* A, int nprobes, unsigned long long seed, float lr,
                           double* loss) try {
   if (!net || !A || nprobes < 1 || nprobes > PMAX || !(lr > 0)) return TBSLA_ERR_INVALID_ARG;
-  HostGraph g;
-  int st = build_graph(A, &g);
-  if (st) return st;
   cudaSetDevice(net->device);
   cudaStream_t s = net->stream;
   Work& w = net->work;
-  if ((st = upload(g, nprobes, &w, s))) return st;
-  const long len = (long)g.n * nprobes;
+  int st = build_graph(A, nprobes, &w, s);
+  if (st) return st;
+  const long len = (long)w.n * nprobes;
   k_gauss<<<row_grid(len), NT, 0, s>>>(len, seed, w.Z.p);
   if ((st = forward(net->wq, w, s)) || (st = backward(net->wq, w, net->dloss, net->grad, s))) return st;
   net->step++;
@@ -982,22 +1367,25 @@ int tbsla_mpnn_train_step(tbsla_mpnn* net, const tbsla_matrix* A, int nprobes, u
 
 int tbsla_mpnn_factor(tbsla_mpnn* net, const tbsla_matrix* A, tbsla_matrix* L) try {
   if (!net || !A || !L || L->format != TBSLA_CSR) return TBSLA_ERR_INVALID_ARG;
-  HostGraph g;
-  int st = build_graph(A, &g);
-  if (st) return st;
   cudaSetDevice(net->device);
   cudaStream_t s = net->stream;
   Work& w = net->work;
-  if ((st = upload(g, 1, &w, s)) || (st = forward(net->wq, w, s))) return st;
+  int st = build_graph(A, 1, &w, s);
+  if (st || (st = forward(net->wq, w, s))) return st;
   std::vector<float> lv(w.nl);
-  MCK(cudaMemcpyAsync(lv.data(), w.lval.p, w.nl * 4, cudaMemcpyDeviceToHost, s));
+  std::vector<int> lrp(w.n + 1, 0), lci(w.nl);
+  if (w.n > 0) {
+    MCK(cudaMemcpyAsync(lv.data(), w.lval.p, w.nl * 4, cudaMemcpyDeviceToHost, s));
+    MCK(cudaMemcpyAsync(lrp.data(), w.lrowptr.p, lrp.size() * 4, cudaMemcpyDeviceToHost, s));
+    MCK(cudaMemcpyAsync(lci.data(), w.lcol.p, w.nl * 4, cudaMemcpyDeviceToHost, s));
+  }
   MCK(cudaStreamSynchronize(s));
   std::vector<double> vals(lv.begin(), lv.end());
   tbsla_info I{};
-  I.n_row = I.n_col = I.ln_row = I.ln_col = g.n;
+  I.n_row = I.n_col = I.ln_row = I.ln_col = w.n;
   I.nnz = w.nl;
   I.NR = I.NC = 1;
-  return tbsla_matrix_set_csr(L, &I, vals.data(), g.lrowptr.data(), g.lcol.data());
+  return tbsla_matrix_set_csr(L, &I, vals.data(), lrp.data(), lci.data());
 } TBSLA_API_CATCH
 
 }  // extern "C"
