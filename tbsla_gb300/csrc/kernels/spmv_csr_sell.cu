@@ -47,7 +47,7 @@ constexpr unsigned FULL = 0xffffffffu;
 
 // K steps of one lane's row: predicated loads (lanes past their row's end
 // issue none, so padding costs no traffic), the K gathers of x in flight
-// together, then K full-warp DFMAs (dead lanes add 0 * 0).
+// together, then K full-warp DFMAs (dead lanes add a finite value times 0).
 template <class V, int K>
 __device__ __forceinline__ double steps_k(const V* __restrict__ sv, const int* __restrict__ sc, long off, int j,
                                           int steps, const double* __restrict__ x, int f_col, uint64_t pol,
@@ -56,7 +56,7 @@ __device__ __forceinline__ double steps_k(const V* __restrict__ sv, const int* _
   int c[K];
 #pragma unroll
   for (int u = 0; u < K; u++) {
-    v[u] = V(0.0f);
+    v[u] = V(sizeof(V) == 8 ? 0.0f : 1.0f);  // any finite value; 1 keeps narrow ones on widen()'s short path
     c[u] = f_col;
   }
 #pragma unroll
@@ -218,7 +218,10 @@ __device__ __forceinline__ bool cut_row_done(const SellPlan& p, int piece, int l
 // solve adds its terms in the same order.  The FP64 operations of the
 // epilogue then overlap the gathers of x instead of running in a pass of
 // their own that GB300's FP64 pipe bounds.
-template <class V, int U, bool PR>
+//
+// CUT: the plan has cut rows (their test alone costs one without them 0.3%:
+// 1.208 against 1.204 ms at n = 2^24).
+template <class V, int U, bool PR, bool CUT>
 __global__ void __launch_bounds__(NT) k_sell(SellPlan p, const V* __restrict__ sv, const int* __restrict__ sc,
                                             int f_col, int accumulate, const double* __restrict__ x,
                                             double* __restrict__ y, unsigned* __restrict__ counter,
@@ -272,7 +275,7 @@ __global__ void __launch_bounds__(NT) k_sell(SellPlan p, const V* __restrict__ s
     const double y0 = (!PR && accumulate && head) ? y[l.row] : 0.0;  // issued before the sum
     double acc = slice_rows<V, U>(sv, sc, (long)d.x * 32 + lane, l.steps, d.y, x, f_col, pol);
     for (int o = (1 << d.z) >> 1; o > 0; o >>= 1) acc = add_rn(acc, __shfl_xor_sync(FULL, acc, o));
-    if (d.w < -1) {  // a piece of a cut row
+    if (CUT && d.w < -1) {  // a piece of a cut row
       const int piece = -2 - d.w;
       head = cut_row_done(p, piece, lane, acc) && lane == 0;
       if constexpr (PR) {
@@ -361,7 +364,7 @@ cudaError_t launch(const SellArgs& a, const double* x, double* y, unsigned* coun
   int dev = 0, sms = 0, per = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_sell<V, U, false>, NT, 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_sell<V, U, false, true>, NT, 0);
   const int grid = std::max(1, sms * std::max(1, per));
   const bool fork = a.side && a.parts > 1 && a.nblocks >= a.parts;
   const int first_part = a.nblocks - a.parts;
@@ -378,8 +381,9 @@ cudaError_t launch(const SellArgs& a, const double* x, double* y, unsigned* coun
     if (e == cudaSuccess && k > 0) e = cudaStreamWaitEvent(ls, a.fork, 0);
     if (e == cudaSuccess && a.ready && b > 0) e = cudaStreamWaitEvent(ls, a.ready[b], 0);
     if (e == cudaSuccess && p.nslices > 0) {
-      k_sell<V, U, false><<<pg, NT, 0, ls>>>(p, static_cast<const V*>(a.svals), a.scols, a.f_col, b > 0 ? 1 : 0,
-                                             x, y, counter + k * kSellCounterRegion, done, PageRankArgs{}, Ctl{});
+      const auto kernel = p.ncut > 0 ? k_sell<V, U, false, true> : k_sell<V, U, false, false>;
+      kernel<<<pg, NT, 0, ls>>>(p, static_cast<const V*>(a.svals), a.scols, a.f_col, b > 0 ? 1 : 0, x, y,
+                                counter + k * kSellCounterRegion, done, PageRankArgs{}, Ctl{});
       e = cudaGetLastError();
     }
     // recorded for an empty plan too: the event then marks the earlier plans
@@ -418,10 +422,10 @@ cudaError_t launch_pr(const SellArgs& a, const double* x, double* y, const PageR
   int dev = 0, sms = 0, per = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_sell<V, U, true>, NT, 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_sell<V, U, true, true>, NT, 0);
   const SellPlan& p = a.blocks[0];
   const int grid = std::max(1, std::min(sms * std::max(1, std::min(per, 8)), (p.nslices + NT / 32 - 1) / (NT / 32)));
-  k_sell<V, U, true><<<grid, NT, 0, s>>>(p, static_cast<const V*>(a.svals), a.scols, a.f_col, 0, x, y, nullptr,
+  k_sell<V, U, true, true><<<grid, NT, 0, s>>>(p, static_cast<const V*>(a.svals), a.scols, a.f_col, 0, x, y, nullptr,
                                          pr.done, pr, ctl);
   return cudaGetLastError();
 }
