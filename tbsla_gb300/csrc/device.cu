@@ -124,7 +124,7 @@ struct DeviceMatrix {
   size_t t_len = 0;
   bool dense_df = false;     // DENSE, every value within the double-float range (any precision)
   float* xdf = nullptr;      // DENSE double-float: x split into xh[ln_col], xl[ln_col]
-  int* df_flag = nullptr;    // DENSE double-float: x out of range in this call
+  int* df_flag = nullptr;    // DENSE double-float: kDenseFlags flags, x out of range in this call
   double* pr_ctl = nullptr;  // PageRank: coefficients [0, 4) and flags (2 int) at [4]
   size_t pr_ctl_len = 0;
   // persistent-kernel control and reduction scratch
@@ -508,7 +508,7 @@ int build(const tbsla_matrix* m, DeviceMatrix* d) {
       if (st) return st;
       // the double-float GEMV when every value is in its range (FP64 values
       // split on load into two floats; FP32 / BF16 values exact in one)
-      if ((st = dalloc(&d->df_flag, 1))) return st;
+      if ((st = dalloc(&d->df_flag, kDenseFlags))) return st;
       bool ok = false;
       TRY(dense_values_df_range(d->vals, d->prec, n, d->df_flag, &ok, d->stream));
       if (ok) {
@@ -516,7 +516,7 @@ int build(const tbsla_matrix* m, DeviceMatrix* d) {
           cudaGetLastError();
           return TBSLA_ERR_ALLOC;
         }
-        d->bytes += (size_t)I.ln_col * 2 * sizeof(float) + 4;
+        d->bytes += (size_t)I.ln_col * 2 * sizeof(float) + kDenseFlags * 4;
         d->dense_df = true;
       }
       return TBSLA_OK;
@@ -583,10 +583,13 @@ CsrArgs csr_args(const tbsla_matrix* m, DeviceMatrix* d) {
   return a;
 }
 
-// r (device) op= A v (device) on stream s, following the format's Ax semantics.
+// r (device) op= A v (device) on stream s, following the format's Ax semantics;
+// `zero_first`: into a zeroed r (which DENSE's kernels then need not read).
 int ax_device(const tbsla_matrix* m, DeviceMatrix* d, double* r, const double* v, int vect_incr,
-              cudaStream_t s) {
+              cudaStream_t s, bool zero_first = false) {
   const tbsla_info& I = m->info;
+  const bool fresh = zero_first && d->dense_df && !skips_empty(m);
+  if (zero_first && !fresh) TRY(cudaMemsetAsync(r, 0, out_len(m) * sizeof(double), s));
   if (skips_empty(m)) return TBSLA_OK;
   switch (m->format) {
     case TBSLA_CSR:
@@ -613,7 +616,7 @@ int ax_device(const tbsla_matrix* m, DeviceMatrix* d, double* r, const double* v
     }
     case TBSLA_DENSE:
       if (d->dense_df)
-        return status_of(dense_gemv_df(d->vals, d->prec, I.ln_row, I.ln_col, v, d->xdf, d->df_flag, r, s));
+        return status_of(dense_gemv_df(d->vals, d->prec, I.ln_row, I.ln_col, v, d->xdf, d->df_flag, r, fresh, s));
       return status_of(dense_gemv(d->vals, d->prec, I.ln_row, I.ln_col, v, r, s));
   }
   return TBSLA_ERR_INVALID_ARG;
@@ -721,8 +724,7 @@ int dev_ax(const tbsla_matrix* m, double* r, const double* v, int vect_incr, boo
   if (st) return st;
   if (!host) {
     cudaStream_t s = stream ? (cudaStream_t)stream : d->stream;
-    if (zero_first) TRY(cudaMemsetAsync(r, 0, out_len(m) * sizeof(double), s));
-    return ax_device(m, d, r, v, vect_incr, s);
+    return ax_device(m, d, r, v, vect_incr, s, zero_first);
   }
   if (!zero_first && skips_empty(m)) return TBSLA_OK;
   size_t nx = in_len(m), ny = out_len(m);
@@ -731,9 +733,9 @@ int dev_ax(const tbsla_matrix* m, double* r, const double* v, int vect_incr, boo
   if (m->format == TBSLA_CSR && d->algo == 2 && d->sell.size() > 1 && nx && !skips_empty(m))
     return ax_host_blocks(m, d, r, v, vect_incr, zero_first);
   if (nx) TRY(cudaMemcpyAsync(d->x, v, nx * sizeof(double), cudaMemcpyHostToDevice, s));
-  if (zero_first) TRY(cudaMemsetAsync(d->y, 0, ny * sizeof(double), s));
-  else if (accumulates(m->format) && ny) TRY(cudaMemcpyAsync(d->y, r, ny * sizeof(double), cudaMemcpyHostToDevice, s));
-  st = ax_device(m, d, d->y, d->x, vect_incr, s);
+  if (!zero_first && accumulates(m->format) && ny)
+    TRY(cudaMemcpyAsync(d->y, r, ny * sizeof(double), cudaMemcpyHostToDevice, s));
+  st = ax_device(m, d, d->y, d->x, vect_incr, s, zero_first);
   if (st) return st;
   if (ny) TRY(cudaMemcpyAsync(r, d->y, ny * sizeof(double), cudaMemcpyDeviceToHost, s));
   return status_of(cudaStreamSynchronize(s));

@@ -23,11 +23,6 @@ namespace {
 
 constexpr int NT = 256;
 constexpr int kDenseU = 4;  // 16-byte loads in flight per thread, CTA-per-row kernel
-// rows per CTA pass, double-float kernel; 2 (each xh / xl load serving two
-// rows) measured 0.366 / 0.329 ms against 0.362 / 0.321 ms with 1 (FP32 /
-// BF16 values, 32768 x 16384)
-constexpr int kDenseDfRows = 1;
-
 __device__ __forceinline__ double2 ld_stream2(const double* p, uint64_t pol) {
   double2 v;
   asm volatile("ld.global.nc.L1::no_allocate.L2::cache_hint.v2.f64 {%0, %1}, [%2], %3;"
@@ -113,26 +108,30 @@ __global__ void __launch_bounds__(NT) k_dense_rows_f64x2(const double* __restric
   }
 }
 
-// FP32 / BF16 values in double-float arithmetic.  Widening every value to
-// FP64 for one FP64 multiply-add kept the FP64 pipe as busy as the FP64
-// matrix does (0.99 ms for 537 M entries) although the bytes halve.  Here:
+// Values in double-float arithmetic.  Widening every value to FP64 for one
+// FP64 multiply-add kept the FP64 pipe as busy as the FP64 matrix does (0.99 ms
+// for 537 M entries) although the bytes halve.  Here:
 //  * x is split once per call into floats xh = fl32(x), xl = fl32(x - xh),
 //    which hold x to 2^-48 relative, kept as two arrays;
-//  * each thread accumulates its columns with compensated Dot2 steps (the
-//    product's and the sum's rounding errors carried exactly into a second
-//    float), 4 columns per step: one load of values (16 bytes FP32, 8 bytes
-//    BF16) and one 16-byte load each of xh and xl, consecutive across the
-//    warp;
-//  * the thread pairs are summed across the warp in double-float (TwoSum-
-//    based additions), and the NT/32 warp values in FP64, in a fixed order
-//    (keeping the warp values in double-float up to one conversion per row,
-//    so that fewer FP64 instructions occupy the pipe, measured 2-6% slower).
+//  * a warp takes R rows and a part of the columns, 128 (BF16: 256) columns a
+//    step: each lane loads 16 bytes of every row (FP64: 32, in one go where the
+//    rows are aligned for it) and their xh / xl, which serve all R rows, and
+//    adds them with compensated Dot2 steps (the product's and the sum's
+//    rounding errors carried exactly into a second float);
+//  * the lanes' pairs are summed across the warp in double-float (TwoSum-
+//    based additions), the R rows at once (each half of the warp goes on with
+//    half of the rows), and the column parts in FP64, in a fixed order.
+// Bound: HBM for FP64 and FP32 values (16384 x 8192: 165 and 101 us, 6.5 and
+// 5.3 TB/s with the launches), instruction issue (about 15 per entry) for BF16
+// (24576 x 8192: 109 us).  With a CTA per row, one row's x loads, its warp
+// reductions and a barrier came to more instructions than the entries
+// themselves: 177, 122 and 164 us, and 65 us for 9000 x 600 FP32, now 12.4.
 // The float arithmetic is exact only inside the float exponent range, so the
 // path needs every nonzero |x| and |a| in [2^-40, 2^40] (products within
 // [2^-80, 2^80], sums of up to 2^31 of them finite, error terms normal): the
 // values are checked once at upload, x by the split kernel on every call,
-// which sets *bad; a launch that reads *bad set runs every row in FP64, in the
-// same kernel (no host round trip).
+// whose CTAs leave a flag each; a launch that reads a set flag runs every row
+// in FP64, in the same kernel (no host round trip).
 constexpr float kDfLo = 9.094947017729282e-13f;  // 2^-40
 constexpr float kDfHi = 1.099511627776e12f;      // 2^40
 
@@ -142,18 +141,19 @@ __device__ __forceinline__ bool df_in_range(double v) {
 }
 
 // xs[0, n) = xh, xs[n, 2n) = xl: separate arrays, so that the GEMV's lanes
-// read consecutive words of each.
-__global__ void k_df_split_x(const double* __restrict__ x, int n, float* __restrict__ xs,
-                             int* __restrict__ bad) {
+// read consecutive words of each.  bad[CTA]: x leaves the range there.
+__global__ void __launch_bounds__(NT) k_df_split_x(const double* __restrict__ x, int n, float* __restrict__ xs,
+                                                  int* __restrict__ bad) {
   int any = 0;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+  for (int i = blockIdx.x * NT + threadIdx.x; i < n; i += gridDim.x * NT) {
     const double v = x[i];
     const float h = __double2float_rn(v);
     xs[i] = h;
     xs[n + i] = __double2float_rn(v - (double)h);
     any |= !df_in_range(v);
   }
-  if (__any_sync(0xffffffffu, any) && threadIdx.x % kWarp == 0) atomicOr(bad, 1);
+  any = __syncthreads_or(any);
+  if (threadIdx.x == 0) bad[blockIdx.x] = any;
 }
 
 template <class V>
@@ -165,151 +165,242 @@ __global__ void k_df_range_vals(const V* __restrict__ a, size_t n, int* __restri
 }
 
 // An FP64 value a = h + l split into two floats on the integer pipe: h is a
-// truncated to its 24 leading significand bits (exact), l the float nearest
-// to the rest a - h (29 bits, exact in FP64, rounded to 24: a is held to
-// about 2^-48 relative).  For a == 0 or |a| in [2^-74, 2^128); the values
-// reaching it passed the [2^-40, 2^40] check.  No FP64 instruction.
+// rounded to 24 significand bits (half away from zero; a carry moves into the
+// exponent by itself), l the float nearest to the rest a - h (at most 2^28 in
+// units of a's last bit, so a is held to 2^-49 relative).  For a == 0 or |a| in
+// [2^-60, 2^60]; the values reaching it passed the [2^-40, 2^40] check.  No
+// FP64 instruction.
 __device__ __forceinline__ void split_f64(double a, float& h, float& l) {
-  const unsigned long long b = (unsigned long long)__double_as_longlong(a);
-  const unsigned hi = (unsigned)(b >> 32), lo = (unsigned)b;
-  const unsigned sign = hi & 0x80000000u;
-  const int e = (int)((hi >> 20) & 0x7ffu);
-  if (e == 0) {
-    h = l = 0.f;
+  const unsigned hi = (unsigned)__double2hiint(a), lo = (unsigned)__double2loint(a);
+  // the low 8 bits of the exponent and the leading 23 of the mantissa; a
+  // float's exponent is e - 896, whose low 8 bits are e's with the top one
+  // flipped
+  const unsigned top = __funnelshift_l(lo, hi, 3) ^ 0x40000000u;
+  const unsigned t = (hi & 0x80000000u) | (top & 0x7fffffffu);
+  h = (hi & 0x7ff00000u) == 0u ? 0.f : __uint_as_float(t + (lo >> 28 & 1u));
+  // the last 29 bits as a signed number (0 for a == 0), times +- 2^(e - 1075)
+  const float scale = __uint_as_float((t & 0xff800000u) - (52u << 23));
+  l = __fmul_rn(__int2float_rn((int)(lo << 3) >> 3), scale);
+}
+
+// A step is 32 * NV columns; one lane's NV values of a row's step, as loaded:
+// 16 bytes (FP64: 32).  VEC: columns c .. c + NV - 1, the row aligned for it;
+// else columns c, c + 32, ...  A column past the row's last one (`last`: its
+// index, VEC its last vector's) is read at `last` instead and meets a zero of
+// x.
+template <class V, bool VEC>
+struct Step;
+template <bool VEC>
+struct Step<double, VEC> {
+  static constexpr int NV = 4;
+  double v[NV];
+  __device__ __forceinline__ void load(const double* p, int c, int last, uint64_t pol) {
+    if constexpr (VEC) {
+      p += min(c, last);
+      asm volatile("ld.global.nc.L1::no_allocate.L2::cache_hint.v2.f64 {%0, %1}, [%2], %3;"
+                   : "=d"(v[0]), "=d"(v[1]) : "l"(p), "l"(pol));
+      asm volatile("ld.global.nc.L1::no_allocate.L2::cache_hint.v2.f64 {%0, %1}, [%2], %3;"
+                   : "=d"(v[2]), "=d"(v[3]) : "l"(p + 2), "l"(pol));
+    } else {
+#pragma unroll
+      for (int k = 0; k < NV; k++) v[k] = ld_stream(p + min(c + 32 * k, last), pol);
+    }
+  }
+  // a = h + l: Dot2 on h (x as xh + xl), then l * xh into the error term
+  // (l * xl is below 2^-48 of the product)
+  __device__ __forceinline__ void add(float& s, float& c, int k, float xh, float xl) const {
+    float h, l;
+    split_f64(v[k], h, l);
+    dot2_step(s, c, h, DF{xh, xl});
+    c = __fmaf_rn(l, xh, c);
+  }
+};
+template <bool VEC>
+struct Step<float, VEC> {
+  static constexpr int NV = 4;
+  float v[NV];
+  __device__ __forceinline__ void load(const float* p, int c, int last, uint64_t pol) {
+    if constexpr (VEC) {
+      asm volatile("ld.global.nc.L1::no_allocate.L2::cache_hint.v4.f32 {%0, %1, %2, %3}, [%4], %5;"
+                   : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]) : "l"(p + min(c, last)), "l"(pol));
+    } else {
+#pragma unroll
+      for (int k = 0; k < NV; k++) v[k] = ld_stream(p + min(c + 32 * k, last), pol);
+    }
+  }
+  __device__ __forceinline__ void add(float& s, float& c, int k, float xh, float xl) const {
+    dot2_step(s, c, v[k], DF{xh, xl});
+  }
+};
+template <bool VEC>
+struct Step<__nv_bfloat16, VEC> {  // a bfloat16 is the high half of its float; VEC: two values a word
+  static constexpr int NV = 8;
+  unsigned v[VEC ? NV / 2 : NV];
+  __device__ __forceinline__ void load(const __nv_bfloat16* p, int c, int last, uint64_t pol) {
+    if constexpr (VEC) {
+      asm volatile("ld.global.nc.L1::no_allocate.L2::cache_hint.v4.u32 {%0, %1, %2, %3}, [%4], %5;"
+                   : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "l"(p + min(c, last)), "l"(pol));
+    } else {
+#pragma unroll
+      for (int k = 0; k < NV; k++) {
+        const __nv_bfloat16 b = ld_stream(p + min(c + 32 * k, last), pol);
+        v[k] = *reinterpret_cast<const unsigned short*>(&b);
+      }
+    }
+  }
+  __device__ __forceinline__ void add(float& s, float& c, int k, float xh, float xl) const {
+    unsigned w;
+    if constexpr (!VEC) w = v[k] << 16;
+    else w = k & 1 ? v[k >> 1] & 0xffff0000u : v[k >> 1] << 16;
+    dot2_step(s, c, __uint_as_float(w), DF{xh, xl});
+  }
+};
+
+// The warp's sums of R values per lane: the halves of the warp go on with half
+// of the values each until one is left, which the remaining lanes add up.
+// Lanes [r * 32 / R, (r + 1) * 32 / R) get value r.
+template <int R>
+__device__ __forceinline__ DF warp_sum_rows(DF (&t)[R]) {
+  int o = 16;
+#pragma unroll
+  for (int n = R; n > 1; n /= 2, o /= 2) {
+    const bool up = threadIdx.x & o;
+#pragma unroll
+    for (int i = 0; i < n / 2; i++) {
+      const DF keep = up ? t[i + n / 2] : t[i], give = up ? t[i] : t[i + n / 2];
+      t[i] = df_add(keep, DF{__shfl_xor_sync(0xffffffffu, give.h, o), __shfl_xor_sync(0xffffffffu, give.l, o)});
+    }
+  }
+#pragma unroll
+  for (; o > 0; o /= 2)
+    t[0] = df_add(t[0], DF{__shfl_xor_sync(0xffffffffu, t[0].h, o), __shfl_xor_sync(0xffffffffu, t[0].l, o)});
+  return t[0];
+}
+
+// y += A x (fresh: y = A x).  The CTA's eight warps are 8 / S groups of R rows
+// times S = 1 << log2s parts of the columns (steps part, part + S, ...).  The
+// values of two steps are loaded, then used: 32 warps on an SM (64 registers)
+// keep as many loads in flight as 24 that load a step ahead (80 registers: BF16
+// 117, FP32 98, FP64 193 us where 109, 101 and 185 were taken then).
+template <class V, int R, bool VEC>
+__global__ void __launch_bounds__(NT, 4) k_dense_df(const V* __restrict__ A, int ln_row, int ln_col, int log2s,
+                                                   const float* __restrict__ xs, const double* __restrict__ x,
+                                                   const int* __restrict__ bad, int nbad, double* __restrict__ y,
+                                                   int fresh) {
+  constexpr int NV = Step<V, VEC>::NV, SC = 32 * NV, NW = NT / kWarp;
+  __shared__ double s_part[NW][R];
+  const int lane = threadIdx.x % kWarp, warp = threadIdx.x / kWarp;
+  const int S = 1 << log2s, part = warp & (S - 1);
+  const long row0 = (((long)blockIdx.x * NW + warp) >> log2s) * R;
+  const uint64_t pol = policy_evict_first();
+  const int nsteps = (ln_col + SC - 1) / SC;
+  // rows past the last one repeat it; their sums are not stored
+  const V* const a0 = A + (size_t)min(row0, (long)ln_row - 1) * ln_col;
+  const int rows = (int)min((long)R, max(1L, ln_row - row0));
+  auto row_at = [&](int r) { return a0 + (size_t)min(r, rows - 1) * ln_col; };
+  int out = 0;  // x out of the range somewhere (looked at when the flags are there: after the sums)
+  for (int k = lane; k < nbad; k += kWarp) out |= bad[k];
+  // (sh, sc): the Dot2 sum of one step (FP32) or two of a lane, then folded
+  // into (th, tl): the rounding of the carried errors grows with the entries
+  // of one sum
+  float sh[R], sc[R], th[R], tl[R];
+#pragma unroll
+  for (int r = 0; r < R; r++) sh[r] = sc[r] = th[r] = tl[r] = 0.f;
+  auto fold = [&]() {
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+      const DF t = two_sum(th[r], sh[r]);
+      th[r] = t.h;
+      tl[r] = __fadd_rn(tl[r], __fadd_rn(t.l, sc[r]));
+      if constexpr (sizeof(V) != 8) {  // keeps tl small against th
+        const DF u = fast_two_sum(th[r], tl[r]);
+        th[r] = u.h;
+        tl[r] = u.l;
+      }
+      sh[r] = sc[r] = 0.f;
+    }
+  };
+  const int last = ln_col - (VEC ? NV : 1), c0 = VEC ? NV * lane : lane;
+  auto load = [&](Step<V, VEC>(&f)[R], int st) {
+#pragma unroll
+    for (int r = 0; r < R; r++) f[r].load(row_at(r), st * SC + c0, last, pol);
+  };
+  auto add = [&](const Step<V, VEC>(&f)[R], int st) {
+    const int c = st * SC + c0;
+#pragma unroll
+    for (int k0 = 0; k0 < NV; k0 += 4) {
+      float xh[4], xl[4];
+      if constexpr (VEC) {
+        const int cc = min(c, last) + k0;
+        const float4 h4 = __ldg(reinterpret_cast<const float4*>(xs + cc));
+        const float4 l4 = __ldg(reinterpret_cast<const float4*>(xs + ln_col + cc));
+        xh[0] = h4.x; xh[1] = h4.y; xh[2] = h4.z; xh[3] = h4.w;
+        xl[0] = l4.x; xl[1] = l4.y; xl[2] = l4.z; xl[3] = l4.w;
+      } else {
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+          const int cc = min(c + 32 * (k0 + k), last);
+          xh[k] = __ldg(xs + cc);
+          xl[k] = __ldg(xs + ln_col + cc);
+        }
+      }
+      if (st == nsteps - 1) {
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+          if ((VEC ? c : c + 32 * (k0 + k)) > last) xh[k] = xl[k] = 0.f;
+      }
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+#pragma unroll
+        for (int r = 0; r < R; r++) f[r].add(sh[r], sc[r], k0 + k, xh[k], xl[k]);
+      }
+    }
+  };
+  int st = part;
+  for (; st + S < nsteps; st += 2 * S) {
+    Step<V, VEC> f0[R], f1[R];
+    load(f0, st);
+    load(f1, st + S);
+    add(f0, st);
+    if constexpr (sizeof(V) == 4) fold();
+    add(f1, st + S);
+    fold();
+  }
+  if (st < nsteps) {
+    Step<V, VEC> f0[R];
+    load(f0, st);
+    add(f0, st);
+  }
+  fold();
+  DF t[R];
+#pragma unroll
+  for (int r = 0; r < R; r++) t[r] = two_sum(th[r], tl[r]);
+  double mine = df_val(warp_sum_rows<R>(t));  // the sum of row lane / (32 / R)
+  if (__any_sync(0xffffffffu, out)) {
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+      double acc = 0;
+      for (int st = part; st < nsteps; st += S)
+        for (int j = st * SC + lane; j < min(st * SC + SC, ln_col); j += kWarp)
+          acc = fma_rn(widen(ld_stream(row_at(r) + j, pol)), __ldg(x + j), acc);
+      acc = warp_sum(acc);
+      if (lane / (kWarp / R) == r) mine = acc;
+    }
+  }
+  const int r = lane / (kWarp / R);
+  const bool head = lane % (kWarp / R) == 0;
+  if (S == 1) {
+    if (head && row0 + r < ln_row) y[row0 + r] = add_rn(fresh ? 0.0 : y[row0 + r], mine);
     return;
   }
-  h = __uint_as_float(sign | ((unsigned)(e - 896) << 23) | ((hi & 0xfffffu) << 3) | (lo >> 29));
-  const float scale = __uint_as_float((unsigned)(e - 948) << 23);  // 2^(e - 1075)
-  const float r = __fmul_rn(__uint2float_rn(lo & 0x1fffffffu), scale);
-  l = sign ? -r : r;
-}
-
-// Values of one lane: out[k] (+ outl[k], the low parts of FP64 values).
-template <class V, int VEC>
-__device__ __forceinline__ void ld_vals_dd(float (&out)[VEC], float (&outl)[VEC], const V* p, uint64_t pol) {
-  static_assert(sizeof(V) == 8, "FP64 values");
-  if constexpr (VEC == 1) {
-    split_f64(ld_stream(reinterpret_cast<const double*>(p), pol), out[0], outl[0]);
-  } else {
-    static_assert(VEC == 4, "four values per lane");
-    double v[4];
-    asm volatile("ld.global.nc.L1::no_allocate.L2::cache_hint.v2.f64 {%0, %1}, [%2], %3;"
-                 : "=d"(v[0]), "=d"(v[1]) : "l"(p), "l"(pol));
-    asm volatile("ld.global.nc.L1::no_allocate.L2::cache_hint.v2.f64 {%0, %1}, [%2], %3;"
-                 : "=d"(v[2]), "=d"(v[3]) : "l"(reinterpret_cast<const double*>(p) + 2), "l"(pol));
-#pragma unroll
-    for (int k = 0; k < 4; k++) split_f64(v[k], out[k], outl[k]);
-  }
-}
-
-template <class V, int VEC>
-__device__ __forceinline__ void ld_vals(float (&out)[VEC], const V* p, uint64_t pol) {
-  if constexpr (VEC == 1) {
-    if constexpr (sizeof(V) == 4) {
-      out[0] = ld_stream(reinterpret_cast<const float*>(p), pol);
-    } else {  // bfloat16: the high 16 bits of a float
-      const __nv_bfloat16 b = ld_stream(reinterpret_cast<const __nv_bfloat16*>(p), pol);
-      out[0] = __uint_as_float((unsigned)*reinterpret_cast<const unsigned short*>(&b) << 16);
-    }
-  } else if constexpr (sizeof(V) == 4) {  // 4 floats: one 16-byte load
-    static_assert(VEC == 4, "four values per lane");
-    uint4 w;
-    asm volatile("ld.global.nc.L1::no_allocate.L2::cache_hint.v4.u32 {%0, %1, %2, %3}, [%4], %5;"
-                 : "=r"(w.x), "=r"(w.y), "=r"(w.z), "=r"(w.w) : "l"(p), "l"(pol));
-    out[0] = __uint_as_float(w.x); out[1] = __uint_as_float(w.y);
-    out[2] = __uint_as_float(w.z); out[3] = __uint_as_float(w.w);
-  } else {  // 4 bfloat16 (the high 16 bits of a float): one 8-byte load
-    static_assert(VEC == 4, "four values per lane");
-    unsigned u0, u1;
-    asm volatile("ld.global.nc.L1::no_allocate.L2::cache_hint.v2.u32 {%0, %1}, [%2], %3;"
-                 : "=r"(u0), "=r"(u1) : "l"(p), "l"(pol));
-    out[0] = __uint_as_float(u0 << 16); out[1] = __uint_as_float(u0 & 0xffff0000u);
-    out[2] = __uint_as_float(u1 << 16); out[3] = __uint_as_float(u1 & 0xffff0000u);
-  }
-}
-
-template <class V, int VEC, int R>
-__global__ void __launch_bounds__(NT) k_dense_rows_df(const V* __restrict__ A, int ln_row, int ln_col,
-                                                     const float* __restrict__ xs,
-                                                     const double* __restrict__ x,
-                                                     const int* __restrict__ bad, double* __restrict__ y) {
-  __shared__ double s_part[2][R][NT / kWarp];
-  const int lane = threadIdx.x % kWarp, warp = threadIdx.x / kWarp;
-  const uint64_t pol = policy_evict_first();
-  const bool fp64 = *bad != 0;
-  const int groups = ln_col / VEC;  // VEC divides ln_col
-  int parity = 0;
-  // R rows per pass share every load of xh / xl
-  for (int row0 = blockIdx.x * R; row0 < ln_row; row0 += gridDim.x * R, parity ^= 1) {
-    const int nr = min(R, ln_row - row0);
-    double w[R];
-    if (fp64) {
-#pragma unroll
-      for (int r = 0; r < R; r++) {
-        double acc = 0;
-        if (r < nr) {
-          const V* a = A + (size_t)(row0 + r) * ln_col;
-          for (int j = threadIdx.x; j < ln_col; j += NT) acc = fma_rn(widen(ld_stream(a + j, pol)), __ldg(x + j), acc);
-        }
-        w[r] = warp_sum(acc);
-      }
-    } else {
-      float sh[R], sc[R];
-#pragma unroll
-      for (int r = 0; r < R; r++) sh[r] = sc[r] = 0.f;
-      for (int g = threadIdx.x; g < groups; g += NT) {
-        float xh[VEC], xl[VEC];
-        if constexpr (VEC == 4) {
-          const float4 h4 = __ldg(reinterpret_cast<const float4*>(xs) + g);
-          const float4 l4 = __ldg(reinterpret_cast<const float4*>(xs + ln_col) + g);
-          xh[0] = h4.x; xh[1] = h4.y; xh[2] = h4.z; xh[3] = h4.w;
-          xl[0] = l4.x; xl[1] = l4.y; xl[2] = l4.z; xl[3] = l4.w;
-        } else {
-          xh[0] = __ldg(xs + g);
-          xl[0] = __ldg(xs + ln_col + g);
-        }
-#pragma unroll
-        for (int r = 0; r < R; r++) {
-          if (r < nr) {
-            float av[VEC];
-            if constexpr (sizeof(V) == 8) {
-              // a = ah + al: Dot2 on ah (x as xh + xl), then al * xh into the
-              // error term (al * xl is below 2^-48 of the product)
-              float al[VEC];
-              ld_vals_dd<V, VEC>(av, al, A + (size_t)(row0 + r) * ln_col + (size_t)g * VEC, pol);
-#pragma unroll
-              for (int k = 0; k < VEC; k++) {
-                dot2_step(sh[r], sc[r], av[k], DF{xh[k], xl[k]});
-                sc[r] = __fmaf_rn(al[k], xh[k], sc[r]);
-              }
-            } else {
-              ld_vals<V, VEC>(av, A + (size_t)(row0 + r) * ln_col + (size_t)g * VEC, pol);
-#pragma unroll
-              for (int k = 0; k < VEC; k++) dot2_step(sh[r], sc[r], av[k], DF{xh[k], xl[k]});
-            }
-          }
-        }
-      }
-#pragma unroll
-      for (int r = 0; r < R; r++) {
-        DF t = two_sum(sh[r], sc[r]);
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
-          t = df_add(t, DF{__shfl_xor_sync(0xffffffffu, t.h, o), __shfl_xor_sync(0xffffffffu, t.l, o)});
-        w[r] = lane == 0 ? df_val(t) : 0.0;
-      }
-    }
-    if (lane == 0) {
-#pragma unroll
-      for (int r = 0; r < R; r++) s_part[parity][r][warp] = w[r];
-    }
-    __syncthreads();
-    if (threadIdx.x < nr) {
-      double t = 0;
-#pragma unroll
-      for (int i = 0; i < NT / kWarp; i++) t = add_rn(t, s_part[parity][threadIdx.x][i]);
-      y[row0 + threadIdx.x] = add_rn(y[row0 + threadIdx.x], t);
-    }
+  if (head) s_part[warp][r] = mine;
+  __syncthreads();
+  if (threadIdx.x < (NW >> log2s) * R) {
+    const int g = threadIdx.x / R, q = threadIdx.x % R;
+    const long row = ((long)blockIdx.x * (NW >> log2s) + g) * R + q;
+    double t = 0;
+    for (int k = 0; k < S; k++) t = add_rn(t, s_part[g * S + k][q]);
+    if (row < ln_row) y[row] = add_rn(fresh ? 0.0 : y[row], t);
   }
 }
 
@@ -474,29 +565,68 @@ cudaError_t dense_values_df_range(const void* vals, int prec, size_t n, int* fla
   return cudaSuccess;
 }
 
+namespace {
+template <class V, int R, bool VEC>
+void launch_dense_df(const V* a, int ln_row, int ln_col, int log2s, const float* xs, const double* x, const int* bad,
+                     int nbad, double* y, int fresh, cudaStream_t s) {
+  const long warps = (((long)ln_row + R - 1) / R) << log2s;
+  const unsigned grid = (unsigned)((warps + NT / kWarp - 1) / (NT / kWarp));
+  k_dense_df<V, R, VEC><<<grid, NT, 0, s>>>(a, ln_row, ln_col, log2s, xs, x, bad, nbad, y, fresh);
+}
+
+// Rows per warp: 4 (FP32) or 2 (the others, whose rows cost more registers a
+// step: with 4, BF16 24576 x 8192 takes 120 us where 2 take 109, FP64 20000 x
+// 8192 238 and 204), fewer where the GPU would not get half a warp's work for
+// each resident warp.  Column parts: until there are four for each resident
+// warp (FP32 16384 x 8192 with 1 / 2 / 4 / 8 parts: 106 / 104 / 102 / 100 us;
+// BF16 24576 x 8192: 106 / 105 / 111 / 128), while a part keeps four steps (FP64
+// 4000 x 2000, 16 steps: 4 parts 20.6 us, 8 parts 22.6).  Wide aligned FP64 rows
+// (5120 columns: where it starts to pay) take four parts at least: a CTA then
+// reads long pieces of few rows, and HBM gives more for fewer streams (20000
+// rows, 2 / 4 / 8 parts: 5120 columns 133 / 132 / 144 us, 16384 columns 396 /
+// 381 / 384).
+template <class V, bool VEC>
+void dense_df_shape(const V* a, int ln_row, int ln_col, const float* xs, const double* x, const int* bad, int nbad,
+                    double* y, int fresh, cudaStream_t s) {
+  constexpr int kMost = sizeof(V) == 4 ? 4 : 2;
+  constexpr long kWarps = 152L * 32;
+  constexpr int SC = 32 * Step<V, VEC>::NV;
+  const int nsteps = (ln_col + SC - 1) / SC;
+  int most = 0;  // log2 of the most parts
+  while (most < 3 && (nsteps >> (most + 1)) >= 4) most++;
+  int r = kMost;
+  while (r > 1 && (((long)ln_row + r - 1) / r << most) < kWarps / 2) r /= 2;
+  int log2s = 0;
+  while (log2s < most && (((long)ln_row + r - 1) / r << log2s) < 4 * kWarps) log2s++;
+  if (sizeof(V) == 8 && VEC && nsteps >= 40) log2s = std::max(log2s, 2);
+  if (r == 1) launch_dense_df<V, 1, VEC>(a, ln_row, ln_col, log2s, xs, x, bad, nbad, y, fresh, s);
+  else if (r == 2) launch_dense_df<V, 2, VEC>(a, ln_row, ln_col, log2s, xs, x, bad, nbad, y, fresh, s);
+  else if constexpr (kMost >= 4) launch_dense_df<V, 4, VEC>(a, ln_row, ln_col, log2s, xs, x, bad, nbad, y, fresh, s);
+}
+
+template <class V>
+void dense_df_vec(const void* vals, int ln_row, int ln_col, const float* xs, const double* x, const int* bad, int nbad,
+                  double* y, int fresh, cudaStream_t s) {
+  const V* a = static_cast<const V*>(vals);
+  // NV values per lane and load when every row starts on a 16-byte boundary
+  // and holds whole vectors (xs from cudaMalloc)
+  constexpr int NV = Step<V, true>::NV;
+  if ((uintptr_t)vals % 16 == 0 && (uintptr_t)xs % 16 == 0 && ln_col % NV == 0)
+    dense_df_shape<V, true>(a, ln_row, ln_col, xs, x, bad, nbad, y, fresh, s);
+  else
+    dense_df_shape<V, false>(a, ln_row, ln_col, xs, x, bad, nbad, y, fresh, s);
+}
+}  // namespace
+
 cudaError_t dense_gemv_df(const void* vals, int prec, int ln_row, int ln_col, const double* x, float* xs,
-                          int* bad, double* y, cudaStream_t s) {
+                          int* bad, double* y, bool fresh, cudaStream_t s) {
   if (ln_row == 0 || ln_col == 0) return cudaSuccess;
-  cudaError_t e = cudaMemsetAsync(bad, 0, sizeof(int), s);
-  if (e) return e;
-  k_df_split_x<<<std::min((ln_col + 255) / 256, 152 * 4), 256, 0, s>>>(x, ln_col, xs, bad);
-  // four values per lane when every row starts on a 16-byte boundary (xs from cudaMalloc)
-  const bool vec = (uintptr_t)vals % 16 == 0 && (uintptr_t)xs % 16 == 0 && ln_col % 4 == 0;
-  constexpr int R = kDenseDfRows;
-  const int grid = (ln_row + R - 1) / R;
-  if (prec == kF64) {
-    const double* a = static_cast<const double*>(vals);
-    if (vec) k_dense_rows_df<double, 4, R><<<grid, NT, 0, s>>>(a, ln_row, ln_col, xs, x, bad, y);
-    else k_dense_rows_df<double, 1, R><<<grid, NT, 0, s>>>(a, ln_row, ln_col, xs, x, bad, y);
-  } else if (prec == kF32) {
-    const float* a = static_cast<const float*>(vals);
-    if (vec) k_dense_rows_df<float, 4, R><<<grid, NT, 0, s>>>(a, ln_row, ln_col, xs, x, bad, y);
-    else k_dense_rows_df<float, 1, R><<<grid, NT, 0, s>>>(a, ln_row, ln_col, xs, x, bad, y);
-  } else {
-    const __nv_bfloat16* a = static_cast<const __nv_bfloat16*>(vals);
-    if (vec) k_dense_rows_df<__nv_bfloat16, 4, R><<<grid, NT, 0, s>>>(a, ln_row, ln_col, xs, x, bad, y);
-    else k_dense_rows_df<__nv_bfloat16, 1, R><<<grid, NT, 0, s>>>(a, ln_row, ln_col, xs, x, bad, y);
-  }
+  const int nbad = std::min((ln_col + NT - 1) / NT, kDenseFlags);
+  k_df_split_x<<<nbad, NT, 0, s>>>(x, ln_col, xs, bad);
+  const int f = fresh ? 1 : 0;
+  if (prec == kF64) dense_df_vec<double>(vals, ln_row, ln_col, xs, x, bad, nbad, y, f, s);
+  else if (prec == kF32) dense_df_vec<float>(vals, ln_row, ln_col, xs, x, bad, nbad, y, f, s);
+  else dense_df_vec<__nv_bfloat16>(vals, ln_row, ln_col, xs, x, bad, nbad, y, f, s);
   return cudaGetLastError();
 }
 
