@@ -189,7 +189,8 @@ int tbsla_matrix_device_bytes(const tbsla_matrix* m, size_t* bytes);
  * implementation's kernels). */
 int tbsla_matrix_kernel_launches(const tbsla_matrix* m, int* launches);
 /* CSR: block budget of the row-block partition (nnz per block, multiple of
- * 256, default 2048); changing it rebuilds the partition. */
+ * 256, default 2048; under TBSLA_CSR_AUTO at most 1024, whose small matrices
+ * gain by more blocks); changing it rebuilds the partition. */
 int tbsla_matrix_set_csr_tile(tbsla_matrix* m, int nnz_per_block);
 /* CSR SpMV kernel: TBSLA_CSR_AUTO (default: row blocks below 2^19 stored
  * entries, where one short launch is latency-bound, else sliced ELL),
@@ -214,9 +215,10 @@ int tbsla_matrix_set_csr_algorithm(tbsla_matrix* m, int algorithm, int items);
  * consecutive rows; longer rows take the fewest lanes (a power of two up to
  * 32) that keep their slice at most long_thr steps wide and are sorted by
  * length over the whole block (defaults 0, 0, 16384, 0; a threshold of 0
- * is automatic: 128 for FP64 values with several column blocks, whose
- * per-block row lengths are about halved, else 64).  Changing them rebuilds the
- * device copy. */
+ * is automatic: with several column blocks 128 for FP64 values, whose
+ * per-block row lengths are about halved, else 64; with one block 16 below
+ * 2^22 entries, 32 below 2^25, else 64, by the rows' mean length).  Changing them rebuilds the device
+ * copy. */
 int tbsla_matrix_set_sell_params(tbsla_matrix* m, int short_thr, int long_thr, int sigma, int col_block);
 /* Batched personalised PageRank with FP32 / BF16 values: gathers of X rows
  * in flight per warp, 8 (default) or 16; a tuning choice, same results. */

@@ -338,7 +338,7 @@ int build_batch(tbsla_batch* B, tbsla_matrix* const* sys, int nsys, int prec) {
     }
     int* pb = nullptr;
     int nb = 0;
-    csr_partition(mrp, ns, 2048, &pb, &nb);
+    csr_partition(mrp, ns, 2048, 0, &pb, &nb);
     for (int t = 1; t <= nb; t++) {
       blocks.push_back((int)o + pb[t]);
       bsys.push_back(s);

@@ -334,9 +334,18 @@ int build_sell(const tbsla_matrix* m, DeviceMatrix* d) {
   // spread over the blocks, so the per-block lengths the thresholds act on
   // are about halved; for FP64 values (whose kernel keeps the next group's
   // columns in flight) doubling the thresholds then pays: at n = 2^24 128 /
-  // 128 is 2.4% faster than 64 / 64.  With one block, or FP32 / BF16 values,
-  // 64 / 64 measured best.
-  const int sthr = m->sell_short > 0 ? m->sell_short : (P > 1 && d->prec == TBSLA_F64 ? 128 : 64);
+  // 128 is 2.4% faster than 64 / 64.  With one block, the widest slice of a
+  // small matrix is a large part of its launch: about 16 up to 2^22 .. 2^23
+  // entries, 32 to 2^25, 64 above (power-law rows, 16 / 32 / 64: 1.4 10^6
+  // entries 21.6 / 23.0 / 28.8 us, 4.2 10^6 33.1 / 33.7 / 40.8, 14 10^6 74.3 /
+  // 67.9 / 69.4, FP32 70.8 / 68.7 / 77.0, 40 10^6 174.8 / 156.5 / 153.0), where
+  // that does not spread the rows of a band, whose neighbours share their
+  // loads of x, over several lanes (27 a row, 8 10^6: 16 32.7, 32 29.3 us; 60 a
+  // row, 18 10^6: 32 50.6, 64 47.4; 4 10^6 or fewer: 16 is faster there too).
+  const long nz = rp[n] - rp[0];
+  const long by = n > 0 ? nz / n : 0;  // entries a row
+  const int one = nz < (1L << 22) || (nz < (1L << 23) && by <= 16) ? 16 : nz < (1L << 25) && by <= 32 ? 32 : 64;
+  const int sthr = m->sell_short > 0 ? m->sell_short : P == 1 ? one : d->prec == TBSLA_F64 ? 128 : 64;
   const int lthr = m->sell_long > 0 ? m->sell_long : sthr;
   long steps = 0;
   d->sell.assign(P - 1 + R, SellPlan{});
@@ -424,20 +433,24 @@ int build(const tbsla_matrix* m, DeviceMatrix* d) {
       if (!st) st = upload_ints(d, &d->idx1, m->idx1.data(), (size_t)end);
       if (!st) st = upload_values(d, m->values.data(), (size_t)end);
       if (st) return st;
-      int tile = std::max(256, std::min(4096, m->csr_tile));
-      d->items = tile <= 1024 ? 4 : tile <= 2048 ? 8 : 16;
-      int* blocks = nullptr;
-      csr_partition(rp, I.ln_row, 256 * d->items, &blocks, &d->nblocks);
-      st = upload_ints(d, &d->blocks, blocks, (size_t)d->nblocks + 1);
-      delete[] blocks;
-      if (st) return st;
       // merge-path tiles and their carry scratch
       const long enz = end - rp[0];
       // automatic kernel: row blocks for small matrices, whose SpMV is one
       // short launch where the sliced-ELL kernel's chain of dependent loads
-      // per slice shows (10^5 entries: 6.2 against 10.3 us); the sliced-ELL
-      // kernel from 2^19 entries on (10^7: 48 against 107 us)
-      d->algo = m->csr_algo >= 0 ? m->csr_algo : (enz < (1L << 19) ? TBSLA_CSR_ROWBLOCK : TBSLA_CSR_SELL);
+      // per slice shows (10^5 entries: 6.2 against 10.5 us; power-law rows, 3000
+      // x 24: 8.4 against 13.6); the sliced-ELL kernel from 2^19 entries on
+      // (10^7: 48 against 107 us; power-law rows, 1.4 10^6: 21.6 against 25).
+      // Below it, row blocks of half the default size give twice the CTAs
+      // (480,000 entries: 10.5 -> 8.4 us, 18,000: 6.3 -> 5.2).
+      const bool small = enz < (1L << 19);
+      int tile = std::max(256, std::min(4096, m->csr_algo < 0 && small ? std::min(1024, m->csr_tile) : m->csr_tile));
+      d->algo = m->csr_algo >= 0 ? m->csr_algo : small ? TBSLA_CSR_ROWBLOCK : TBSLA_CSR_SELL;
+      d->items = tile <= 1024 ? 4 : tile <= 2048 ? 8 : 16;
+      int* blocks = nullptr;
+      csr_partition(rp, I.ln_row, 256 * d->items, d->algo == TBSLA_CSR_ROWBLOCK ? kCsrMaxSteps : 0, &blocks, &d->nblocks);
+      st = upload_ints(d, &d->blocks, blocks, (size_t)d->nblocks + 1);
+      delete[] blocks;
+      if (st) return st;
       d->merge_items = m->merge_items;
       d->ntiles = merge_tiles(I.ln_row, enz, d->merge_items);
       if ((st = dalloc(&d->coord, (size_t)d->ntiles + 1)) || (st = dalloc(&d->carry_row, (size_t)d->ntiles)) ||

@@ -42,6 +42,11 @@ struct Smem {
 
 // Dynamic shared memory of a stream block: x[NT*ITEMS] doubles then
 // values[NT*ITEMS] in the storage precision.
+// Lanes per row of a stream block.
+__host__ __device__ __forceinline__ int row_lanes(int nrows) {
+  return nrows <= 8 ? 32 : nrows <= 16 ? 16 : nrows <= 32 ? 8 : nrows <= 64 ? 4 : nrows <= 128 ? 2 : 1;
+}
+
 template <class V, int ITEMS>
 constexpr size_t stage_bytes() { return (size_t)NT * ITEMS * (sizeof(double) + sizeof(V)); }
 
@@ -85,7 +90,7 @@ __device__ __forceinline__ void csr_block(const CsrArgs& a, int b, const double*
     }
   }
   __syncthreads();
-  const int G = nrows <= 8 ? 32 : nrows <= 16 ? 16 : nrows <= 32 ? 8 : nrows <= 64 ? 4 : nrows <= 128 ? 2 : 1;
+  const int G = row_lanes(nrows);
   const int g = tid / G, lane = tid % G;
   double acc = 0;
   if (g < nrows) {

@@ -151,7 +151,10 @@ cudaError_t sell_spmv(const SellArgs& a, const double* x, double* y, unsigned* c
 // Row-block partition of a CSR row pointer (host): blocks of consecutive
 // rows with at most `tile` entries and at most 256 rows each; a row longer
 // than `tile` forms a block on its own.  Returns the boundaries.
-void csr_partition(const int* rowptr, int n_row, int tile, int** out, int* nblocks);
+// With max_steps > 0, a row that the block's lanes per row would walk in more
+// than that many steps forms a block on its own too.
+void csr_partition(const int* rowptr, int n_row, int tile, int max_steps, int** out, int* nblocks);
+constexpr int kCsrMaxSteps = 32;
 
 // PageRank step on CSR with the iterate carried unnormalised: with
 // s = coef_in[0] = 1/S (S = sum x) and t = coef_in[1],

