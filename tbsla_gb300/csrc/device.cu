@@ -8,8 +8,8 @@
 //         values / columns
 //   ELL   columns int32[max_col*ln_row] and values V[max_col*ln_row],
 //         slot-major (transposed from the reference's row-major)
-//   COO/  rows, cols int32[nnz] and values V[nnz], stably sorted by row
-//   SCOO
+//   COO/  as CSR (below), rows min_row .. max_row; hypersparse ones: rows, cols
+//   SCOO  int32[nnz] and values V[nnz], stably sorted by row
 //   DENSE values V[ln_row*ln_col], row-major
 // V is the storage precision (double / float / bfloat16); products and sums
 // are always FP64.  Vectors are FP64.
@@ -88,7 +88,7 @@ struct DeviceMatrix {
   int* blocks = nullptr;  // CSR row-block partition
   int nblocks = 0;
   int items = 8;
-  int algo = 0;            // CSR: 0 merge path, 1 row blocks, 2 sliced ELL
+  int algo = 0;            // CSR: 0 merge path, 1 row blocks, 2 sliced ELL; COO / SCOO: 0 by triplet chunks
   int* coord = nullptr;    // CSR merge path: first row of each tile
   int* carry_row = nullptr;
   double* carry_val = nullptr;
@@ -133,6 +133,26 @@ struct DeviceMatrix {
   size_t partials_len = 0;
   double* result = nullptr;
 
+  void free_plans() {
+    for (SellPlan& p : sell)
+      for (void* q : {(void*)p.slice, (void*)p.lane, (void*)p.lane_len, (void*)p.piece_cut, (void*)p.piece_at,
+                      (void*)p.cut_first, (void*)p.piece_sum, (void*)p.cut_done, (void*)p.cut_terms})
+        if (q) cudaFree(q);
+    sell.clear();
+  }
+  // a row layout that did not fit (nothing launched on it but copies and fills)
+  void free_rows() {
+    if (stream) cudaStreamSynchronize(stream);
+    free_plans();
+    for (void** p : {&vals, (void**)&idx0, (void**)&idx1, (void**)&blocks, &svals, (void**)&scols,
+                     (void**)&sell_counter}) {
+      if (*p) cudaFree(*p);
+      *p = nullptr;
+    }
+    bytes = 0;
+    algo = 0;
+  }
+
   ~DeviceMatrix() {
     cudaSetDevice(device);
     if (stream) cudaStreamSynchronize(stream);
@@ -144,10 +164,7 @@ struct DeviceMatrix {
                     (void*)bplan.piece_sum,
                     (void*)bplan.cut_done})
       if (p) cudaFree(p);
-    for (SellPlan& p : sell)
-      for (void* q : {(void*)p.slice, (void*)p.lane, (void*)p.lane_len, (void*)p.piece_cut, (void*)p.piece_at,
-                      (void*)p.cut_first, (void*)p.piece_sum, (void*)p.cut_done, (void*)p.cut_terms})
-        if (q) cudaFree(q);
+    free_plans();
     for (cudaEvent_t e : xready)
       if (e) cudaEventDestroy(e);
     if (fork_ev) cudaEventDestroy(fork_ev);
@@ -210,8 +227,9 @@ int dev_host_free(void* p) { return status_of(cudaFreeHost(p)); }
 namespace {
 
 // Stable counting sort of COO/SCOO triplets by row (device copy order).
+// ends[i]: one past the last triplet of row rmin + i.
 void sort_by_row(const tbsla_matrix* m, long nnz, int rmin, int rmax, std::vector<int>& rows,
-                 std::vector<int>& cols, std::vector<double>& vals) {
+                 std::vector<int>& cols, std::vector<double>& vals, std::vector<long>& ends) {
   const int* r = m->idx0.data();
   const int* c = m->idx1.data();
   const double* v = m->values.data();
@@ -228,6 +246,8 @@ void sort_by_row(const tbsla_matrix* m, long nnz, int rmin, int rmax, std::vecto
     cols[p] = c[k];
     vals[p] = v[k];
   }
+  pos.pop_back();
+  ends.swap(pos);
 }
 
 // Host <-> device copies of the large arrays go straight from and to the
@@ -285,7 +305,7 @@ SellArgs sell_args(const tbsla_matrix* m, const DeviceMatrix* d) {
   a.prec = d->prec;
   a.rowptr = d->idx0;
   a.colidx = d->idx1;
-  a.f_col = m->info.f_col;
+  a.f_col = m->format == TBSLA_COO ? 0 : m->info.f_col;
   a.svals = d->svals;
   a.scols = d->scols;
   // automatic: 8 steps in flight (the column blocks keep x in L2, where
@@ -300,20 +320,20 @@ SellArgs sell_args(const tbsla_matrix* m, const DeviceMatrix* d) {
   return a;
 }
 
-// Sliced-ELL device layout of a CSR matrix: the columns are split into
-// blocks of at most `sell_colblock` columns (0: 8,388,608, 64 MiB of x), the
-// plans (row classes, slices, offsets) are made on the host
+constexpr long kSellMin = 1L << 19;  // entries from which on the automatic kernel is sliced ELL
+
+// Sliced-ELL device layout of a matrix in CSR (n rows, nc columns from f_col
+// on; host arrays rp, ci, device copies idx0, idx1, vals): the columns are
+// split into blocks of at most `sell_colblock` columns (0: 8,388,608, 64 MiB
+// of x), the plans (row classes, slices, offsets) are made on the host
 // from the per-block row lengths, and the slice arrays are filled on the
 // device from the CSR copy.
-int build_sell(const tbsla_matrix* m, DeviceMatrix* d) {
+int build_sell(const tbsla_matrix* m, DeviceMatrix* d, int n, int nc, int f_col, const int* rp, const int* ci) {
   using tbsla_impl::parallel_for;
-  const tbsla_info& I = m->info;
-  const int n = I.ln_row, nc = std::max(I.ln_col, 1);
+  nc = std::max(nc, 1);
   const long cb = m->sell_colblock > 0 ? m->sell_colblock : 8388608L;
   const int P = (int)std::max<long>(1, (nc + cb - 1) / cb);
   const int W = (int)(((long)nc + P - 1) / P);
-  const int* rp = m->idx0.data();
-  const int* ci = m->idx1.data();
   std::vector<int> lens((size_t)P * n, 0);
   if (P == 1) {
     for (int i = 0; i < n; i++) lens[i] = rp[i + 1] - rp[i];
@@ -321,7 +341,7 @@ int build_sell(const tbsla_matrix* m, DeviceMatrix* d) {
     parallel_for(n, [&](long b, long e) {
       for (long i = b; i < e; i++)
         for (int j = rp[i]; j < rp[i + 1]; j++) {
-          const int k = std::min(P - 1, std::max(0, (ci[j] - I.f_col) / W));
+          const int k = std::min(P - 1, std::max(0, (ci[j] - f_col) / W));
           lens[(size_t)k * n + i]++;
         }
     });
@@ -416,6 +436,52 @@ int build_sell(const tbsla_matrix* m, DeviceMatrix* d) {
   return TBSLA_OK;
 }
 
+// COO / SCOO triplets, sorted by row, as the CSR rows min_row .. max_row: the
+// kernels of the row layouts need no row index per triplet, no scan by keys and
+// no pass for the rows that cross chunks.  Row blocks and sliced ELL on either
+// side of the line that CSR has; for sliced ELL the CSR copy is freed once the
+// layout is filled (12 bytes an entry, FP64, where the triplets take 16).  Only
+// where a row of the range has a triplet on average: else the arrays over the
+// rows outgrow the triplets.
+// Bound: the gathers of x, as for CSR.  FP64, 2^22 rows x 10: 251 -> 183 us (with
+// triplet chunks: 142 us of gathers, key compares and the carry pass on top);
+// 10,000 x 14: 14.5 -> 6.2; power-law rows, 10^6 x 14: 87 -> 69.
+int build_coo_rows(const tbsla_matrix* m, DeviceMatrix* d, const std::vector<long>& ends,
+                   const std::vector<int>& cols, const std::vector<double>& vals) {
+  const tbsla_info& I = m->info;
+  const bool scoo = m->format == TBSLA_SCOO;
+  std::vector<int> rp(1, 0);
+  rp.insert(rp.end(), ends.begin(), ends.end());
+  const int n = (int)rp.size() - 1;
+  int st = upload_ints(d, &d->idx0, rp.data(), rp.size());
+  if (!st) st = upload_ints(d, &d->idx1, cols.data(), cols.size());
+  if (!st) st = upload_values(d, vals.data(), vals.size());
+  if (st) return st;
+  if (d->nnz < kSellMin) {
+    d->algo = TBSLA_CSR_ROWBLOCK;
+    d->items = 4;
+    int* blocks = nullptr;
+    csr_partition(rp.data(), n, 256 * d->items, kCsrMaxSteps, &blocks, &d->nblocks);
+    st = upload_ints(d, &d->blocks, blocks, (size_t)d->nblocks + 1);
+    const cudaError_t e = cudaStreamSynchronize(d->stream);
+    delete[] blocks;
+    return st ? st : status_of(e);
+  }
+  d->algo = TBSLA_CSR_SELL;
+  const size_t copy = d->bytes;
+  st = build_sell(m, d, n, scoo ? I.ln_col : I.n_col, scoo ? I.f_col : 0, rp.data(), cols.data());
+  if (!st) st = status_of(cudaStreamSynchronize(d->stream));
+  if (st) return st;
+  for (int** p : {&d->idx0, &d->idx1}) {
+    cudaFree(*p);
+    *p = nullptr;
+  }
+  cudaFree(d->vals);
+  d->vals = nullptr;
+  d->bytes -= copy;
+  return TBSLA_OK;
+}
+
 int build(const tbsla_matrix* m, DeviceMatrix* d) {
   const tbsla_info& I = m->info;
   // the matrix's own stream at the greatest priority, so that work forked
@@ -442,7 +508,7 @@ int build(const tbsla_matrix* m, DeviceMatrix* d) {
       // (10^7: 48 against 107 us; power-law rows, 1.4 10^6: 21.6 against 25).
       // Below it, row blocks of half the default size give twice the CTAs
       // (480,000 entries: 10.5 -> 8.4 us, 18,000: 6.3 -> 5.2).
-      const bool small = enz < (1L << 19);
+      const bool small = enz < kSellMin;
       int tile = std::max(256, std::min(4096, m->csr_algo < 0 && small ? std::min(1024, m->csr_tile) : m->csr_tile));
       d->algo = m->csr_algo >= 0 ? m->csr_algo : small ? TBSLA_CSR_ROWBLOCK : TBSLA_CSR_SELL;
       d->items = tile <= 1024 ? 4 : tile <= 2048 ? 8 : 16;
@@ -459,7 +525,7 @@ int build(const tbsla_matrix* m, DeviceMatrix* d) {
       d->bytes += (size_t)d->ntiles * 16 + 4;
       TRY(csr_merge_setup(d->idx0, I.ln_row, enz, d->merge_items, d->coord, d->stream));
       if (d->algo == 2) {
-        st = build_sell(m, d);
+        st = build_sell(m, d, I.ln_row, I.ln_col, I.f_col, rp, m->idx1.data());
         if (st) return st;
       }
       return status_of(cudaStreamSynchronize(d->stream));
@@ -503,8 +569,15 @@ int build(const tbsla_matrix* m, DeviceMatrix* d) {
       d->max_row = rmax;
       std::vector<int> rows, cols;
       std::vector<double> vals;
-      sort_by_row(m, nnz, rmin, rmax, rows, cols, vals);
-      int st = upload_ints(d, &d->idx0, rows.data(), nnz);
+      std::vector<long> ends;
+      sort_by_row(m, nnz, rmin, rmax, rows, cols, vals, ends);
+      int st = TBSLA_OK;
+      if (nnz < INT_MAX && (long)rmax - rmin < nnz) {
+        st = build_coo_rows(m, d, ends, cols, vals);
+        if (st != TBSLA_ERR_ALLOC) return st;
+        d->free_rows();  // no room for the copies: the triplets alone take less
+      }
+      st = upload_ints(d, &d->idx0, rows.data(), nnz);
       if (!st) st = upload_ints(d, &d->idx1, cols.data(), nnz);
       if (!st) st = upload_values(d, vals.data(), nnz);
       const long nch = coo_chunks(nnz);
@@ -591,7 +664,7 @@ CsrArgs csr_args(const tbsla_matrix* m, DeviceMatrix* d) {
   a.colidx = d->idx1;
   a.blocks = d->blocks;
   a.nblocks = d->nblocks;
-  a.f_col = m->info.f_col;
+  a.f_col = m->format == TBSLA_COO ? 0 : m->info.f_col;
   a.items = d->items;
   return a;
 }
@@ -601,12 +674,13 @@ CsrArgs csr_args(const tbsla_matrix* m, DeviceMatrix* d) {
 int ax_device(const tbsla_matrix* m, DeviceMatrix* d, double* r, const double* v, int vect_incr,
               cudaStream_t s, bool zero_first = false) {
   const tbsla_info& I = m->info;
-  const bool fresh = zero_first && d->dense_df && !skips_empty(m);
+  const bool coo_rows = (m->format == TBSLA_COO || m->format == TBSLA_SCOO) && d->algo > 0;
+  const bool fresh = zero_first && (d->dense_df || coo_rows) && !skips_empty(m);
   if (zero_first && !fresh) TRY(cudaMemsetAsync(r, 0, out_len(m) * sizeof(double), s));
   if (skips_empty(m)) return TBSLA_OK;
   switch (m->format) {
     case TBSLA_CSR:
-      if (d->algo == 1) return status_of(csr_spmv(csr_args(m, d), v, r, s));
+      if (d->algo == 1) return status_of(csr_spmv(csr_args(m, d), v, r, false, s));
       if (d->algo == 2) return status_of(sell_spmv(sell_args(m, d), v, r, d->sell_counter, s));
       {
         MergeArgs a{d->vals, d->prec, d->idx0, d->idx1, I.ln_row, d->nnz - m->idx0[0], I.f_col,
@@ -621,7 +695,19 @@ int ax_device(const tbsla_matrix* m, DeviceMatrix* d, double* r, const double* v
       bool scoo = m->format == TBSLA_SCOO;
       long off = (long)vect_incr - (scoo ? I.f_row : 0);
       long len = scoo ? I.ln_row : I.n_row;
-      if (d->min_row + off < 0 || d->max_row + off >= len) return TBSLA_ERR_INVALID_ARG;
+      const bool in = d->min_row + off >= 0 && d->max_row + off < len;
+      if (coo_rows) {
+        // into a zeroed r: the rows min_row .. max_row are written, those before and after zeroed
+        const long lo = in ? d->min_row + off : len, hi = in ? d->max_row + off + 1 : len;
+        if (fresh && lo > 0) TRY(cudaMemsetAsync(r, 0, (size_t)lo * sizeof(double), s));
+        if (fresh && hi < len) TRY(cudaMemsetAsync(r + hi, 0, (size_t)(len - hi) * sizeof(double), s));
+        if (!in) return TBSLA_ERR_INVALID_ARG;
+        if (d->algo == 1) return status_of(csr_spmv(csr_args(m, d), v, r + lo, !fresh, s));
+        SellArgs a = sell_args(m, d);
+        a.add = !fresh;
+        return status_of(sell_spmv(a, v, r + lo, d->sell_counter, s));
+      }
+      if (!in) return TBSLA_ERR_INVALID_ARG;
       const long nch = coo_chunks(d->nnz);
       CooCarry cc{d->coo_carry, d->coo_carry + nch, reinterpret_cast<int*>(d->coo_carry + 2 * nch)};
       return status_of(coo_spmv(d->vals, d->prec, d->idx0, d->idx1, d->nnz, (int)off,
@@ -651,6 +737,12 @@ int dev_bytes(const tbsla_matrix* m, size_t* bytes) {
   return TBSLA_OK;
 }
 
+static int sell_launches(const DeviceMatrix* d) {
+  int k = 0;
+  for (const SellPlan& p : d->sell) k += p.nslices > 0;
+  return k;
+}
+
 int dev_launches(const tbsla_matrix* m, int* launches) {
   int st;
   DeviceMatrix* d = ensure(m, &st);
@@ -659,13 +751,13 @@ int dev_launches(const tbsla_matrix* m, int* launches) {
   if (skips_empty(m))
     k = 0;
   else if (m->format == TBSLA_COO || m->format == TBSLA_SCOO)
-    k = d->nnz > 0;
+    k = d->algo == 2 ? sell_launches(d) : d->nnz > 0;
   else if (m->format == TBSLA_DENSE)
     k = d->dense_df ? 2 : 1;  // double-float: the split of x, then the GEMV
   else if (m->format != TBSLA_CSR)
     k = 1;
   else if (d->algo == 2)
-    for (const SellPlan& p : d->sell) k += p.nslices > 0;
+    k = sell_launches(d);
   else
     k = d->algo == 1 ? 1 : 2;
   *launches = k;

@@ -31,8 +31,8 @@ struct CsrArgs {
   int f_col;
   int items;  // nnz budget per block / 256 (4, 8 or 16)
 };
-// y[row] = (A x)[row] for every row of the partition.
-cudaError_t csr_spmv(const CsrArgs& a, const double* x, double* y, cudaStream_t s);
+// y[row] = (A x)[row] for every row of the partition (+= with add).
+cudaError_t csr_spmv(const CsrArgs& a, const double* x, double* y, bool add, cudaStream_t s);
 // Merge-path CSR SpMV (the default CSR kernel): tiles of 256*items items of
 // the merged (row ends, entries) sequence; coord[ntiles+1] holds each tile's
 // first row, carry_row / carry_val[ntiles] are per-tile scratch.
@@ -121,6 +121,7 @@ struct SellArgs {
   void* svals;  // slice arrays of all blocks
   int* scols;
   int unroll;               // steps per lane in flight: 4, 8 or 16
+  bool add = false;         // y += A x (else y = A x)
   int nblocks;              // column blocks
   const SellPlan* blocks;   // host array of plans holding device pointers
   // optional, per plan: the launch of plan b > 0 waits for ready[b] (its
@@ -140,7 +141,7 @@ struct SellArgs {
 };
 // Fills the slice arrays of every block from the CSR device arrays.
 cudaError_t sell_fill(const SellArgs& a, cudaStream_t s);
-// y = A x, one launch per plan; counter: kSellCounterWords unsigned of
+// y = A x (y += A x with add), one launch per plan; counter: kSellCounterWords unsigned of
 // zeroed scratch (a region per launch that may run at once), reset by each
 // launch; a set *done (device) makes the launches no-ops.
 constexpr int kSellCounterRegion = 1024;

@@ -1,4 +1,7 @@
-// COO / SCOO SpMV as a segmented reduction over a row-sorted device copy.
+// COO / SCOO SpMV as a segmented reduction over a row-sorted device copy: for
+// matrices with fewer triplets than rows between the first and the last one
+// (50,000 rows x 2500 triplets), whose rows the CSR kernels, which the others
+// run, would mostly find empty; and for more than 2^31 triplets.
 //
 // Replaces tbsla::cpp::MatrixCOO::Ax (src/cpp/matrix/MatrixCOO.cpp:135-142)
 // and tbsla::cpp::MatrixSCOO::Ax (src/cpp/matrix/MatrixSCOO.cpp:154-164):

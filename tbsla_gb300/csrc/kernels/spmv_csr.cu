@@ -40,18 +40,23 @@ namespace {
 
 using namespace csr;
 
+// y = A x; add: y += A x, a row without entries not touched.
 struct EpiStore {
   double* y;
-  __device__ __forceinline__ void emit(int row, double s, double*) const { y[row] = s; }
+  int add;
+  __device__ __forceinline__ void emit(int row, double s, double*) const {
+    if (!add) y[row] = s;
+    else if (s != 0.0) y[row] = add_rn(y[row], s);
+  }
 };
 
 template <class V, int ITEMS>
 __global__ void __launch_bounds__(NT) k_csr_spmv(CsrArgs a, const double* __restrict__ x,
-                                                double* __restrict__ y) {
+                                                double* __restrict__ y, int add) {
   extern __shared__ __align__(16) unsigned char stage[];
   __shared__ Smem sm;
   const uint64_t pol = policy_evict_first();
-  EpiStore epi{y};
+  EpiStore epi{y, add};
   csr_block<V, ITEMS>(a, blockIdx.x, x, epi, nullptr, stage, sm, pol);
 }
 
@@ -530,20 +535,20 @@ __global__ void k_df_to_f64(const float2* src, double* dst, long n) {
 }
 
 template <class V, int ITEMS>
-cudaError_t launch_spmv(const CsrArgs& a, const double* x, double* y, cudaStream_t s) {
+cudaError_t launch_spmv(const CsrArgs& a, const double* x, double* y, bool add, cudaStream_t s) {
   constexpr size_t smem = stage_bytes<V, ITEMS>();
   cudaError_t ready = smem_opt_in<k_csr_spmv<V, ITEMS>>(smem);
   if (ready != cudaSuccess) return ready;
-  k_csr_spmv<V, ITEMS><<<a.nblocks, NT, smem, s>>>(a, x, y);
+  k_csr_spmv<V, ITEMS><<<a.nblocks, NT, smem, s>>>(a, x, y, add ? 1 : 0);
   return cudaGetLastError();
 }
 
 template <class V>
-cudaError_t spmv_items(const CsrArgs& a, const double* x, double* y, cudaStream_t s) {
+cudaError_t spmv_items(const CsrArgs& a, const double* x, double* y, bool add, cudaStream_t s) {
   switch (a.items) {
-    case 4: return launch_spmv<V, 4>(a, x, y, s);
-    case 8: return launch_spmv<V, 8>(a, x, y, s);
-    case 16: return launch_spmv<V, 16>(a, x, y, s);
+    case 4: return launch_spmv<V, 4>(a, x, y, add, s);
+    case 8: return launch_spmv<V, 8>(a, x, y, add, s);
+    case 16: return launch_spmv<V, 16>(a, x, y, add, s);
   }
   return cudaErrorInvalidValue;
 }
@@ -739,12 +744,12 @@ cudaError_t df_to_f64(const void* src, double* dst, long n, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-cudaError_t csr_spmv(const CsrArgs& a, const double* x, double* y, cudaStream_t s) {
+cudaError_t csr_spmv(const CsrArgs& a, const double* x, double* y, bool add, cudaStream_t s) {
   if (a.nblocks == 0) return cudaSuccess;
   switch (a.prec) {
-    case kF64: return spmv_items<double>(a, x, y, s);
-    case kF32: return spmv_items<float>(a, x, y, s);
-    case kBF16: return spmv_items<__nv_bfloat16>(a, x, y, s);
+    case kF64: return spmv_items<double>(a, x, y, add, s);
+    case kF32: return spmv_items<float>(a, x, y, add, s);
+    case kBF16: return spmv_items<__nv_bfloat16>(a, x, y, add, s);
   }
   return cudaErrorInvalidValue;
 }

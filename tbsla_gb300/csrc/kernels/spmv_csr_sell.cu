@@ -296,7 +296,8 @@ __global__ void __launch_bounds__(NT) k_sell(SellPlan p, const V* __restrict__ s
       cur = nxt;
       nxt += nwarps;
     } else {
-      if (head) y[l.row] = accumulate ? add_rn(y0, acc) : acc;
+      // (adding: a row without entries is not touched)
+      if (head && (l.len > 0 || !accumulate)) y[l.row] = accumulate ? add_rn(y0, acc) : acc;
       if (lane == 0) after = cl.resolve(after);
       cur = nxt;
       nxt = __shfl_sync(FULL, after, 0);
@@ -383,7 +384,7 @@ cudaError_t launch(const SellArgs& a, const double* x, double* y, unsigned* coun
     if (e == cudaSuccess && a.ready && b > 0) e = cudaStreamWaitEvent(ls, a.ready[b], 0);
     if (e == cudaSuccess && p.nslices > 0) {
       const auto kernel = p.ncut > 0 ? k_sell<V, U, false, true> : k_sell<V, U, false, false>;
-      kernel<<<pg, NT, 0, ls>>>(p, static_cast<const V*>(a.svals), a.scols, a.f_col, b > 0 ? 1 : 0, x, y,
+      kernel<<<pg, NT, 0, ls>>>(p, static_cast<const V*>(a.svals), a.scols, a.f_col, b > 0 || a.add ? 1 : 0, x, y,
                                 counter + k * kSellCounterRegion, done, PageRankArgs{}, Ctl{});
       e = cudaGetLastError();
     }
