@@ -140,12 +140,19 @@ struct DeviceMatrix {
         if (q) cudaFree(q);
     sell.clear();
   }
-  // a row layout that did not fit (nothing launched on it but copies and fills)
-  void free_rows() {
+  // a sliced-ELL layout that did not fit (nothing launched on it but fills)
+  void free_sell() {
     if (stream) cudaStreamSynchronize(stream);
     free_plans();
-    for (void** p : {&vals, (void**)&idx0, (void**)&idx1, (void**)&blocks, &svals, (void**)&scols,
-                     (void**)&sell_counter}) {
+    for (void** p : {&svals, (void**)&scols, (void**)&sell_counter}) {
+      if (*p) cudaFree(*p);
+      *p = nullptr;
+    }
+  }
+  // COO / SCOO: the row layout
+  void free_rows() {
+    free_sell();
+    for (void** p : {&vals, (void**)&idx0, (void**)&idx1, (void**)&blocks}) {
       if (*p) cudaFree(*p);
       *p = nullptr;
     }
@@ -320,7 +327,24 @@ SellArgs sell_args(const tbsla_matrix* m, const DeviceMatrix* d) {
   return a;
 }
 
-constexpr long kSellMin = 1L << 19;  // entries from which on the automatic kernel is sliced ELL
+// The automatic SpMV kernel: row blocks for small matrices, whose SpMV is one
+// short launch where the sliced-ELL kernel's chain of dependent loads per slice
+// shows (10^5 entries: 6.2 against 10.5 us; power-law rows, 3000 x 24: 8.4
+// against 13.6), up to 2^19 entries, and to 3 2^20 where no row is long (560,000
+// entries: 8.3 against 12.5 us, 2 10^6: 14.5 and 19.5, 3.2 10^6: 22.8 each; with
+// long rows, 2.1 10^6: 35 and 25); the sliced-ELL kernel from there on (10^7: 48
+// against 107 us).
+constexpr long kSellMin = 1L << 19, kSellMinShort = 3L << 20;
+constexpr int kShortRow = 64;
+bool row_blocks_first(const int* rp, int n) {
+  const long nz = (long)rp[n] - rp[0];
+  if (nz < kSellMin) return true;
+  if (nz >= kSellMinShort) return false;
+  for (int i = 0; i < n; i++)
+    if (rp[i + 1] - rp[i] > kShortRow) return false;
+  return true;
+}
+
 
 // Sliced-ELL device layout of a matrix in CSR (n rows, nc columns from f_col
 // on; host arrays rp, ci, device copies idx0, idx1, vals): the columns are
@@ -457,7 +481,7 @@ int build_coo_rows(const tbsla_matrix* m, DeviceMatrix* d, const std::vector<lon
   if (!st) st = upload_ints(d, &d->idx1, cols.data(), cols.size());
   if (!st) st = upload_values(d, vals.data(), vals.size());
   if (st) return st;
-  if (d->nnz < kSellMin) {
+  if (row_blocks_first(rp.data(), n)) {
     d->algo = TBSLA_CSR_ROWBLOCK;
     d->items = 4;
     int* blocks = nullptr;
@@ -499,18 +523,12 @@ int build(const tbsla_matrix* m, DeviceMatrix* d) {
       if (!st) st = upload_ints(d, &d->idx1, m->idx1.data(), (size_t)end);
       if (!st) st = upload_values(d, m->values.data(), (size_t)end);
       if (st) return st;
-      // merge-path tiles and their carry scratch
-      const long enz = end - rp[0];
-      // automatic kernel: row blocks for small matrices, whose SpMV is one
-      // short launch where the sliced-ELL kernel's chain of dependent loads
-      // per slice shows (10^5 entries: 6.2 against 10.5 us; power-law rows, 3000
-      // x 24: 8.4 against 13.6); the sliced-ELL kernel from 2^19 entries on
-      // (10^7: 48 against 107 us; power-law rows, 1.4 10^6: 21.6 against 25).
-      // Below it, row blocks of half the default size give twice the CTAs
-      // (480,000 entries: 10.5 -> 8.4 us, 18,000: 6.3 -> 5.2).
-      const bool small = enz < kSellMin;
-      int tile = std::max(256, std::min(4096, m->csr_algo < 0 && small ? std::min(1024, m->csr_tile) : m->csr_tile));
-      d->algo = m->csr_algo >= 0 ? m->csr_algo : small ? TBSLA_CSR_ROWBLOCK : TBSLA_CSR_SELL;
+      const long enz = end - rp[0];  // merge-path tiles and their carry scratch
+      d->algo = m->csr_algo >= 0 ? m->csr_algo : row_blocks_first(rp, I.ln_row) ? TBSLA_CSR_ROWBLOCK : TBSLA_CSR_SELL;
+      // automatic: row blocks of half the default size, which give twice the
+      // CTAs (480,000 entries: 10.5 -> 8.4 us, 18,000: 6.3 -> 5.2)
+      const int budget = m->csr_algo < 0 && d->algo == TBSLA_CSR_ROWBLOCK ? std::min(1024, m->csr_tile) : m->csr_tile;
+      int tile = std::max(256, std::min(4096, budget));
       d->items = tile <= 1024 ? 4 : tile <= 2048 ? 8 : 16;
       int* blocks = nullptr;
       csr_partition(rp, I.ln_row, 256 * d->items, d->algo == TBSLA_CSR_ROWBLOCK ? kCsrMaxSteps : 0, &blocks, &d->nblocks);
@@ -953,7 +971,7 @@ int dev_normalize_cols(tbsla_matrix* m, const double* s) {
   // keep the host arrays (the reference layout) in step with the device
   TRY(cudaMemcpyAsync(m->values.data(), v64, d->nnz * 8, cudaMemcpyDeviceToHost, str));
   if (owned) TRY(convert_values(v64, d->vals, d->prec, d->nnz, str));
-  if (d->algo == 2 && d->svals) TRY(sell_fill(sell_args(m, d), str));  // slice copy
+  if (d->svals) TRY(sell_fill(sell_args(m, d), str));  // slice copy
   d->colw_ok = false;
   TRY(cudaStreamSynchronize(str));
   if (owned) cudaFree(v64);
@@ -1000,7 +1018,7 @@ int dev_normalize_rows(tbsla_matrix* m, const double* s) {
   // keep the host arrays (the reference layout) in step with the device
   TRY(cudaMemcpyAsync(m->values.data(), v64, d->nnz * 8, cudaMemcpyDeviceToHost, str));
   if (owned) TRY(convert_values(v64, d->vals, d->prec, d->nnz, str));
-  if (d->algo == 2 && d->svals) TRY(sell_fill(sell_args(m, d), str));  // slice copy
+  if (d->svals) TRY(sell_fill(sell_args(m, d), str));  // slice copy
   d->colw_ok = false;
   TRY(cudaStreamSynchronize(str));
   if (owned) cudaFree(v64);
@@ -1073,7 +1091,7 @@ int dev_apply_exponential(tbsla_matrix* m, const double* max_abs, int base) {
   // keep the host arrays (the reference layout) in step with the device
   TRY(cudaMemcpyAsync(m->values.data(), v64, d->nnz * 8, cudaMemcpyDeviceToHost, str));
   if (owned) TRY(convert_values(v64, d->vals, d->prec, d->nnz, str));
-  if (d->algo == 2 && d->svals) TRY(sell_fill(sell_args(m, d), str));
+  if (d->svals) TRY(sell_fill(sell_args(m, d), str));
   d->colw_ok = false;
   TRY(cudaStreamSynchronize(str));
   if (owned) cudaFree(v64);
@@ -1144,6 +1162,17 @@ void initial_coefficients(const DeviceMatrix* d, double beta, double c[2]) {
 }
 }  // namespace
 
+static int pagerank_layout(const tbsla_matrix* m, DeviceMatrix* d) {
+  const tbsla_info& I = m->info;
+  if (!d->sell.empty() || I.ln_col > 8388608) return TBSLA_OK;
+  int st = build_sell(m, d, I.ln_row, I.ln_col, I.f_col, m->idx0.data(), m->idx1.data());
+  if (st == TBSLA_ERR_ALLOC) {  // no room: the row-block kernel
+    d->free_sell();
+    st = TBSLA_OK;
+  }
+  return st;
+}
+
 int dev_page_rank(tbsla_matrix* m, double beta, double eps, int max_it, double* result,
                   int* iterations, double* error) {
   if (m->format != TBSLA_CSR) return TBSLA_ERR_UNSUPPORTED;
@@ -1156,8 +1185,13 @@ int dev_page_rank(tbsla_matrix* m, double beta, double eps, int max_it, double* 
   const int n = I.n_row;
   cudaStream_t s = d->stream;
   // the sliced-ELL kernel (FP64-efficient on skewed rows) with a separate
-  // epilogue pass, or the row-block kernel with the epilogue fused
-  const bool sell = d->algo == 2;
+  // epilogue pass, or the row-block kernel with the epilogue fused.  Under the
+  // automatic kernel the former at every size: its warps take slices of equal
+  // work where the row-block kernel's CTAs draw blocks one by one (a step of n
+  // x mean 5000 x 8: 24 -> 20 us, 50,000 x 10: 31 -> 22; 60 with long rows in
+  // the blocks)
+  if (m->csr_algo < 0 && d->algo == 1 && m->pr_fused && I.nnz > 0 && (st = pagerank_layout(m, d))) return st;
+  const bool sell = !d->sell.empty();
   int sms = 152;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, d->device);
   int grid = sell ? 8 * sms : (I.nnz > 0 ? csr_pagerank_grid(d->items, d->prec) : 1);

@@ -62,3 +62,43 @@ def test_page_rank(gpu):
         out.append(m.page_rank(beta=0.85, epsilon=1e-12, max_iterations=500)[0])
     for x in out[:2]:
         assert np.abs(x - out[2]).sum() <= 1e-12
+
+
+@pytest.mark.parametrize("count", [(1 << 19) - 1, 1 << 19, (3 << 20) - 1, 3 << 20])
+@pytest.mark.parametrize("longest", [64, 65])
+def test_kernel_by_size(gpu, count, longest):
+    """Either side of the sizes where the automatic kernel changes."""
+    T = gpu
+    n = 60_000
+    rng = np.random.default_rng(count + longest)
+    lens = np.full(n, count // n)
+    lens[n // 2] = longest
+    lens[: count - lens.sum()] += 1
+    rp = np.concatenate(([0], np.cumsum(lens)))
+    ci = rng.integers(0, n, rp[-1])
+    v = rng.uniform(-1, 1, rp[-1])
+    m = T.MatrixCSR.from_arrays(n, n, rp, ci, v)
+    x = rng.uniform(-1, 1, n)
+    a = m.arrays()
+    ref = oracle.csr_ax(a["rowptr"], a["colidx"], v, x)
+    scale = oracle.csr_absrow(a["rowptr"], a["colidx"], v, x)
+    assert oracle.rel_err_normalized(m.spmv(x), ref, scale) <= TOL
+
+
+def test_page_rank_after_an_update(gpu):
+    """PageRank's layout of a small matrix follows a change of the values: the
+    vector of a matrix made from the changed arrays, bit for bit."""
+    T = gpu
+    n = 2000
+    rng = np.random.default_rng(9)
+    rp = np.concatenate(([0], np.cumsum(rng.integers(0, 12, n))))
+    ci = rng.integers(0, n, rp[-1])
+    m = T.MatrixCSR.from_arrays(n, n, rp, ci, rng.uniform(0.5, 1.5, rp[-1]))
+    first, *_ = m.page_rank(beta=0.5)
+    sums = np.zeros(n)
+    m.make_stochastic(sums)
+    a = m.arrays()
+    fresh = T.MatrixCSR.from_arrays(n, n, a["rowptr"], a["colidx"], a["values"])
+    x, it, *_ = m.page_rank(beta=0.85)
+    y, jt, *_ = fresh.page_rank(beta=0.85)
+    assert it == jt and np.array_equal(x, y) and not np.array_equal(x, first)
