@@ -408,6 +408,11 @@ cudaError_t csr_normalize_cols(double* vals, const int* rowptr, const int* colid
 long radix_scratch(long n);
 cudaError_t radix_sort_pairs(uint64_t* keys, uint64_t* keys_alt, int* vals, int* vals_alt, long n, int bits,
                              unsigned* scratch, int* result_in_alt, cudaStream_t s);
+// w[c] = the sum of column c's values (c relative to f_col), added in entry
+// order; scratch: column_sums_scratch(n, n_col) words.
+long column_sums_scratch(long n, int n_col);
+cudaError_t column_sums_ordered(const void* vals, int prec, const int* colidx, long n, int f_col, int n_col,
+                                unsigned* scratch, double* w, cudaStream_t s);
 // Exclusive scan in place; scratch: scan_scratch(n) words.
 long scan_scratch(long n);
 cudaError_t exclusive_scan(unsigned* a, long n, unsigned* scratch, cudaStream_t s);

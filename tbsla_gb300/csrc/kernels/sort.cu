@@ -1,5 +1,5 @@
-// Stable LSD radix sort of (64-bit key, int32 value) pairs, and the COO ->
-// CSR ordering built on it.
+// Stable LSD radix sort of (64- or 32-bit key, int32 value) pairs, the COO ->
+// CSR ordering and the column sums in entry order built on it.
 //
 // Replaces the ordering step of tbsla::cpp::MatrixCSR(const MatrixCOO&)
 // (src/cpp/matrix/MatrixCSR.cpp:49-96 with compare_row,
@@ -30,7 +30,8 @@ constexpr int RADIX = 256;
 constexpr int SCAN_CHUNK = 2048;  // elements per CTA in the scan (8 per thread)
 constexpr unsigned FULL = 0xffffffffu;
 
-__global__ void __launch_bounds__(RT) k_hist(const uint64_t* __restrict__ keys, long n, int shift, int ntiles,
+template <class K>
+__global__ void __launch_bounds__(RT) k_hist(const K* __restrict__ keys, long n, int shift, int ntiles,
                                             unsigned* __restrict__ hist) {
   __shared__ unsigned h[RADIX];
   for (int d = threadIdx.x; d < RADIX; d += RT) h[d] = 0;
@@ -44,8 +45,9 @@ __global__ void __launch_bounds__(RT) k_hist(const uint64_t* __restrict__ keys, 
   for (int d = threadIdx.x; d < RADIX; d += RT) hist[(long)d * ntiles + blockIdx.x] = h[d];
 }
 
-__global__ void __launch_bounds__(RT) k_scatter(const uint64_t* __restrict__ keys, const int* __restrict__ vals,
-                                               uint64_t* __restrict__ okeys, int* __restrict__ ovals, long n,
+template <class K>
+__global__ void __launch_bounds__(RT) k_scatter(const K* __restrict__ keys, const int* __restrict__ vals,
+                                               K* __restrict__ okeys, int* __restrict__ ovals, long n,
                                                int shift, int ntiles, const unsigned* __restrict__ offs) {
   __shared__ unsigned base[RADIX];
   __shared__ unsigned wcnt[RT / kWarp][RADIX];
@@ -58,7 +60,7 @@ __global__ void __launch_bounds__(RT) k_scatter(const uint64_t* __restrict__ key
     __syncthreads();
     const long i = t0 + (long)r * RT + threadIdx.x;
     const bool valid = i < n;
-    const uint64_t key = valid ? keys[i] : 0;
+    const K key = valid ? keys[i] : 0;
     const int dg = valid ? (int)((key >> shift) & (RADIX - 1)) : RADIX;  // RADIX: no key
     const unsigned peers = __match_any_sync(FULL, dg);
     const int rank = __popc(peers & lt);
@@ -166,8 +168,10 @@ long radix_scratch(long n) {
   return (long)RADIX * ntiles + scan_scratch((long)RADIX * ntiles);
 }
 
-cudaError_t radix_sort_pairs(uint64_t* keys, uint64_t* keys_alt, int* vals, int* vals_alt, long n, int bits,
-                             unsigned* scratch, int* result_in_alt, cudaStream_t s) {
+namespace {
+template <class K>
+cudaError_t sort_pairs(K* keys, K* keys_alt, int* vals, int* vals_alt, long n, int bits, unsigned* scratch,
+                       int* result_in_alt, cudaStream_t s) {
   *result_in_alt = 0;
   if (n <= 1) return cudaSuccess;
   const long ntiles = (n + TILE - 1) / TILE;
@@ -175,8 +179,8 @@ cudaError_t radix_sort_pairs(uint64_t* keys, uint64_t* keys_alt, int* vals, int*
   unsigned* sc = scratch + RADIX * ntiles;
   int flip = 0;
   for (int shift = 0; shift < bits; shift += 8) {
-    const uint64_t* ki = flip ? keys_alt : keys;
-    uint64_t* ko = flip ? keys : keys_alt;
+    const K* ki = flip ? keys_alt : keys;
+    K* ko = flip ? keys : keys_alt;
     const int* vi = flip ? vals_alt : vals;
     int* vo = flip ? vals : vals_alt;
     k_hist<<<(unsigned)ntiles, RT, 0, s>>>(ki, n, shift, (int)ntiles, hist);
@@ -190,6 +194,108 @@ cudaError_t radix_sort_pairs(uint64_t* keys, uint64_t* keys_alt, int* vals, int*
   }
   *result_in_alt = flip;
   return cudaSuccess;
+}
+
+// 32-bit keys (columns) and their entries' indices, in entry order.
+__global__ void k_column_keys(const int* __restrict__ colidx, long n, int f_col, unsigned* __restrict__ keys,
+                              int* __restrict__ idx) {
+  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
+    keys[i] = (unsigned)(colidx[i] - f_col);
+    idx[i] = (int)i;
+  }
+}
+
+// start[c]: the first of the sorted keys that is c or more (c <= n_col).
+__global__ void k_column_starts(const unsigned* __restrict__ keys, long n, int n_col, int* __restrict__ start) {
+  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i <= n; i += (long)gridDim.x * blockDim.x) {
+    const long from = i > 0 ? (long)keys[i - 1] + 1 : 0, to = i < n ? (long)keys[i] : n_col;
+    for (long c = from; c <= to; c++) start[c] = (int)i;
+  }
+}
+
+// w[c] = sum of column c's values, added one by one in entry order from 0 (the
+// order of a loop over the entries, so the same bits).  A lane per column; a
+// column of more than kLaneColumn entries by its whole warp: 32 values loaded
+// at once, added in order by shuffles.
+constexpr int kLaneColumn = 64;
+template <class V>
+__global__ void __launch_bounds__(RT) k_column_sums_ordered(const V* __restrict__ vals, const int* __restrict__ perm,
+                                                           const int* __restrict__ start, int n_col,
+                                                           double* __restrict__ w) {
+  const int lane = threadIdx.x & 31;
+  for (long c0 = (blockIdx.x * (long)RT + threadIdx.x) / kWarp * kWarp; c0 < n_col; c0 += (long)gridDim.x * RT) {
+    const long c = c0 + lane;
+    const int a = c < n_col ? start[c] : 0, e = c < n_col ? start[c + 1] : 0;
+    double sum = 0.0;
+    if (e - a <= kLaneColumn) {
+      int t = a;
+      for (; t + 4 <= e; t += 4) {
+        double v[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) v[u] = widen(vals[perm[t + u]]);
+#pragma unroll
+        for (int u = 0; u < 4; u++) sum = add_rn(sum, v[u]);
+      }
+      for (; t < e; t++) sum = add_rn(sum, widen(vals[perm[t]]));
+    }
+    for (unsigned left = __ballot_sync(FULL, e - a > kLaneColumn); left; left &= left - 1) {
+      const int src = __ffs(left) - 1;
+      const int la = __shfl_sync(FULL, a, src), le = __shfl_sync(FULL, e, src);
+      double s = 0.0, v = la + lane < le ? widen(vals[perm[la + lane]]) : 0.0;
+      for (int t = la; t < le; t += kWarp) {
+        const int next = t + kWarp + lane;
+        const double vn = next < le ? widen(vals[perm[next]]) : 0.0;
+        const int m = min(kWarp, le - t);
+        if (m == kWarp) {
+#pragma unroll
+          for (int u = 0; u < kWarp; u++) s = add_rn(s, __shfl_sync(FULL, v, u));
+        } else {
+          for (int u = 0; u < m; u++) s = add_rn(s, __shfl_sync(FULL, v, u));
+        }
+        v = vn;
+      }
+      if (lane == src) sum = s;
+    }
+    if (c < n_col) w[c] = sum;
+  }
+}
+}  // namespace
+
+cudaError_t radix_sort_pairs(uint64_t* keys, uint64_t* keys_alt, int* vals, int* vals_alt, long n, int bits,
+                             unsigned* scratch, int* result_in_alt, cudaStream_t s) {
+  return sort_pairs(keys, keys_alt, vals, vals_alt, n, bits, scratch, result_in_alt, s);
+}
+
+long column_sums_scratch(long n, int n_col) { return 4 * n + n_col + 1 + radix_scratch(n); }
+
+cudaError_t column_sums_ordered(const void* vals, int prec, const int* colidx, long n, int f_col, int n_col,
+                                unsigned* scratch, double* w, cudaStream_t s) {
+  if (n_col <= 0) return cudaSuccess;
+  unsigned *keys = scratch, *alt = keys + n;
+  int *perm = reinterpret_cast<int*>(alt + n), *perm_alt = perm + n, *start = perm_alt + n;
+  int bits = 0, in_alt = 0;
+  while (bits < 31 && (1L << bits) < (long)n_col) bits++;
+  if (n > 0) k_column_keys<<<grid_for(n), RT, 0, s>>>(colidx, n, f_col, keys, perm);
+  cudaError_t e = cudaGetLastError();
+  if (e == cudaSuccess)
+    e = sort_pairs(keys, alt, perm, perm_alt, n, bits, reinterpret_cast<unsigned*>(start + n_col + 1), &in_alt, s);
+  if (e != cudaSuccess) return e;
+  const int* p = in_alt ? perm_alt : perm;
+  k_column_starts<<<grid_for(n + 1), RT, 0, s>>>(in_alt ? alt : keys, n, n_col, start);
+  const int grid = grid_for(n_col);
+  switch (prec) {
+    case kF64:
+      k_column_sums_ordered<<<grid, RT, 0, s>>>(static_cast<const double*>(vals), p, start, n_col, w);
+      break;
+    case kF32:
+      k_column_sums_ordered<<<grid, RT, 0, s>>>(static_cast<const float*>(vals), p, start, n_col, w);
+      break;
+    case kBF16:
+      k_column_sums_ordered<<<grid, RT, 0, s>>>(static_cast<const __nv_bfloat16*>(vals), p, start, n_col, w);
+      break;
+    default: return cudaErrorInvalidValue;
+  }
+  return cudaGetLastError();
 }
 
 // COO -> DENSE (MatrixDENSE.cpp:15-37): the entries in (row, column) order,
