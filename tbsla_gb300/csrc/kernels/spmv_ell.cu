@@ -19,7 +19,12 @@ namespace tbsla_gpu {
 
 namespace {
 
-constexpr int NT = 256;
+// Bound: FP64 issue (a multiply and an add per slot, 16 cycles a warp and SM:
+// 51 of 65 us at 1.5 10^6 rows x 10) and the gathers of x (51 us).  Small CTAs
+// spread a few rows over all SMs (50,000 rows x 10: 256 threads 8.3 us, 64 6.3)
+// and leave a shorter last wave (1.5 10^6 x 10: 65.7 -> 65.2; 32: 69); more slots
+// in flight lose as many warps (8: 9 slots of 4 10^6 rows 160 us, not 144).
+constexpr int NT = 64;
 
 template <class V, bool SHIFT>
 __global__ void __launch_bounds__(NT) k_ell(const V* __restrict__ vals, const int* __restrict__ cols,
