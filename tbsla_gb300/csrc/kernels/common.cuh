@@ -62,6 +62,19 @@ __device__ __forceinline__ int ld_stream(const int* p, uint64_t pol) {
 // diagonal part of a row block hits L1).
 __device__ __forceinline__ double ld_gather(const double* p) { return __ldg(p); }
 
+// As ld_gather for a kernel launched with launch_early: an ordinary load, since
+// x may be written while the kernel already waits (p without __restrict__).
+__device__ __forceinline__ double ld_gather_late(const double* p) { return *p; }
+
+template <bool LATE>
+__device__ __forceinline__ double gather(const double* p) {
+  return LATE ? ld_gather_late(p) : ld_gather(p);
+}
+
+// First statement of a kernel launched with launch_early: waits until the
+// kernels before it in the stream have ended and their writes can be seen.
+__device__ __forceinline__ void wait_for_earlier() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // Narrowing to the storage precision, round to nearest even.  bfloat16 is
 // rounded from the double's bits directly (no intermediate float rounding):
 // add half an ulp of the 8-bit significand (ties to even), drop the low 45
@@ -153,6 +166,28 @@ cudaError_t smem_opt_in(size_t smem) {
   e = cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e == cudaSuccess && bit) done.fetch_or(bit, std::memory_order_acq_rel);
   return e;
+}
+
+// Launches a kernel that begins with wait_for_earlier: it is set up, and its
+// CTAs start, as soon as the CTAs of the kernel before it in the stream have
+// ended, where an ordinary launch first waits for that kernel's completion (CSR
+// row blocks, calls in a row: 10,000 x 10 6.2 -> 3.0 us, 30,000 x 10 6.2 -> 4.1).
+// No kernel asks for its successor before its own CTAs end: those that would
+// then wait on the SMs cost more than they save (30,000 x 10: 7.1 us).
+template <class... P, class... A>
+cudaError_t launch_early(void (*kernel)(P...), unsigned grid, unsigned threads, size_t smem, cudaStream_t s,
+                         const A&... args) {
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c{};
+  c.gridDim = dim3(grid);
+  c.blockDim = dim3(threads);
+  c.dynamicSmemBytes = smem;
+  c.stream = s;
+  c.attrs = &at;
+  c.numAttrs = 1;
+  return cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
 }
 
 }  // namespace tbsla_gpu

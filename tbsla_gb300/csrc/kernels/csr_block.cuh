@@ -11,7 +11,7 @@ namespace csr {
 
 constexpr int NT = 256;
 
-template <class V>
+template <class V, bool LATE = false>
 __device__ __forceinline__ double row_dot_cta(const V* vals, const int* colidx, int s, int e,
                                               const double* x, int f_col, uint64_t pol) {
   double acc = 0;
@@ -21,15 +21,15 @@ __device__ __forceinline__ double row_dot_cta(const V* vals, const int* colidx, 
     int c2 = ld_stream(colidx + j + 2 * NT, pol), c3 = ld_stream(colidx + j + 3 * NT, pol);
     V v0 = ld_stream(vals + j, pol), v1 = ld_stream(vals + j + NT, pol);
     V v2 = ld_stream(vals + j + 2 * NT, pol), v3 = ld_stream(vals + j + 3 * NT, pol);
-    double x0 = ld_gather(x + c0 - f_col), x1 = ld_gather(x + c1 - f_col);
-    double x2 = ld_gather(x + c2 - f_col), x3 = ld_gather(x + c3 - f_col);
+    double x0 = gather<LATE>(x + c0 - f_col), x1 = gather<LATE>(x + c1 - f_col);
+    double x2 = gather<LATE>(x + c2 - f_col), x3 = gather<LATE>(x + c3 - f_col);
     acc = fma_rn(widen(v0), x0, acc);
     acc = fma_rn(widen(v1), x1, acc);
     acc = fma_rn(widen(v2), x2, acc);
     acc = fma_rn(widen(v3), x3, acc);
   }
   for (; j < e; j += NT)
-    acc = fma_rn(widen(ld_stream(vals + j, pol)), ld_gather(x + ld_stream(colidx + j, pol) - f_col), acc);
+    acc = fma_rn(widen(ld_stream(vals + j, pol)), gather<LATE>(x + ld_stream(colidx + j, pol) - f_col), acc);
   return acc;
 }
 
@@ -51,7 +51,7 @@ template <class V, int ITEMS>
 constexpr size_t stage_bytes() { return (size_t)NT * ITEMS * (sizeof(double) + sizeof(V)); }
 
 // One block of the partition; epi.emit(row, sum, red) per row.
-template <class V, int ITEMS, class Epi>
+template <class V, int ITEMS, class Epi, bool LATE = false>
 __device__ __forceinline__ void csr_block(const CsrArgs& a, int b, const double* x, const Epi& epi,
                                           double* red, unsigned char* stage, Smem& sm, uint64_t pol) {
   const V* vals = static_cast<const V*>(a.vals);
@@ -62,7 +62,7 @@ __device__ __forceinline__ void csr_block(const CsrArgs& a, int b, const double*
   const int tid = threadIdx.x;
   if (nrows == 1) {
     const int s = a.rowptr[r0], e = a.rowptr[r0 + 1];
-    double acc = row_dot_cta(vals, a.colidx, s, e, x, a.f_col, pol);
+    double acc = row_dot_cta<V, LATE>(vals, a.colidx, s, e, x, a.f_col, pol);
     acc = block_sum<NT>(acc, sm.red);
     if (tid == 0) epi.emit(r0, acc, red);
     return;
@@ -85,7 +85,7 @@ __device__ __forceinline__ void csr_block(const CsrArgs& a, int b, const double*
   for (int k = 0; k < ITEMS; k++) {
     const int i = k * NT + tid;
     if (i < cnt) {
-      s_x[i] = ld_gather(x + cidx[k] - a.f_col);
+      s_x[i] = gather<LATE>(x + cidx[k] - a.f_col);
       s_v[i] = vv[k];
     }
   }

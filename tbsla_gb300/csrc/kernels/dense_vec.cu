@@ -121,11 +121,11 @@ __global__ void __launch_bounds__(NT) k_dense_rows_f64x2(const double* __restric
 //  * the lanes' pairs are summed across the warp in double-float (TwoSum-
 //    based additions), the R rows at once (each half of the warp goes on with
 //    half of the rows), and the column parts in FP64, in a fixed order.
-// Bound: HBM for FP64 and FP32 values (16384 x 8192: 165 and 101 us, 6.5 and
-// 5.3 TB/s with the launches), instruction issue (about 15 per entry) for BF16
-// (24576 x 8192: 109 us).  With a CTA per row, one row's x loads, its warp
+// Bound: HBM for FP64 and FP32 values (16384 x 8192: 161 and 97 us, 6.7 and
+// 5.5 TB/s with the launches), instruction issue (about 15 per entry) for BF16
+// (24576 x 8192: 104 us).  With a CTA per row, one row's x loads, its warp
 // reductions and a barrier came to more instructions than the entries
-// themselves: 177, 122 and 164 us, and 65 us for 9000 x 600 FP32, now 12.4.
+// themselves: 177, 122 and 164 us, and 65 us for 9000 x 600 FP32, now 7.8.
 // The float arithmetic is exact only inside the float exponent range, so the
 // path needs every nonzero |x| and |a| in [2^-40, 2^40] (products within
 // [2^-80, 2^80], sums of up to 2^31 of them finite, error terms normal): the
@@ -142,8 +142,8 @@ __device__ __forceinline__ bool df_in_range(double v) {
 
 // xs[0, n) = xh, xs[n, 2n) = xl: separate arrays, so that the GEMV's lanes
 // read consecutive words of each.  bad[CTA]: x leaves the range there.
-__global__ void __launch_bounds__(NT) k_df_split_x(const double* __restrict__ x, int n, float* __restrict__ xs,
-                                                  int* __restrict__ bad) {
+__global__ void __launch_bounds__(NT) k_df_split_x(const double* x, int n, float* xs, int* bad) {
+  wait_for_earlier();
   int any = 0;
   for (int i = blockIdx.x * NT + threadIdx.x; i < n; i += gridDim.x * NT) {
     const double v = x[i];
@@ -284,9 +284,9 @@ __device__ __forceinline__ DF warp_sum_rows(DF (&t)[R]) {
 // 117, FP32 98, FP64 193 us where 109, 101 and 185 were taken then).
 template <class V, int R, bool VEC>
 __global__ void __launch_bounds__(NT, 4) k_dense_df(const V* __restrict__ A, int ln_row, int ln_col, int log2s,
-                                                   const float* __restrict__ xs, const double* __restrict__ x,
-                                                   const int* __restrict__ bad, int nbad, double* __restrict__ y,
-                                                   int fresh) {
+                                                   const float* xs, const double* x, const int* bad, int nbad,
+                                                   double* y, int fresh) {
+  wait_for_earlier();
   constexpr int NV = Step<V, VEC>::NV, SC = 32 * NV, NW = NT / kWarp;
   __shared__ double s_part[NW][R];
   const int lane = threadIdx.x % kWarp, warp = threadIdx.x / kWarp;
@@ -332,16 +332,16 @@ __global__ void __launch_bounds__(NT, 4) k_dense_df(const V* __restrict__ A, int
       float xh[4], xl[4];
       if constexpr (VEC) {
         const int cc = min(c, last) + k0;
-        const float4 h4 = __ldg(reinterpret_cast<const float4*>(xs + cc));
-        const float4 l4 = __ldg(reinterpret_cast<const float4*>(xs + ln_col + cc));
+        const float4 h4 = *reinterpret_cast<const float4*>(xs + cc);
+        const float4 l4 = *reinterpret_cast<const float4*>(xs + ln_col + cc);
         xh[0] = h4.x; xh[1] = h4.y; xh[2] = h4.z; xh[3] = h4.w;
         xl[0] = l4.x; xl[1] = l4.y; xl[2] = l4.z; xl[3] = l4.w;
       } else {
 #pragma unroll
         for (int k = 0; k < 4; k++) {
           const int cc = min(c + 32 * (k0 + k), last);
-          xh[k] = __ldg(xs + cc);
-          xl[k] = __ldg(xs + ln_col + cc);
+          xh[k] = xs[cc];
+          xl[k] = xs[ln_col + cc];
         }
       }
       if (st == nsteps - 1) {
@@ -382,7 +382,7 @@ __global__ void __launch_bounds__(NT, 4) k_dense_df(const V* __restrict__ A, int
       double acc = 0;
       for (int st = part; st < nsteps; st += S)
         for (int j = st * SC + lane; j < min(st * SC + SC, ln_col); j += kWarp)
-          acc = fma_rn(widen(ld_stream(row_at(r) + j, pol)), __ldg(x + j), acc);
+          acc = fma_rn(widen(ld_stream(row_at(r) + j, pol)), x[j], acc);
       acc = warp_sum(acc);
       if (lane / (kWarp / R) == r) mine = acc;
     }
@@ -567,11 +567,11 @@ cudaError_t dense_values_df_range(const void* vals, int prec, size_t n, int* fla
 
 namespace {
 template <class V, int R, bool VEC>
-void launch_dense_df(const V* a, int ln_row, int ln_col, int log2s, const float* xs, const double* x, const int* bad,
+cudaError_t launch_dense_df(const V* a, int ln_row, int ln_col, int log2s, const float* xs, const double* x, const int* bad,
                      int nbad, double* y, int fresh, cudaStream_t s) {
   const long warps = (((long)ln_row + R - 1) / R) << log2s;
   const unsigned grid = (unsigned)((warps + NT / kWarp - 1) / (NT / kWarp));
-  k_dense_df<V, R, VEC><<<grid, NT, 0, s>>>(a, ln_row, ln_col, log2s, xs, x, bad, nbad, y, fresh);
+  return launch_early(k_dense_df<V, R, VEC>, grid, NT, 0, s, a, ln_row, ln_col, log2s, xs, x, bad, nbad, y, fresh);
 }
 
 // Rows per warp: 4 (FP32) or 2 (the others, whose rows cost more registers a
@@ -586,7 +586,7 @@ void launch_dense_df(const V* a, int ln_row, int ln_col, int log2s, const float*
 // rows, 2 / 4 / 8 parts: 5120 columns 133 / 132 / 144 us, 16384 columns 396 /
 // 381 / 384).
 template <class V, bool VEC>
-void dense_df_shape(const V* a, int ln_row, int ln_col, const float* xs, const double* x, const int* bad, int nbad,
+cudaError_t dense_df_shape(const V* a, int ln_row, int ln_col, const float* xs, const double* x, const int* bad, int nbad,
                     double* y, int fresh, cudaStream_t s) {
   constexpr int kMost = sizeof(V) == 4 ? 4 : 2;
   constexpr long kWarps = 152L * 32;
@@ -599,22 +599,22 @@ void dense_df_shape(const V* a, int ln_row, int ln_col, const float* xs, const d
   int log2s = 0;
   while (log2s < most && (((long)ln_row + r - 1) / r << log2s) < 4 * kWarps) log2s++;
   if (sizeof(V) == 8 && VEC && nsteps >= 40) log2s = std::max(log2s, 2);
-  if (r == 1) launch_dense_df<V, 1, VEC>(a, ln_row, ln_col, log2s, xs, x, bad, nbad, y, fresh, s);
-  else if (r == 2) launch_dense_df<V, 2, VEC>(a, ln_row, ln_col, log2s, xs, x, bad, nbad, y, fresh, s);
-  else if constexpr (kMost >= 4) launch_dense_df<V, 4, VEC>(a, ln_row, ln_col, log2s, xs, x, bad, nbad, y, fresh, s);
+  if (r == 1) return launch_dense_df<V, 1, VEC>(a, ln_row, ln_col, log2s, xs, x, bad, nbad, y, fresh, s);
+  if constexpr (kMost >= 4)
+    if (r == 4) return launch_dense_df<V, 4, VEC>(a, ln_row, ln_col, log2s, xs, x, bad, nbad, y, fresh, s);
+  return launch_dense_df<V, 2, VEC>(a, ln_row, ln_col, log2s, xs, x, bad, nbad, y, fresh, s);
 }
 
 template <class V>
-void dense_df_vec(const void* vals, int ln_row, int ln_col, const float* xs, const double* x, const int* bad, int nbad,
+cudaError_t dense_df_vec(const void* vals, int ln_row, int ln_col, const float* xs, const double* x, const int* bad, int nbad,
                   double* y, int fresh, cudaStream_t s) {
   const V* a = static_cast<const V*>(vals);
   // NV values per lane and load when every row starts on a 16-byte boundary
   // and holds whole vectors (xs from cudaMalloc)
   constexpr int NV = Step<V, true>::NV;
   if ((uintptr_t)vals % 16 == 0 && (uintptr_t)xs % 16 == 0 && ln_col % NV == 0)
-    dense_df_shape<V, true>(a, ln_row, ln_col, xs, x, bad, nbad, y, fresh, s);
-  else
-    dense_df_shape<V, false>(a, ln_row, ln_col, xs, x, bad, nbad, y, fresh, s);
+    return dense_df_shape<V, true>(a, ln_row, ln_col, xs, x, bad, nbad, y, fresh, s);
+  return dense_df_shape<V, false>(a, ln_row, ln_col, xs, x, bad, nbad, y, fresh, s);
 }
 }  // namespace
 
@@ -622,12 +622,12 @@ cudaError_t dense_gemv_df(const void* vals, int prec, int ln_row, int ln_col, co
                           int* bad, double* y, bool fresh, cudaStream_t s) {
   if (ln_row == 0 || ln_col == 0) return cudaSuccess;
   const int nbad = std::min((ln_col + NT - 1) / NT, kDenseFlags);
-  k_df_split_x<<<nbad, NT, 0, s>>>(x, ln_col, xs, bad);
+  cudaError_t e = launch_early(k_df_split_x, nbad, NT, 0, s, x, ln_col, xs, bad);
+  if (e != cudaSuccess) return e;
   const int f = fresh ? 1 : 0;
-  if (prec == kF64) dense_df_vec<double>(vals, ln_row, ln_col, xs, x, bad, nbad, y, f, s);
-  else if (prec == kF32) dense_df_vec<float>(vals, ln_row, ln_col, xs, x, bad, nbad, y, f, s);
-  else dense_df_vec<__nv_bfloat16>(vals, ln_row, ln_col, xs, x, bad, nbad, y, f, s);
-  return cudaGetLastError();
+  if (prec == kF64) return dense_df_vec<double>(vals, ln_row, ln_col, xs, x, bad, nbad, y, f, s);
+  if (prec == kF32) return dense_df_vec<float>(vals, ln_row, ln_col, xs, x, bad, nbad, y, f, s);
+  return dense_df_vec<__nv_bfloat16>(vals, ln_row, ln_col, xs, x, bad, nbad, y, f, s);
 }
 
 cudaError_t vec_add(double* y, const double* x, long n, cudaStream_t s) {

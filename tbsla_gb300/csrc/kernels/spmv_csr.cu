@@ -51,13 +51,13 @@ struct EpiStore {
 };
 
 template <class V, int ITEMS>
-__global__ void __launch_bounds__(NT) k_csr_spmv(CsrArgs a, const double* __restrict__ x,
-                                                double* __restrict__ y, int add) {
+__global__ void __launch_bounds__(NT) k_csr_spmv(CsrArgs a, const double* x, double* y, int add) {
   extern __shared__ __align__(16) unsigned char stage[];
   __shared__ Smem sm;
+  wait_for_earlier();
   const uint64_t pol = policy_evict_first();
   EpiStore epi{y, add};
-  csr_block<V, ITEMS>(a, blockIdx.x, x, epi, nullptr, stage, sm, pol);
+  csr_block<V, ITEMS, EpiStore, true>(a, blockIdx.x, x, epi, nullptr, stage, sm, pol);
 }
 
 template <class V, int ITEMS>
@@ -539,8 +539,7 @@ cudaError_t launch_spmv(const CsrArgs& a, const double* x, double* y, bool add, 
   constexpr size_t smem = stage_bytes<V, ITEMS>();
   cudaError_t ready = smem_opt_in<k_csr_spmv<V, ITEMS>>(smem);
   if (ready != cudaSuccess) return ready;
-  k_csr_spmv<V, ITEMS><<<a.nblocks, NT, smem, s>>>(a, x, y, add ? 1 : 0);
-  return cudaGetLastError();
+  return launch_early(k_csr_spmv<V, ITEMS>, a.nblocks, NT, smem, s, a, x, y, add ? 1 : 0);
 }
 
 template <class V>

@@ -49,9 +49,9 @@ constexpr unsigned FULL = 0xffffffffu;
 // K steps of one lane's row: predicated loads (lanes past their row's end
 // issue none, so padding costs no traffic), the K gathers of x in flight
 // together, then K full-warp DFMAs (dead lanes add a finite value times 0).
-template <class V, int K>
+template <class V, int K, bool LATE>
 __device__ __forceinline__ double steps_k(const V* __restrict__ sv, const int* __restrict__ sc, long off, int j,
-                                          int steps, const double* __restrict__ x, int f_col, uint64_t pol,
+                                          int steps, const double* x, int f_col, uint64_t pol,
                                           double acc) {
   V v[K];
   int c[K];
@@ -69,7 +69,7 @@ __device__ __forceinline__ double steps_k(const V* __restrict__ sv, const int* _
   }
   double xv[K];
 #pragma unroll
-  for (int u = 0; u < K; u++) xv[u] = (j + u < steps) ? ld_gather(x + c[u] - f_col) : 0.0;
+  for (int u = 0; u < K; u++) xv[u] = (j + u < steps) ? gather<LATE>(x + c[u] - f_col) : 0.0;
   __syncwarp();
 #pragma unroll
   for (int u = 0; u < K; u++) acc = fma_rn(widen(v[u]), xv[u], acc);
@@ -84,14 +84,14 @@ __device__ __forceinline__ double steps_k(const V* __restrict__ sv, const int* _
 // latency (the gathers), not for two (the columns, then the gathers).  It
 // costs 9 registers (FP64: 71 -> 80, still 3 CTAs per SM; FP32 values would
 // drop from 4 CTAs per SM to 3, which loses more than the overlap gains).
-template <class V, int U>
+template <class V, int U, bool LATE>
 __device__ __forceinline__ double slice_rows(const V* __restrict__ sv, const int* __restrict__ sc, long off,
-                                             int steps, int width, const double* __restrict__ x, int f_col,
+                                             int steps, int width, const double* x, int f_col,
                                              uint64_t pol) {
   double acc = 0;
   int j = 0;
   if (sizeof(V) != 8) {
-    for (; j + U <= width; j += U) acc = steps_k<V, U>(sv, sc, off, j, steps, x, f_col, pol, acc);
+    for (; j + U <= width; j += U) acc = steps_k<V, U, LATE>(sv, sc, off, j, steps, x, f_col, pol, acc);
   } else if (U <= width) {
     int cn[U];
 #pragma unroll
@@ -102,7 +102,7 @@ __device__ __forceinline__ double slice_rows(const V* __restrict__ sv, const int
 #pragma unroll
       for (int u = 0; u < U; u++) {
         const bool live = j + u < steps;
-        xv[u] = live ? ld_gather(x + cn[u] - f_col) : 0.0;
+        xv[u] = live ? gather<LATE>(x + cn[u] - f_col) : 0.0;
         v[u] = live ? ld_stream(sv + off + (long)(j + u) * 32, pol) : V(0.0f);
       }
       const bool more = j + 2 * U <= width;
@@ -116,18 +116,18 @@ __device__ __forceinline__ double slice_rows(const V* __restrict__ sv, const int
   }
   // remainder (< U steps) in binary pieces
   if (U > 8 && j + 8 <= width) {
-    acc = steps_k<V, 8>(sv, sc, off, j, steps, x, f_col, pol, acc);
+    acc = steps_k<V, 8, LATE>(sv, sc, off, j, steps, x, f_col, pol, acc);
     j += 8;
   }
   if (U > 4 && j + 4 <= width) {
-    acc = steps_k<V, 4>(sv, sc, off, j, steps, x, f_col, pol, acc);
+    acc = steps_k<V, 4, LATE>(sv, sc, off, j, steps, x, f_col, pol, acc);
     j += 4;
   }
   if (j + 2 <= width) {
-    acc = steps_k<V, 2>(sv, sc, off, j, steps, x, f_col, pol, acc);
+    acc = steps_k<V, 2, LATE>(sv, sc, off, j, steps, x, f_col, pol, acc);
     j += 2;
   }
-  if (j < width) acc = steps_k<V, 1>(sv, sc, off, j, steps, x, f_col, pol, acc);
+  if (j < width) acc = steps_k<V, 1, LATE>(sv, sc, off, j, steps, x, f_col, pol, acc);
   return acc;
 }
 
@@ -222,11 +222,15 @@ __device__ __forceinline__ bool cut_row_done(const SellPlan& p, int piece, int l
 //
 // CUT: the plan has cut rows (their test alone costs one without them 0.3%:
 // 1.208 against 1.204 ms at n = 2^24).
-template <class V, int U, bool PR, bool CUT>
+//
+// LATE: launched with launch_early.  Of several plans, whose gathers miss more,
+// the launches are ordinary ones and gather through the read-only path (n =
+// 2^24: 1.201 against 1.215 ms).
+template <class V, int U, bool PR, bool CUT, bool LATE>
 __global__ void __launch_bounds__(NT) k_sell(SellPlan p, const V* __restrict__ sv, const int* __restrict__ sc,
-                                            int f_col, int accumulate, const double* __restrict__ x,
-                                            double* __restrict__ y, unsigned* __restrict__ counter,
-                                            const int* __restrict__ done, PageRankArgs pr, Ctl ctl) {
+                                            int f_col, int accumulate, const double* x, double* y, unsigned* counter,
+                                            const int* done, PageRankArgs pr, Ctl ctl) {
+  if (LATE) wait_for_earlier();
   // a set done flag (an iteration that has converged) makes the launch a
   // no-op; no warp has touched the counters then
   if (done && *(volatile const int*)done) return;
@@ -274,7 +278,7 @@ __global__ void __launch_bounds__(NT) k_sell(SellPlan p, const V* __restrict__ s
     const Lane l = slice_lane(p, d, meta, cur, lane);
     bool head = l.row >= 0 && (lane & ((1 << d.z) - 1)) == 0;
     const double y0 = (!PR && accumulate && head) ? y[l.row] : 0.0;  // issued before the sum
-    double acc = slice_rows<V, U>(sv, sc, (long)d.x * 32 + lane, l.steps, d.y, x, f_col, pol);
+    double acc = slice_rows<V, U, LATE>(sv, sc, (long)d.x * 32 + lane, l.steps, d.y, x, f_col, pol);
     for (int o = (1 << d.z) >> 1; o > 0; o >>= 1) acc = add_rn(acc, __shfl_xor_sync(FULL, acc, o));
     if (CUT && d.w < -1) {  // a piece of a cut row
       const int piece = -2 - d.w;
@@ -366,7 +370,7 @@ cudaError_t launch(const SellArgs& a, const double* x, double* y, unsigned* coun
   int dev = 0, sms = 0, per = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_sell<V, U, false, true>, NT, 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_sell<V, U, false, true, true>, NT, 0);
   const int grid = std::max(1, sms * std::max(1, per));
   const bool fork = a.side && a.parts > 1 && a.nblocks >= a.parts;
   const int first_part = a.nblocks - a.parts;
@@ -383,10 +387,18 @@ cudaError_t launch(const SellArgs& a, const double* x, double* y, unsigned* coun
     if (e == cudaSuccess && k > 0) e = cudaStreamWaitEvent(ls, a.fork, 0);
     if (e == cudaSuccess && a.ready && b > 0) e = cudaStreamWaitEvent(ls, a.ready[b], 0);
     if (e == cudaSuccess && p.nslices > 0) {
-      const auto kernel = p.ncut > 0 ? k_sell<V, U, false, true> : k_sell<V, U, false, false>;
-      kernel<<<pg, NT, 0, ls>>>(p, static_cast<const V*>(a.svals), a.scols, a.f_col, b > 0 || a.add ? 1 : 0, x, y,
-                                counter + k * kSellCounterRegion, done, PageRankArgs{}, Ctl{});
-      e = cudaGetLastError();
+      const V* sv = static_cast<const V*>(a.svals);
+      const int add = b > 0 || a.add ? 1 : 0;
+      unsigned* region = counter + k * kSellCounterRegion;
+      // several plans: their launches wait on events, an ordinary launch
+      if (a.nblocks == 1) {
+        const auto kernel = p.ncut > 0 ? k_sell<V, U, false, true, true> : k_sell<V, U, false, false, true>;
+        e = launch_early(kernel, pg, NT, 0, ls, p, sv, a.scols, a.f_col, add, x, y, region, done, PageRankArgs{}, Ctl{});
+      } else {
+        const auto kernel = p.ncut > 0 ? k_sell<V, U, false, true, false> : k_sell<V, U, false, false, false>;
+        kernel<<<pg, NT, 0, ls>>>(p, sv, a.scols, a.f_col, add, x, y, region, done, PageRankArgs{}, Ctl{});
+        e = cudaGetLastError();
+      }
     }
     // recorded for an empty plan too: the event then marks the earlier plans
     if (e == cudaSuccess && a.after && a.after[b]) e = cudaEventRecord(a.after[b], ls);
@@ -424,12 +436,11 @@ cudaError_t launch_pr(const SellArgs& a, const double* x, double* y, const PageR
   int dev = 0, sms = 0, per = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_sell<V, U, true, true>, NT, 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_sell<V, U, true, true, true>, NT, 0);
   const SellPlan& p = a.blocks[0];
   const int grid = std::max(1, std::min(sms * std::max(1, std::min(per, 8)), (p.nslices + NT / 32 - 1) / (NT / 32)));
-  k_sell<V, U, true, true><<<grid, NT, 0, s>>>(p, static_cast<const V*>(a.svals), a.scols, a.f_col, 0, x, y, nullptr,
-                                         pr.done, pr, ctl);
-  return cudaGetLastError();
+  return launch_early(k_sell<V, U, true, true, true>, grid, NT, 0, s, p, static_cast<const V*>(a.svals), a.scols, a.f_col, 0,
+                      x, y, nullptr, pr.done, pr, ctl);
 }
 
 template <class V>

@@ -29,7 +29,8 @@ constexpr int NT = 64;
 template <class V, bool SHIFT>
 __global__ void __launch_bounds__(NT) k_ell(const V* __restrict__ vals, const int* __restrict__ cols,
                                            int ln_row, int max_col, int f_col,
-                                           const double* __restrict__ x, double* __restrict__ y) {
+                                           const double* x, double* y) {
+  wait_for_earlier();
   const int i = blockIdx.x * NT + threadIdx.x;
   if (i >= ln_row) return;
   const uint64_t pol = policy_evict_first();
@@ -47,7 +48,7 @@ __global__ void __launch_bounds__(NT) k_ell(const V* __restrict__ vals, const in
     }
     double xv[4];
 #pragma unroll
-    for (int u = 0; u < 4; u++) xv[u] = ld_gather(x + c[u]);
+    for (int u = 0; u < 4; u++) xv[u] = ld_gather_late(x + c[u]);
 #pragma unroll
     for (int u = 0; u < 4; u++) acc = add_rn(acc, mul_rn(v[u], xv[u]));
   }
@@ -55,7 +56,7 @@ __global__ void __launch_bounds__(NT) k_ell(const V* __restrict__ vals, const in
     const size_t k = (size_t)j * ln_row + i;
     int c = ld_stream(cols + k, pol) - f_col;
     if (SHIFT && c < 0) c = 0;
-    acc = add_rn(acc, mul_rn(widen(ld_stream(vals + k, pol)), ld_gather(x + c)));
+    acc = add_rn(acc, mul_rn(widen(ld_stream(vals + k, pol)), ld_gather_late(x + c)));
   }
   y[i] = acc;
 }
@@ -77,10 +78,8 @@ cudaError_t launch(const void* vals, const int* cols, int ln_row, int max_col, i
                    const double* x, double* y, cudaStream_t s) {
   const int grid = (ln_row + NT - 1) / NT;
   if (f_col != 0)
-    k_ell<V, true><<<grid, NT, 0, s>>>(static_cast<const V*>(vals), cols, ln_row, max_col, f_col, x, y);
-  else
-    k_ell<V, false><<<grid, NT, 0, s>>>(static_cast<const V*>(vals), cols, ln_row, max_col, 0, x, y);
-  return cudaGetLastError();
+    return launch_early(k_ell<V, true>, grid, NT, 0, s, static_cast<const V*>(vals), cols, ln_row, max_col, f_col, x, y);
+  return launch_early(k_ell<V, false>, grid, NT, 0, s, static_cast<const V*>(vals), cols, ln_row, max_col, 0, x, y);
 }
 
 }  // namespace
