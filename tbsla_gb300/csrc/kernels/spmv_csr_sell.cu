@@ -300,8 +300,10 @@ __global__ void __launch_bounds__(NT) k_sell(SellPlan p, const V* __restrict__ s
       cur = nxt;
       nxt += nwarps;
     } else {
-      // (adding: a row without entries is not touched)
-      if (head && (l.len > 0 || !accumulate)) y[l.row] = accumulate ? add_rn(y0, acc) : acc;
+      // adding: a zero sum leaves y as it is, so a row without entries is not
+      // touched (a test of l.len costs a register across the sum: 1.3% at 2^24)
+      if (head && !(accumulate && (__double_as_longlong(acc) << 1) == 0))
+        y[l.row] = accumulate ? add_rn(y0, acc) : acc;
       if (lane == 0) after = cl.resolve(after);
       cur = nxt;
       nxt = __shfl_sync(FULL, after, 0);
