@@ -193,9 +193,11 @@ int tbsla_matrix_kernel_launches(const tbsla_matrix* m, int* launches);
  * gain by more blocks); changing it rebuilds the partition. */
 int tbsla_matrix_set_csr_tile(tbsla_matrix* m, int nnz_per_block);
 /* CSR SpMV kernel: TBSLA_CSR_AUTO (default: row blocks below 2^19 stored
- * entries, where one short launch is latency-bound, else sliced ELL),
+ * entries, and below 3 2^20 without rows of more than 64, where one short
+ * launch is latency-bound, else sliced ELL; PageRank on sliced ELL at every
+ * size),
  * TBSLA_CSR_SELL (sliced-ELL device layout, slices of 32 lanes over rows of
- * similar length, see tbsla_matrix_set_sell_params; `items` = steps per
+ * similar length, long rows in pieces, see tbsla_matrix_set_sell_params; `items` = steps per
  * lane in flight, 4/8/16, 0 = 8), TBSLA_CSR_MERGE (merge-path split,
  * `items` row ends + entries per thread, 4/8/16, 0 = 8) or
  * TBSLA_CSR_ROWBLOCK (row-block adaptive, see
@@ -223,11 +225,11 @@ int tbsla_matrix_set_sell_params(tbsla_matrix* m, int short_thr, int long_thr, i
 /* Batched personalised PageRank with FP32 / BF16 values: gathers of X rows
  * in flight per warp, 8 (default) or 16; a tuning choice, same results. */
 int tbsla_matrix_set_pagerank_gather(tbsla_matrix* m, int gather);
-/* Batched PageRank with FP32 / BF16 values: 1 (default) a warp takes a
- * whole row block and walks its entries as one stream, `gather` X rows in
- * flight across row boundaries; 0 a warp per row.  The same Y bit for bit
- * (each row sums in entry order either way); the norms' partial sums are
- * added in another order.  The row-block form keeps X row offsets in 32
+/* Batched PageRank: 1 (default) a warp takes an item of about equal work (a
+ * run of rows, or a piece of a long one) and walks its entries as one stream,
+ * `gather` X rows in flight across row boundaries; 0 a warp per row (FP32 /
+ * BF16 values).  The same Y up to rounding; the norms' partial sums are
+ * added in another order.  The stream form keeps X row offsets in 32
  * bits, so with n_col * nvec >= 2^31 the warp-per-row form runs whatever
  * this setting.  No reference counterpart. */
 int tbsla_matrix_set_pagerank_stream(tbsla_matrix* m, int stream);

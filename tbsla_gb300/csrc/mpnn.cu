@@ -790,8 +790,8 @@ __global__ void k_adam(int np, float* __restrict__ theta, const float* __restric
 // feature-major, hT[f * n + i], so that a thread per node reads and writes
 // them coalesced across its warp (32 consecutive nodes, 128 bytes per
 // feature).  Every kernel does the FP32 operations of the training path's
-// kernels (k_layer0, k_aggregate + k_layer, k_head) in the same order, so the
-// factor is bit-identical to tbsla_mpnn_factor's.
+// kernels (k_layer0, k_gather + k_layer, k_head), so the factor is
+// tbsla_mpnn_factor's up to the order of FP32 sums.
 
 constexpr int DMAX = 8;  // diagonal slots per system
 

@@ -95,3 +95,65 @@ def test_captured(gpu, kind, n):
             work(side.cuda_stream)
         torch.cuda.synchronize()
         assert torch.equal(got, r) and r.abs().max() > 0
+
+
+@pytest.mark.parametrize("captured", [False, True])
+@pytest.mark.parametrize("kind,n", CASES)
+def test_two_streams(gpu, kind, n, captured):
+    """Two matrices on two streams that wait for one another by events: each
+    product reads what the other stream wrote, behind a slow kernel there."""
+    torch = pytest.importorskip("torch")
+    m, w = matrix(gpu, kind, n), matrix(gpu, kind, n)
+    m.upload()
+    w.upload()
+    x = torch.linspace(-1, 1, n, dtype=torch.float64, device="cuda")
+    src, a, b, c, d = (x.clone() for _ in range(5))
+    big = torch.ones(1 << 25, device="cuda")
+    s1, s2 = torch.cuda.Stream(), torch.cuda.Stream()
+
+    def work():
+        with torch.cuda.stream(s1):
+            for _ in range(4):
+                big.mul_(1.0)
+            m.spmv_device(a, src, stream=s1.cuda_stream)
+            e1 = torch.cuda.Event()
+            e1.record(s1)
+        with torch.cuda.stream(s2):
+            s2.wait_event(e1)
+            w.spmv_device(b, a, stream=s2.cuda_stream)  # a: from s1
+            for _ in range(4):
+                big.mul_(1.0)
+            w.spmv_device(c, b, stream=s2.cuda_stream)
+            e2 = torch.cuda.Event()
+            e2.record(s2)
+        with torch.cuda.stream(s1):
+            m.spmv_device(d, a, stream=s1.cuda_stream)
+            s1.wait_event(e2)
+            m.spmv_device(d, c, stream=s1.cuda_stream)  # c: from s2
+
+    torch.cuda.synchronize()
+    if captured:
+        work()
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.stream(s1):
+            graph.capture_begin()
+            work()
+            graph.capture_end()
+    for scale in (1.0, -3.0, 0.5):
+        for t in (a, b, c, d):
+            t.fill_(7.0)
+        src.copy_(x * scale)
+        torch.cuda.synchronize()
+        graph.replay() if captured else work()
+        torch.cuda.synchronize()
+        want = src
+        for _ in range(3):
+            t = torch.empty_like(x)
+            m.spmv_device(t, want, stream=s1.cuda_stream)
+            torch.cuda.synchronize()
+            want = t
+        last = torch.empty_like(x)
+        m.spmv_device(last, c, stream=s1.cuda_stream)
+        torch.cuda.synchronize()
+        assert torch.equal(c, want) and torch.equal(d, last) and d.abs().max() > 0
