@@ -441,7 +441,7 @@ def run_ours(a):
                    "format": "CSR", "n": n, "nnz": nnz, "value_dtype": a.prec, "x_y_dtype": "f64",
                    "bytes_per_step": B, "csr_kernel": a.algo, "autotune": tuned,
                    "work_split": {"merge": f"{a.items} items/thread", "rowblock": f"{a.tile} nnz/block",
-                                  "sell": f"one lane per row <= {a.sell.split(',')[0] if a.sell.split(',')[0] != '0' else 'auto (128 for FP64 with column blocks, else 64)'} sorted per "
+                                  "sell": f"one lane per row <= {a.sell.split(',')[0] if a.sell.split(',')[0] != '0' else 'auto (128 for FP64 with column blocks, 64 for others, 16 to 64 by size with one block)'} sorted per "
                                           f"{a.sell.split(',')[2]}-row window, else 2..32 lanes per row, slices "
                                           f"<= {a.sell.split(',')[1] if a.sell.split(',')[1] != '0' else 'the same'} steps; "
                                           f"{a.items or 'automatic'} steps/lane in flight; "

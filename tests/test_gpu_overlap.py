@@ -3,6 +3,9 @@ products in which each reads what the one before wrote, and writes what that
 one read, against the same products with a synchronisation after each, and
 inside a captured graph behind a copy and a memset.  Bit for bit: the kernels
 sum in a fixed order."""
+import contextlib
+import gc
+
 import numpy as np
 import pytest
 
@@ -29,6 +32,27 @@ def matrix(T, kind, n):
     if kind == "sell":
         m.set_algorithm(m.SELL)
     return m
+
+
+@contextlib.contextmanager
+def capture(torch, stream):
+    """A graph captured on `stream`; matrices that other tests left to the
+    collector are freed before, not during the capture (a free ends it)."""
+    gc.collect()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    enabled = gc.isenabled()
+    gc.disable()
+    try:
+        with torch.cuda.stream(stream):
+            graph.capture_begin()
+            try:
+                yield graph
+            finally:
+                graph.capture_end()
+    finally:
+        if enabled:
+            gc.enable()
 
 
 CASES = [("csr", 300), ("csr", 40_000), ("sell", 300), ("sell", 40_000), ("sell", 400_000), ("coo", 2000), ("coo", 400_000),
@@ -78,13 +102,10 @@ def test_captured(gpu, kind, n):
         m.Ax_device(r, a, stream=stream)
         m.Ax_device(r, b, stream=stream)
 
-    graph = torch.cuda.CUDAGraph()
     with torch.cuda.stream(side):
         work(side.cuda_stream)
-        side.synchronize()
-        graph.capture_begin()
+    with capture(torch, side) as graph:
         work(side.cuda_stream)
-        graph.capture_end()
     for scale in (1.0, -3.0):
         src.copy_(x * scale)
         torch.cuda.synchronize()
@@ -134,12 +155,8 @@ def test_two_streams(gpu, kind, n, captured):
     torch.cuda.synchronize()
     if captured:
         work()
-        torch.cuda.synchronize()
-        graph = torch.cuda.CUDAGraph()
-        with torch.cuda.stream(s1):
-            graph.capture_begin()
+        with capture(torch, s1) as graph:
             work()
-            graph.capture_end()
     for scale in (1.0, -3.0, 0.5):
         for t in (a, b, c, d):
             t.fill_(7.0)
