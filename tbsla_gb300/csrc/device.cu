@@ -391,6 +391,13 @@ int build_sell(const tbsla_matrix* m, DeviceMatrix* d, int n, int nc, int f_col,
   const int one = nz < (1L << 22) || (nz < (1L << 23) && by <= 16) ? 16 : nz < (1L << 25) && by <= 32 ? 32 : 64;
   const int sthr = m->sell_short > 0 ? m->sell_short : P == 1 ? one : d->prec == TBSLA_F64 ? 128 : 64;
   const int lthr = m->sell_long > 0 ? m->sell_long : sthr;
+  // FP64 values, one block, from 2^22 entries: pieces of twice long_thr, since
+  // shorter ones join more sums than they spread (power-law rows, 45 10^6
+  // entries: 1x 203 us, 2x 198, uncut 198; 39 10^6: 143, 140, 140; 4 10^6: 29.9,
+  // 27.8, 34.8).  Below, and with the narrow types, whose PageRank steps deal
+  // their slices statically, as long as the slices (FP32 59.6 10^6, a step: 1x 300
+  // us, 2x 322; FP64 2 10^6: 20.5, 21.9).
+  const int piece = P == 1 && m->sell_long <= 0 && d->prec == TBSLA_F64 && nz >= (1L << 22) ? 2 * lthr : lthr;
   long steps = 0;
   d->sell.assign(P - 1 + R, SellPlan{});
   int st = TBSLA_OK;
@@ -405,7 +412,7 @@ int build_sell(const tbsla_matrix* m, DeviceMatrix* d, int n, int nc, int f_col,
       L = part.data();
     }
     SellPlan hp;
-    sell_plan_build(L, n, sthr, lthr, m->sell_sigma, blk > 0, steps, &hp);
+    sell_plan_build(L, n, sthr, lthr, piece, m->sell_sigma, blk > 0, steps, &hp);
     hp.col_lo = blk * W;
     hp.col_hi = blk == P - 1 ? INT_MAX : (blk + 1) * W;
     hp.row_lo = blk == P - 1 ? r0 : 0;

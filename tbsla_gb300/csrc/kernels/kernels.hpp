@@ -108,9 +108,10 @@ struct SellPlan {
 constexpr int kRowParts = 2;
 // Host: plan of one column block from its per-row entry counts L[n]
 // (arrays allocated with new[]); rows with no entry are left out when
-// skip_empty; step offsets start at step0.
-void sell_plan_build(const int* L, int n, int short_thr, int long_thr, int sigma, bool skip_empty, long step0,
-                     SellPlan* p);
+// skip_empty; step offsets start at step0; a row that 32 lanes would walk in
+// more than `piece` steps is cut into pieces of at most that many.
+void sell_plan_build(const int* L, int n, int short_thr, int long_thr, int piece, int sigma, bool skip_empty,
+                     long step0, SellPlan* p);
 void sell_plan_free(SellPlan* p);
 struct SellArgs {
   const void* vals;  // CSR copy (the slice arrays are filled from it)

@@ -467,13 +467,14 @@ cudaError_t launch_u(const SellArgs& a, const double* x, double* y, unsigned* co
 
 }  // namespace
 
-void sell_plan_build(const int* L, int n, int sthr, int lthr, int sigma, bool skip_empty, long step0,
+void sell_plan_build(const int* L, int n, int sthr, int lthr, int piece, int sigma, bool skip_empty, long step0,
                      SellPlan* p) {
   using tbsla_impl::parallel_for_items;
   *p = SellPlan{};
   p->n = n;
   sthr = std::max(1, std::min(sthr, 255));
   lthr = std::max(lthr, 1);
+  piece = std::max(piece, lthr);
   sigma = std::max(32, std::min(sigma, 1 << 23));
   auto len = [&](int i) { return L[i]; };
   // lanes per row (log2) of a row longer than short_thr
@@ -520,10 +521,10 @@ void sell_plan_build(const int* L, int n, int sthr, int lthr, int sigma, bool sk
     auto& v = lng[g];
     sort_wide(v);
     const int per = 32 >> g;
-    // a row past 32 * long_thr entries: equal pieces, whole steps each
+    // a row past 32 * piece entries: equal pieces, whole steps each
     size_t q0 = 0;
-    for (; g == 5 && q0 < v.size() && (len(v[q0]) + 31) >> 5 > lthr; q0++) {
-      const int l = len(v[q0]), steps = (l + 31) >> 5, np = (steps + lthr - 1) / lthr;
+    for (; g == 5 && q0 < v.size() && (len(v[q0]) + 31) >> 5 > piece; q0++) {
+      const int l = len(v[q0]), steps = (l + 31) >> 5, np = (steps + piece - 1) / piece;
       const int size = 32 * ((steps + np - 1) / np);
       cut_first.push_back((int)piece_at.size());
       for (int at = 0; at < l; at += size) {

@@ -3,7 +3,8 @@ at which a row forms a block on its own, among blocks of each lane count,
 against the oracle.
 
 Tolerance: the FP64 bar of test_gpu_spmv.py, 1e-13 of sum_j |a_ij x_j| per
-entry (rows of at most 1500 entries, one rounding of 1.1e-16 each)."""
+entry (rows of at most 1500 entries, one rounding of 1.1e-16 each; the longer
+rows of the last test add at most 64 entries a lane, then their pieces)."""
 import numpy as np
 import pytest
 
@@ -102,3 +103,26 @@ def test_page_rank_after_an_update(gpu):
     x, it, *_ = m.page_rank(beta=0.85)
     y, jt, *_ = fresh.page_rank(beta=0.85)
     assert it == jt and np.array_equal(x, y) and not np.array_equal(x, first)
+
+
+@pytest.mark.parametrize("prec", ["f64", "f32"])
+def test_long_rows_by_size(gpu, prec):
+    """2^22 entries and more, where FP64 rows are cut into longer pieces: rows
+    around one and two pieces of 32 lanes x 32 and x 64 steps."""
+    T = gpu
+    n = 600_000
+    rng = np.random.default_rng(22)
+    lens = np.full(n, 8)
+    lens[rng.choice(n, 10, replace=False)] = (1023, 1024, 1025, 2047, 2048, 2049, 4096, 4097, 8193, 70_001)
+    rp = np.concatenate(([0], np.cumsum(lens)))
+    ci = rng.integers(0, n, rp[-1])
+    v = rng.uniform(-1, 1, rp[-1])
+    m = T.MatrixCSR.from_arrays(n, n, rp, ci, v)
+    m.set_precision({"f64": T.F64, "f32": T.F32}[prec])
+    w = v if prec == "f64" else v.astype(np.float32).astype(np.float64)
+    x = rng.uniform(-1, 1, n)
+    a = m.arrays()
+    y = m.spmv(x)
+    ref = oracle.csr_ax(a["rowptr"], a["colidx"], w, x)
+    assert oracle.rel_err_normalized(y, ref, oracle.csr_absrow(a["rowptr"], a["colidx"], w, x)) <= TOL
+    assert np.array_equal(m.spmv(x), y)
