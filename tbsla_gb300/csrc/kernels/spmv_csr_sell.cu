@@ -19,13 +19,14 @@
 // consecutive words (256-byte coalesced loads) and no work item takes much
 // longer than another: one warp per slice, fetched dynamically, widest first.
 //
-// A row too long for 32 lanes in long_thr steps is cut into pieces, a slice
-// each, because a hub row on one warp was the critical path of the whole
+// A row that 32 lanes would walk in more than `piece` steps is cut into pieces, a
+// slice each, because a hub row on one warp was the critical path of the whole
 // launch: PageRank on a 2^22-node graph whose longest row holds 89,090 entries
-// went from 37.4 to 12.5 ms (36 steps), an SpMV of 10^6 power-law rows of up
-// to 7,400 entries (FP32 values) from 103.6 to 92.5 us.  long_thr is where
-// the cut lies because a slice of that width is the widest item the other
-// rows make, so a piece never takes longer than they do.
+// went from 37.4 to 12.5 ms by it (36 steps; 10.8 with the later changes), an
+// SpMV of 10^6 power-law rows of up to 7,400 entries (FP32 values) from 103.6 to
+// 92.5 us (now 72).  `piece` is long_thr, the widest item the other rows make, so
+// a piece never takes longer than they do; twice that for large FP64 matrices,
+// where more pieces cost more than they spread.
 //
 // Each lane sums its entries in entry order with fused multiply-adds; G > 1
 // lanes of a row are combined by a fixed butterfly of additions.
