@@ -197,7 +197,10 @@ struct DeviceMatrix {
       int st = dalloc(&counter, 4);
       if (st) return st;
       TRY(cudaMemsetAsync(counter, 0, 4 * sizeof(unsigned), stream));
-      st = dalloc(&result, 256);
+    }
+    // on its own: a call that found no room for it leaves the counters behind
+    if (!result) {
+      const int st = dalloc(&result, 256);
       if (st) return st;
     }
     size_t need = std::max<size_t>(nred_per_cta * grid, (size_t)kSumBlocks * 32);

@@ -1,0 +1,135 @@
+"""Calls during which one allocation fails, on the device or on the host: the
+library's objects linked once more with cudaMalloc and operator new behind a
+counter, so that the n-th one of a call reports no room (no memory is taken).
+
+Each call either raises the library's out-of-memory error or gives the right
+answer by the path that needs less; the same call again, with room, is right,
+and the device bytes are those of the layout that is there."""
+import glob
+import json
+import os
+import subprocess
+import sys
+import textwrap
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+SHIM = r"""
+#include <cstddef>
+#include <new>
+typedef int cudaError_t;
+static thread_local int t_kind = 0, t_left = 0, t_hit = 0;
+static thread_local size_t t_min = 0;
+static bool fails(int kind, size_t n) {
+  if (t_kind != kind || n < t_min || t_left-- > 0) return false;
+  t_kind = 0;
+  t_hit = 1;
+  return true;
+}
+extern "C" {
+cudaError_t __real_cudaMalloc(void**, size_t);
+cudaError_t __wrap_cudaMalloc(void** p, size_t n) { return fails(1, n) ? 2 : __real_cudaMalloc(p, n); }
+void* __real__Znwm(size_t);
+void* __wrap__Znwm(size_t n) {
+  if (fails(2, n)) throw std::bad_alloc();
+  return __real__Znwm(n);
+}
+// kind 1: cudaMalloc, 2: operator new; the allocation after `skip` others of at least `min` bytes fails
+void shim_arm(int kind, int skip, size_t min) { t_kind = kind; t_left = skip; t_min = min; t_hit = 0; }
+int shim_hit() { t_kind = 0; return t_hit; }
+}
+"""
+
+CHILD = r"""
+import ctypes, json, sys
+sys.path.insert(0, {root!r})
+real = ctypes.CDLL
+ctypes.CDLL = lambda p, *a, **k: real({lib!r} if str(p).endswith("libtbsla_gb300.so") else p, *a, **k)
+import numpy as np
+import tbsla_gb300 as T
+import oracle
+shim = real({lib!r})
+shim.shim_arm.argtypes = [ctypes.c_int, ctypes.c_int, ctypes.c_size_t]
+T.device_init(0)
+
+def graph(n, extra, hub, seed):
+    rng = np.random.default_rng(seed)
+    row = np.concatenate((rng.integers(0, n, extra), np.full(hub, 3)))
+    col = rng.integers(0, n, len(row))
+    order = np.argsort(row, kind="stable")
+    row, col = row[order], col[order]
+    rp = np.concatenate(([0], np.cumsum(np.bincount(row, minlength=n)))).astype(np.int32)
+    return rp, col.astype(np.int32), 1.0 / np.bincount(col, minlength=n)[col], row.astype(np.int32)
+
+def sweep(make, call, right, kind, least):
+    # the n-th allocation of the call fails, for n = 0, 1, ... until none is left
+    out = []
+    for skip in range(200):
+        m = make()
+        shim.shim_arm(kind, skip, least)
+        try:
+            ok, err = right(call(m)), None
+        except T.TbslaError as e:
+            ok, err = None, e.status
+        if not shim.shim_hit():
+            assert ok
+            break
+        assert ok or err == -3, (skip, ok, err)
+        out.append(ok is not None)
+        for _ in range(2):
+            assert right(call(m)), skip
+        full = make()
+        call(full)
+        out[-1] = (out[-1], m.device_bytes(), full.device_bytes())
+    else:
+        raise AssertionError("no end")
+    return out
+{body}
+"""
+
+
+@pytest.fixture(scope="module")
+def lib(gpu, tmp_path_factory):
+    import importlib.util
+
+    spec = importlib.util.spec_from_file_location("_tbsla_build", os.path.join(ROOT, "tbsla_gb300", "build.py"))
+    b = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(b)
+    d = tmp_path_factory.mktemp("shim")
+    (d / "shim.cpp").write_text(SHIM)
+    subprocess.run(["g++", "-O1", "-fPIC", "-c", str(d / "shim.cpp"), "-o", str(d / "shim.o")], check=True)
+    objs = [o for o in glob.glob(os.path.join(b.BUILD, "*.o")) if os.path.basename(o).startswith("csrc_")]
+    assert objs
+    out = str(d / "libshim.so")
+    subprocess.run([b._nvcc(), *b.ARCH, "-shared", "-o", out, *objs, str(d / "shim.o"), "-lpthread",
+                    "-Xlinker", "--wrap=cudaMalloc", "-Xlinker", "--wrap=_Znwm"], check=True)
+    return out
+
+
+def run(lib, body):
+    src = CHILD.format(root=ROOT, lib=lib, body=textwrap.dedent(body))
+    r = subprocess.run([sys.executable, "-c", src], capture_output=True, text=True, timeout=600)
+    assert r.returncode == 0, r.stdout + r.stderr
+    return json.loads(r.stdout.strip().splitlines()[-1])
+
+
+def test_page_rank_scratch(lib):
+    """The iterates and control words of the row-block step: the second call
+    makes what the first had no room for."""
+    call = "m.page_rank(0.85, 1e-13, 60)[0]"
+    out = run(lib, f"""
+    rp, ci, v, _ = graph(3000, 20_000, 5000, 1)
+    ref = oracle.pagerank(rp, ci, v, beta=0.85, epsilon=1e-13, max_iterations=60)[0]
+    def make():
+        m = T.MatrixCSR.from_arrays(3000, 3000, rp, ci, v)
+        m.set_algorithm(m.ROWBLOCK)
+        m.kernel_launches()
+        return m
+    right = lambda y: bool(np.abs(y - ref).sum() <= 1e-11)
+    print(json.dumps(sweep(make, lambda m: {call}, right, 1, 1)))
+    """)
+    assert len(out) >= 6 and not any(ok for ok, _, _ in out)
+    assert all(b == full for _, b, full in out)
