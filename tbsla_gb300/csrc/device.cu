@@ -116,6 +116,7 @@ struct DeviceMatrix {
   size_t bx0_len = 0, bx1_len = 0, btele_len = 0, bw_len = 0, bcoef_len = 0;
   BatchPlan bplan;        // its work items, built at the first batched solve
   int bplan_budget = 0;
+  size_t bplan_bytes = 0;  // its share of `bytes`
   double* x = nullptr;
   size_t x_len = 0;
   double* y = nullptr;
@@ -1308,6 +1309,9 @@ int batch_plan(const tbsla_matrix* m, DeviceMatrix* d, int grid) {
   for (void* q : {(void*)b.item, (void*)b.piece_cut, (void*)b.cut_first, (void*)b.piece_sum, (void*)b.cut_done})
     if (q) cudaFree(q);
   b = BatchPlan{};
+  d->bytes -= d->bplan_bytes;
+  d->bplan_bytes = 0;
+  const size_t before = d->bytes;
   int st = upload_array(d, &b.item, items.data(), items.size());
   if (!st) st = upload_array(d, &b.piece_cut, cut.data(), cut.size());
   if (!st) st = upload_array(d, &b.cut_first, first.data(), first.size());
@@ -1318,11 +1322,13 @@ int batch_plan(const tbsla_matrix* m, DeviceMatrix* d, int grid) {
   if (st) {  // no plan: the next call builds it again
     if (b.item) cudaFree(b.item);
     b.item = nullptr;
+    d->bytes = before;
     return st;
   }
   b.nitems = (int)items.size();
   b.npieces = (int)cut.size();
   d->bplan_budget = budget;
+  d->bplan_bytes = d->bytes - before;
   return TBSLA_OK;
 }
 }  // namespace

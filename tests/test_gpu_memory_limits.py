@@ -116,13 +116,15 @@ def run(lib, body):
     return json.loads(r.stdout.strip().splitlines()[-1])
 
 
-def test_page_rank_scratch(lib):
-    """The iterates and control words of the row-block step: the second call
-    makes what the first had no room for."""
-    call = "m.page_rank(0.85, 1e-13, 60)[0]"
+@pytest.mark.parametrize("batched", [False, True])
+def test_page_rank_scratch(lib, batched):
+    """The iterates, control words and work items of the row-block steps: the
+    second call makes what the first had no room for."""
+    call = "m.page_rank_batched(tele, 0.85, 1e-13, 60)[0][:, 3]" if batched else "m.page_rank(0.85, 1e-13, 60)[0]"
     out = run(lib, f"""
     rp, ci, v, _ = graph(3000, 20_000, 5000, 1)
     ref = oracle.pagerank(rp, ci, v, beta=0.85, epsilon=1e-13, max_iterations=60)[0]
+    tele = np.full((3000, 8), 1 / 3000)
     def make():
         m = T.MatrixCSR.from_arrays(3000, 3000, rp, ci, v)
         m.set_algorithm(m.ROWBLOCK)
@@ -133,3 +135,23 @@ def test_page_rank_scratch(lib):
     """)
     assert len(out) >= 6 and not any(ok for ok, _, _ in out)
     assert all(b == full for _, b, full in out)
+
+
+def test_batched_plan_bytes(gpu):
+    """The work items of the batched step follow the gathers in flight (another
+    grid, another item size); their bytes are counted once."""
+    import numpy as np
+
+    T = gpu
+    n = 200_000
+    rng = np.random.default_rng(4)
+    rp = np.arange(0, 12 * n + 1, 12)
+    ci = rng.integers(0, n, 12 * n)
+    m = T.MatrixCSR.from_arrays(n, n, rp, ci, 1.0 / np.bincount(ci, minlength=n)[ci])
+    m.set_precision(T.F32)
+    seen = {}
+    for gather in (8, 16, 8, 16, 8):
+        m.set_pagerank_gather(gather)
+        m.page_rank_batched(np.full((n, 2), 1.0 / n), 0.85, 1e-3, 5)
+        seen.setdefault(gather, []).append(m.device_bytes())
+    assert len(set(seen[8])) == 1 and len(set(seen[16])) == 1 and seen[8][0] != seen[16][0]
