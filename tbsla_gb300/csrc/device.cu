@@ -20,6 +20,7 @@
 #include <cmath>
 #include <cstdint>
 #include <cstring>
+#include <new>
 #include <vector>
 
 #include "device.hpp"
@@ -98,6 +99,8 @@ struct DeviceMatrix {
   void* svals = nullptr;
   int* scols = nullptr;
   unsigned* sell_counter = nullptr;
+  bool sell_ready = false;  // the layout is complete (plans uploaded, slices filled)
+  bool no_pr_layout = false;  // PageRank's layout did not fit beside this copy: not tried again
   int sell_parts = 1;  // trailing plans that split the last column block by rows
   std::vector<cudaStream_t> side;  // row parts 1..: falling priorities
   cudaEvent_t fork_ev = nullptr;
@@ -141,9 +144,10 @@ struct DeviceMatrix {
         if (q) cudaFree(q);
     sell.clear();
   }
-  // a sliced-ELL layout that did not fit (nothing launched on it but fills)
+  // a sliced-ELL layout that was not finished (nothing launched on it but fills)
   void free_sell() {
     if (stream) cudaStreamSynchronize(stream);
+    sell_ready = false;
     free_plans();
     for (void** p : {&svals, (void**)&scols, (void**)&sell_counter}) {
       if (*p) cudaFree(*p);
@@ -468,6 +472,7 @@ int build_sell(const tbsla_matrix* m, DeviceMatrix* d, int n, int nc, int f_col,
   d->bytes += len * (prec_size(d->prec) + 4);
   TRY(cudaMemsetAsync(d->sell_counter, 0, kSellCounterWords * sizeof(unsigned), d->stream));
   TRY(sell_fill(sell_args(m, d), d->stream));
+  d->sell_ready = true;
   return TBSLA_OK;
 }
 
@@ -1196,15 +1201,32 @@ void initial_coefficients(const DeviceMatrix* d, double beta, double c[2]) {
 }
 }  // namespace
 
+// The sliced-ELL layout of a matrix on the row-block kernel, beside its CSR
+// copy.  A layout that was not finished is taken down whatever stopped it (an
+// error, an exception from a host allocation), so that no later call meets a
+// part of one; without room for it, on the device or the host, the row-block
+// kernel runs, and the layout is not tried again.
 static int pagerank_layout(const tbsla_matrix* m, DeviceMatrix* d) {
   const tbsla_info& I = m->info;
-  if (!d->sell.empty() || I.ln_col > 8388608) return TBSLA_OK;
-  int st = build_sell(m, d, I.ln_row, I.ln_col, I.f_col, m->idx0.data(), m->idx1.data());
-  if (st == TBSLA_ERR_ALLOC) {  // no room: the row-block kernel
-    d->free_sell();
-    st = TBSLA_OK;
+  if (d->sell_ready || d->no_pr_layout || I.ln_col > 8388608) return TBSLA_OK;
+  struct Undo {
+    DeviceMatrix* d;
+    size_t bytes;
+    ~Undo() {
+      if (d->sell_ready) return;
+      d->free_sell();
+      d->bytes = bytes;
+    }
+  } undo{d, d->bytes};
+  int st;
+  try {
+    st = build_sell(m, d, I.ln_row, I.ln_col, I.f_col, m->idx0.data(), m->idx1.data());
+  } catch (const std::bad_alloc&) {
+    st = TBSLA_ERR_ALLOC;
   }
-  return st;
+  if (st != TBSLA_ERR_ALLOC) return st;
+  d->no_pr_layout = true;
+  return TBSLA_OK;
 }
 
 int dev_page_rank(tbsla_matrix* m, double beta, double eps, int max_it, double* result,
@@ -1225,7 +1247,7 @@ int dev_page_rank(tbsla_matrix* m, double beta, double eps, int max_it, double* 
   // x mean 5000 x 8: 24 -> 20 us, 50,000 x 10: 31 -> 22; 60 with long rows in
   // the blocks)
   if (m->csr_algo < 0 && d->algo == 1 && m->pr_fused && I.nnz > 0 && (st = pagerank_layout(m, d))) return st;
-  const bool sell = !d->sell.empty();
+  const bool sell = d->sell_ready;
   int sms = 152;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, d->device);
   int grid = sell ? 8 * sms : (I.nnz > 0 ? csr_pagerank_grid(d->items, d->prec) : 1);
