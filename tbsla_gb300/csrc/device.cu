@@ -20,6 +20,7 @@
 #include <cmath>
 #include <cstdint>
 #include <cstring>
+#include <memory>
 #include <new>
 #include <vector>
 
@@ -314,6 +315,15 @@ int upload_array(DeviceMatrix* d, T** dst, const T* src, size_t n) {
   return status_of(cudaMemcpyAsync(*dst, src, n * sizeof(T), cudaMemcpyHostToDevice, d->stream));
 }
 
+// Waits for the copies queued on the matrix's stream, whatever the status so
+// far: on a host whose page tables the GPU reads, a copy may still be under way
+// when the call that queued it returns, and a local array that it reads must
+// outlive it on a failed path too.
+int settled(DeviceMatrix* d, int st) {
+  const int e = status_of(cudaStreamSynchronize(d->stream));
+  return st ? st : e;
+}
+
 SellArgs sell_args(const tbsla_matrix* m, const DeviceMatrix* d) {
   SellArgs a;
   a.vals = d->vals;
@@ -442,7 +452,7 @@ int build_sell(const tbsla_matrix* m, DeviceMatrix* d, int n, int nc, int f_col,
       if (!st) st = status_of(cudaMemsetAsync(dp.cut_done, 0, (size_t)hp.ncut * sizeof(unsigned), d->stream));
       d->bytes += (size_t)hp.npieces * 8 + (size_t)hp.ncut * 28;
     }
-    if (!st) st = status_of(cudaStreamSynchronize(d->stream));  // host plan arrays are freed next
+    st = settled(d, st);  // host plan arrays are freed next
     sell_plan_free(&hp);
     steps += dp.sell_len / 32;
   }
@@ -496,16 +506,16 @@ int build_coo_rows(const tbsla_matrix* m, DeviceMatrix* d, const std::vector<lon
   int st = upload_ints(d, &d->idx0, rp.data(), rp.size());
   if (!st) st = upload_ints(d, &d->idx1, cols.data(), cols.size());
   if (!st) st = upload_values(d, vals.data(), vals.size());
+  st = settled(d, st);
   if (st) return st;
   if (row_blocks_first(rp.data(), n)) {
     d->algo = TBSLA_CSR_ROWBLOCK;
     d->items = 4;
     int* blocks = nullptr;
     csr_partition(rp.data(), n, 256 * d->items, kCsrMaxSteps, &blocks, &d->nblocks);
-    st = upload_ints(d, &d->blocks, blocks, (size_t)d->nblocks + 1);
-    const cudaError_t e = cudaStreamSynchronize(d->stream);
+    st = settled(d, upload_ints(d, &d->blocks, blocks, (size_t)d->nblocks + 1));
     delete[] blocks;
-    return st ? st : status_of(e);
+    return st;
   }
   d->algo = TBSLA_CSR_SELL;
   const size_t copy = d->bytes;
@@ -548,7 +558,7 @@ int build(const tbsla_matrix* m, DeviceMatrix* d) {
       d->items = tile <= 1024 ? 4 : tile <= 2048 ? 8 : 16;
       int* blocks = nullptr;
       csr_partition(rp, I.ln_row, 256 * d->items, d->algo == TBSLA_CSR_ROWBLOCK ? kCsrMaxSteps : 0, &blocks, &d->nblocks);
-      st = upload_ints(d, &d->blocks, blocks, (size_t)d->nblocks + 1);
+      st = settled(d, upload_ints(d, &d->blocks, blocks, (size_t)d->nblocks + 1));
       delete[] blocks;
       if (st) return st;
       d->merge_items = m->merge_items;
@@ -617,8 +627,7 @@ int build(const tbsla_matrix* m, DeviceMatrix* d) {
       const long nch = coo_chunks(nnz);
       if (!st) st = dalloc(&d->coo_carry, (size_t)(2 * nch + (nch + 1) / 2));
       if (!st) d->bytes += (size_t)nch * 20;
-      if (!st) st = status_of(cudaStreamSynchronize(d->stream));
-      return st;
+      return settled(d, st);
     }
     case TBSLA_DENSE: {
       if (I.nnz == 0) return TBSLA_OK;
@@ -678,16 +687,13 @@ DeviceMatrix* ensure(const tbsla_matrix* m, int* st) {
   *st = check_device();
   if (*st) return nullptr;
   cudaSetDevice(g_device);
-  auto* d = new DeviceMatrix();
+  std::unique_ptr<DeviceMatrix> d(new DeviceMatrix());  // given back on every failure path
   d->device = g_device;
   d->prec = m->precision;
-  *st = build(m, d);
-  if (*st) {
-    delete d;
-    return nullptr;
-  }
-  m->dev = d;
-  return d;
+  *st = build(m, d.get());
+  if (*st) return nullptr;
+  m->dev = d.get();
+  return d.release();
 }
 
 CsrArgs csr_args(const tbsla_matrix* m, DeviceMatrix* d) {
@@ -1340,7 +1346,7 @@ int batch_plan(const tbsla_matrix* m, DeviceMatrix* d, int grid) {
   if (!st) st = dalloc(&b.piece_sum, 32 * cut.size());
   if (!st) st = dalloc(&b.cut_done, first.size());
   if (!st) st = status_of(cudaMemsetAsync(b.cut_done, 0, first.size() * sizeof(unsigned), d->stream));
-  if (!st) st = status_of(cudaStreamSynchronize(d->stream));
+  st = settled(d, st);
   if (st) {  // no plan: the next call builds it again
     if (b.item) cudaFree(b.item);
     b.item = nullptr;

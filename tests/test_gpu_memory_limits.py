@@ -162,6 +162,22 @@ def test_page_rank_layout(lib, kind, least):
     assert sum(b == bare and ok for ok, b, _ in runs) >= (4 if kind == 1 else 1)
 
 
+@pytest.mark.parametrize("count", [40_000, 700_000])
+def test_triplet_rows(lib, count):
+    """COO below and above 2^19 triplets: without room for the row layout the
+    triplets themselves are kept."""
+    out = run(lib, f"""
+    rp, ci, v, row = graph(9000, {count}, 20_000, 2)
+    x = np.random.default_rng(3).uniform(-1, 1, 9000)
+    ref = oracle.coo_ax(9000, row, ci, v, x)
+    scale = oracle.coo_ax(9000, row, ci, np.abs(v), np.abs(x))
+    make = lambda: T.MatrixCOO.from_arrays(9000, 9000, row, ci, v)
+    right = lambda y: bool(oracle.rel_err_normalized(y, ref, scale) <= 1e-13)
+    print(json.dumps(sweep(make, lambda m: m.spmv(x), right, 1, 1)))
+    """)
+    assert sum(ok and b != full for ok, b, full in out) >= 3
+
+
 def test_batched_plan_bytes(gpu):
     """The work items of the batched step follow the gathers in flight (another
     grid, another item size); their bytes are counted once."""
