@@ -189,8 +189,8 @@ int tbsla_matrix_device_bytes(const tbsla_matrix* m, size_t* bytes);
  * implementation's kernels). */
 int tbsla_matrix_kernel_launches(const tbsla_matrix* m, int* launches);
 /* CSR: block budget of the row-block partition (nnz per block, multiple of
- * 256, default 2048; under TBSLA_CSR_AUTO at most 1024, whose small matrices
- * gain by more blocks); changing it rebuilds the partition. */
+ * 256); until it is called 2048, or 1024 under TBSLA_CSR_AUTO, whose small
+ * matrices gain by more blocks.  Changing it rebuilds the partition. */
 int tbsla_matrix_set_csr_tile(tbsla_matrix* m, int nnz_per_block);
 /* CSR SpMV kernel: TBSLA_CSR_AUTO (default: row blocks below 2^19 stored
  * entries, and below 3 2^20 without rows of more than 64, where one short

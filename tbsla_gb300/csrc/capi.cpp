@@ -268,10 +268,9 @@ int tbsla_matrix_set_csr_tile(tbsla_matrix* m, int nnz_per_block) try {
   if (!m || nnz_per_block < 256 || nnz_per_block > 4096 || nnz_per_block % 256 != 0)
     return TBSLA_ERR_INVALID_ARG;
   int items = nnz_per_block <= 1024 ? 4 : nnz_per_block <= 2048 ? 8 : 16;
-  if (m->csr_tile != 256 * items) {
-    m->invalidate();
-    m->csr_tile = 256 * items;
-  }
+  const int now = dev_csr_tile(m);
+  if (now && now != 256 * items) m->invalidate();
+  m->csr_tile = 256 * items;
   return TBSLA_OK;
 } TBSLA_API_CATCH
 

@@ -354,6 +354,7 @@ SellArgs sell_args(const tbsla_matrix* m, const DeviceMatrix* d) {
 // against 107 us).
 constexpr long kSellMin = 1L << 19, kSellMinShort = 3L << 20;
 constexpr int kShortRow = 64;
+constexpr int kCsrTile = 2048;  // row-block budget where none is set
 bool row_blocks_first(const int* rp, int n) {
   const long nz = (long)rp[n] - rp[0];
   if (nz < kSellMin) return true;
@@ -551,9 +552,9 @@ int build(const tbsla_matrix* m, DeviceMatrix* d) {
       if (st) return st;
       const long enz = end - rp[0];  // merge-path tiles and their carry scratch
       d->algo = m->csr_algo >= 0 ? m->csr_algo : row_blocks_first(rp, I.ln_row) ? TBSLA_CSR_ROWBLOCK : TBSLA_CSR_SELL;
-      // automatic: row blocks of half the default size, which give twice the
-      // CTAs (480,000 entries: 10.5 -> 8.4 us, 18,000: 6.3 -> 5.2)
-      const int budget = m->csr_algo < 0 && d->algo == TBSLA_CSR_ROWBLOCK ? std::min(1024, m->csr_tile) : m->csr_tile;
+      // no size set, automatic kernel: half the other kernels' default, which
+      // gives twice the CTAs (480,000 entries: 10.5 -> 8.4 us, 18,000: 6.3 -> 5.2)
+      const int budget = m->csr_tile ? m->csr_tile : m->csr_algo < 0 && d->algo == TBSLA_CSR_ROWBLOCK ? 1024 : kCsrTile;
       int tile = std::max(256, std::min(4096, budget));
       d->items = tile <= 1024 ? 4 : tile <= 2048 ? 8 : 16;
       int* blocks = nullptr;
@@ -782,6 +783,8 @@ static int sell_launches(const DeviceMatrix* d) {
   for (const SellPlan& p : d->sell) k += p.nslices > 0;
   return k;
 }
+
+int dev_csr_tile(const tbsla_matrix* m) { return m->dev && m->format == TBSLA_CSR ? 256 * m->dev->items : 0; }
 
 int dev_launches(const tbsla_matrix* m, int* launches) {
   int st;
@@ -1478,9 +1481,10 @@ int dev_autotune(tbsla_matrix* m, int reps, tbsla_tuning* best, tbsla_tuning* tr
   const int thr[4][2] = {{64, 64}, {128, 128}, {32, 32}, {64, 255}};
   for (int cb : blocks)
     for (auto& t : thr)
-      for (int u : {8, 16}) cand.push_back({TBSLA_CSR_SELL, u, t[0], t[1], 16384, cb, m->csr_tile, 0.0});
+      for (int u : {8, 16}) cand.push_back({TBSLA_CSR_SELL, u, t[0], t[1], 16384, cb, m->csr_tile ? m->csr_tile : kCsrTile, 0.0});
   const tbsla_tuning keep{m->csr_algo, m->csr_algo == TBSLA_CSR_MERGE ? m->merge_items : m->sell_unroll,
-                          m->sell_short, m->sell_long, m->sell_sigma, m->sell_colblock, m->csr_tile, 0.0};
+                          m->sell_short, m->sell_long, m->sell_sigma, m->sell_colblock,
+                          m->csr_tile ? m->csr_tile : kCsrTile, 0.0};
   cand.push_back({TBSLA_CSR_MERGE, 8, keep.short_thr, keep.long_thr, keep.sigma, keep.col_block, keep.tile, 0});
   cand.push_back({TBSLA_CSR_ROWBLOCK, 0, keep.short_thr, keep.long_thr, keep.sigma, keep.col_block, 2048, 0});
   double *x = nullptr, *y = nullptr;
