@@ -365,6 +365,9 @@ bool row_blocks_first(const int* rp, int n) {
 }
 
 
+// Columns per block of the sliced-ELL layout.
+long sell_colblock(const tbsla_matrix* m) { return m->sell_colblock > 0 ? m->sell_colblock : 8388608L; }
+
 // Sliced-ELL device layout of a matrix in CSR (n rows, nc columns from f_col
 // on; host arrays rp, ci, device copies idx0, idx1, vals): the columns are
 // split into blocks of at most `sell_colblock` columns (0: 8,388,608, 64 MiB
@@ -374,7 +377,7 @@ bool row_blocks_first(const int* rp, int n) {
 int build_sell(const tbsla_matrix* m, DeviceMatrix* d, int n, int nc, int f_col, const int* rp, const int* ci) {
   using tbsla_impl::parallel_for;
   nc = std::max(nc, 1);
-  const long cb = m->sell_colblock > 0 ? m->sell_colblock : 8388608L;
+  const long cb = sell_colblock(m);
   const int P = (int)std::max<long>(1, (nc + cb - 1) / cb);
   const int W = (int)(((long)nc + P - 1) / P);
   std::vector<int> lens((size_t)P * n, 0);
@@ -1214,10 +1217,12 @@ void initial_coefficients(const DeviceMatrix* d, double beta, double c[2]) {
 // copy.  A layout that was not finished is taken down whatever stopped it (an
 // error, an exception from a host allocation), so that no later call meets a
 // part of one; without room for it, on the device or the host, the row-block
-// kernel runs, and the layout is not tried again.
+// kernel runs, and the layout is not tried again.  Only as one column block,
+// which a step runs in one launch (columns set to blocks of 100 would take 30
+// launches a step of 3000 nodes).
 static int pagerank_layout(const tbsla_matrix* m, DeviceMatrix* d) {
   const tbsla_info& I = m->info;
-  if (d->sell_ready || d->no_pr_layout || I.ln_col > 8388608) return TBSLA_OK;
+  if (d->sell_ready || d->no_pr_layout || I.ln_col > sell_colblock(m)) return TBSLA_OK;
   struct Undo {
     DeviceMatrix* d;
     size_t bytes;

@@ -37,3 +37,23 @@ def test_tile_under_the_automatic_kernel(gpu):
     for tile in (1024, 2048, 4096):
         assert size[m.AUTO, tile] == size[m.ROWBLOCK, tile]
     assert size[m.AUTO, None] == size[m.AUTO, 1024] > size[m.AUTO, 2048] > size[m.AUTO, 4096]
+
+
+@pytest.mark.parametrize("col_block,makes", [(0, True), (3000, True), (2999, False), (100, False)])
+def test_page_rank_layout_is_one_column_block(gpu, col_block, makes):
+    """PageRank on a small matrix makes its sliced-ELL layout only where that
+    is one launch a step, not one per column block."""
+    T = gpu
+    n = 3000
+    rng = np.random.default_rng(2)
+    rp = np.concatenate(([0], np.cumsum(rng.integers(0, 16, n)))).astype(np.int32)
+    ci = rng.integers(0, n, rp[-1]).astype(np.int32)
+    v = 1.0 / np.bincount(ci, minlength=n)[ci]
+    m = T.MatrixCSR.from_arrays(n, n, rp, ci, v)
+    m.set_sell_params(0, 0, 16384, col_block)
+    m.upload()
+    before = m.device_bytes()
+    x, it, _, ok = m.page_rank(0.85, 1e-10, 500)
+    ref = oracle.pagerank(rp, ci, v, 0.85, 1e-10, it, stop_early=False)[0]
+    assert ok and np.abs(x - ref).sum() <= 1e-10
+    assert (m.device_bytes() > before) == makes
