@@ -500,6 +500,13 @@ int build_sell(const tbsla_matrix* m, DeviceMatrix* d, int n, int nc, int f_col,
 // Bound: the gathers of x, as for CSR.  FP64, 2^22 rows x 10: 251 -> 183 us (with
 // triplet chunks: 142 us of gathers, key compares and the carry pass on top);
 // 10,000 x 14: 14.5 -> 6.2; power-law rows, 10^6 x 14: 87 -> 69.
+// A row longer than kCooRowBlockMost triplets goes to sliced ELL at every size,
+// which spreads it over warps as the triplet chunks did: a row block is one CTA
+// (FP64, longest row 3000 / 10,000 / 30,000 / 100,000 / 400,000: of 400,000
+// triplets row blocks 7.7 / 11.0 / 18.8 / 50 / 187 us, sliced ELL 11.5 / 11.1 /
+// 10.6 / 11.9 / 16.1, chunks 12.4 / 14.4 / 20.5 / 36 / 139; of 100,000 row blocks
+// 5.4 / 8.8 / 17.8 / 50, sliced ELL 9.4 / 9.8 / 11.1 / 9.6).
+constexpr int kCooRowBlockMost = 10 << 10;
 int build_coo_rows(const tbsla_matrix* m, DeviceMatrix* d, const std::vector<long>& ends,
                    const std::vector<int>& cols, const std::vector<double>& vals) {
   const tbsla_info& I = m->info;
@@ -512,7 +519,9 @@ int build_coo_rows(const tbsla_matrix* m, DeviceMatrix* d, const std::vector<lon
   if (!st) st = upload_values(d, vals.data(), vals.size());
   st = settled(d, st);
   if (st) return st;
-  if (row_blocks_first(rp.data(), n)) {
+  int longest = 0;
+  for (int i = 0; i < n; i++) longest = std::max(longest, rp[i + 1] - rp[i]);
+  if (row_blocks_first(rp.data(), n) && longest <= kCooRowBlockMost) {
     d->algo = TBSLA_CSR_ROWBLOCK;
     d->items = 4;
     int* blocks = nullptr;

@@ -57,3 +57,33 @@ def test_page_rank_layout_is_one_column_block(gpu, col_block, makes):
     ref = oracle.pagerank(rp, ci, v, 0.85, 1e-10, it, stop_early=False)[0]
     assert ok and np.abs(x - ref).sum() <= 1e-10
     assert (m.device_bytes() > before) == makes
+
+
+@pytest.mark.parametrize("prec", ["f64", "f32"])
+@pytest.mark.parametrize("fmt", ["coo", "scoo"])
+@pytest.mark.parametrize("longest", [10_239, 10_240, 10_241, 60_000])
+def test_triplets_with_a_long_row(gpu, longest, fmt, prec):
+    """A row of more than 10 2^10 triplets takes a small matrix from the row
+    blocks (values, columns, row starts and blocks) to sliced ELL (slices, and
+    4.5 bytes a row of descriptors instead of 4 of row starts)."""
+    T = gpu
+    n, rest = 20_000, 40_000
+    rng = np.random.default_rng(longest)
+    row = rng.integers(0, n, rest)
+    row[row == n // 3] = n // 3 + 1
+    row = np.concatenate((row, np.full(longest, n // 3), [0, n - 1])).astype(np.int32)
+    col = rng.integers(0, n, len(row)).astype(np.int32)
+    v = rng.uniform(-1, 1, len(row))
+    m = T.MatrixCOO.from_arrays(n, n, row, col, v)
+    if fmt == "scoo":
+        m = T.MatrixSCOO(m)
+    m.set_precision({"f64": T.F64, "f32": T.F32}[prec])
+    w = v if prec == "f64" else v.astype(np.float32).astype(np.float64)
+    x, r0 = rng.uniform(-1, 1, n), rng.uniform(-1, 1, n)
+    r = r0.copy()
+    m.Ax(r, x)
+    scale = oracle.coo_ax(n, row, col, np.abs(w), np.abs(x), np.abs(r0))
+    assert oracle.rel_err_normalized(r, oracle.coo_ax(n, row, col, w, x, r0.copy()), scale) <= TOL
+    assert oracle.rel_err_normalized(m.spmv(x), oracle.coo_ax(n, row, col, w, x), scale) <= TOL
+    entry = 12 if prec == "f64" else 8
+    assert (m.device_bytes() > entry * len(row) + 4.3 * n) == (longest > 10_240)
