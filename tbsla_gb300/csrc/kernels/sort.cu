@@ -205,11 +205,19 @@ __global__ void k_column_keys(const int* __restrict__ colidx, long n, int f_col,
   }
 }
 
-// start[c]: the first of the sorted keys that is c or more (c <= n_col).
+// start[c]: the first of the sorted keys that is c or more (c <= n_col).  A
+// binary search per column: a thread per key that fills the columns up to it
+// leaves a run of empty columns to one thread (2^22 columns, the first 1000
+// used: 24.5 -> 10.5 ms of a first solve).
 __global__ void k_column_starts(const unsigned* __restrict__ keys, long n, int n_col, int* __restrict__ start) {
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i <= n; i += (long)gridDim.x * blockDim.x) {
-    const long from = i > 0 ? (long)keys[i - 1] + 1 : 0, to = i < n ? (long)keys[i] : n_col;
-    for (long c = from; c <= to; c++) start[c] = (int)i;
+  for (long c = blockIdx.x * (long)blockDim.x + threadIdx.x; c <= n_col; c += (long)gridDim.x * blockDim.x) {
+    long lo = 0, hi = n;
+    while (lo < hi) {
+      const long mid = (lo + hi) >> 1;
+      if ((long)keys[mid] < c) lo = mid + 1;
+      else hi = mid;
+    }
+    start[c] = (int)lo;
   }
 }
 
@@ -281,7 +289,7 @@ cudaError_t column_sums_ordered(const void* vals, int prec, const int* colidx, l
     e = sort_pairs(keys, alt, perm, perm_alt, n, bits, reinterpret_cast<unsigned*>(start + n_col + 1), &in_alt, s);
   if (e != cudaSuccess) return e;
   const int* p = in_alt ? perm_alt : perm;
-  k_column_starts<<<grid_for(n + 1), RT, 0, s>>>(in_alt ? alt : keys, n, n_col, start);
+  k_column_starts<<<grid_for((long)n_col + 1), RT, 0, s>>>(in_alt ? alt : keys, n, n_col, start);
   const int grid = grid_for(n_col);
   switch (prec) {
     case kF64:

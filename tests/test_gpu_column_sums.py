@@ -39,3 +39,22 @@ def test_weights(gpu, prec, n, extra):
     again = T.MatrixCSR.from_arrays(n, n, rp, col, v)
     again.set_precision({"f64": T.F64, "f32": T.F32, "bf16": T.BF16}[prec])
     assert np.array_equal(again.page_rank(beta=0.85, epsilon=1e-13, max_iterations=60)[0], x)
+
+
+@pytest.mark.parametrize("used", ["first", "last", "ends", "one"])
+def test_empty_columns(gpu, used):
+    """Runs of empty columns before, between and after the others (a column
+    per thread looks for its first entry)."""
+    T = gpu
+    n, count = 70_001, 150_000
+    rng = np.random.default_rng(len(used))
+    cols = {"first": np.arange(40), "last": np.arange(n - 40, n), "ends": np.r_[:20, n - 20:n], "one": [n // 2]}[used]
+    col = rng.choice(cols, count).astype(np.int32)
+    row = np.sort(rng.integers(0, n, count))
+    rp = np.concatenate(([0], np.cumsum(np.bincount(row, minlength=n)))).astype(np.int32)
+    v = rng.uniform(0.5, 1.0, count)
+    v /= np.bincount(col, v, minlength=n)[col]
+    m = T.MatrixCSR.from_arrays(n, n, rp, col, v)
+    x, *_ = m.page_rank(beta=0.85, epsilon=1e-13, max_iterations=60)
+    ref = oracle.pagerank(rp, col, v, beta=0.85, epsilon=1e-13, max_iterations=60)
+    assert np.abs(x - ref[0]).sum() <= 1e-12
