@@ -1173,13 +1173,38 @@ bool column_weights_device(const tbsla_matrix* m, DeviceMatrix* d, std::vector<d
   if (n < kColumnSumsMin || n >= INT_MAX) return false;
   unsigned* scratch = nullptr;
   if (dalloc(&scratch, (size_t)column_sums_scratch(n, I.ln_col)) != TBSLA_OK) return false;
+  struct Free {
+    unsigned* p;
+    ~Free() { cudaFree(p); }
+  } give_back{scratch};
   const size_t skip = (size_t)m->idx0[0];
+  std::vector<ColumnRange> hubs;
+  const int* sorted = nullptr;
   *st = status_of(column_sums_ordered(static_cast<const char*>(d->vals) + skip * prec_size(d->prec), d->prec,
-                                      d->idx1 + skip, n, I.f_col, I.ln_col, scratch, d->colw, d->stream));
+                                      d->idx1 + skip, n, I.f_col, I.ln_col, scratch, d->colw, &sorted, &hubs,
+                                      d->stream));
+  size_t most = 0;
+  for (const ColumnRange& h : hubs) most = std::max(most, (size_t)h.len);
+  std::vector<int> at(most);
+  std::vector<double> sum(hubs.size());
+  // the host's columns, under the device's
+  cudaStream_t side = nullptr;
+  if (!*st && !hubs.empty()) *st = status_of(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
+  for (size_t k = 0; k < hubs.size() && !*st; k++) {
+    const ColumnRange& h = hubs[k];
+    *st = status_of(cudaMemcpyAsync(at.data(), sorted + h.first, (size_t)h.len * 4, cudaMemcpyDeviceToHost, side));
+    const int e = status_of(cudaStreamSynchronize(side));
+    if (!*st) *st = e;
+    if (*st) break;
+    const double* v = m->values.data() + skip;
+    double s = 0.0;
+    for (int t = 0; t < h.len; t++) s += stored_value(v[at[t]], d->prec);
+    sum[k] = s;
+    *st = status_of(cudaMemcpyAsync(d->colw + h.col, &sum[k], 8, cudaMemcpyHostToDevice, d->stream));
+  }
+  if (side) cudaStreamDestroy(side);
   if (!*st) *st = status_of(cudaMemcpyAsync(w.data(), d->colw, w.size() * 8, cudaMemcpyDeviceToHost, d->stream));
-  const cudaError_t e = cudaStreamSynchronize(d->stream);
-  if (!*st) *st = status_of(e);
-  cudaFree(scratch);
+  *st = settled(d, *st);
   return true;
 }
 

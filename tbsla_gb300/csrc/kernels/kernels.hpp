@@ -410,10 +410,16 @@ long radix_scratch(long n);
 cudaError_t radix_sort_pairs(uint64_t* keys, uint64_t* keys_alt, int* vals, int* vals_alt, long n, int bits,
                              unsigned* scratch, int* result_in_alt, cudaStream_t s);
 // w[c] = the sum of column c's values (c relative to f_col), added in entry
-// order; scratch: column_sums_scratch(n, n_col) words.
+// order; scratch: column_sums_scratch(n, n_col) words.  Synchronises on s.  A few
+// very long columns may be left to the host, which adds them sooner: hubs, whose
+// entries are sorted[first .. first + len) (device, in the scratch) in order.
+struct ColumnRange {
+  int col, first, len;
+};
 long column_sums_scratch(long n, int n_col);
 cudaError_t column_sums_ordered(const void* vals, int prec, const int* colidx, long n, int f_col, int n_col,
-                                unsigned* scratch, double* w, cudaStream_t s);
+                                unsigned* scratch, double* w, const int** sorted, std::vector<ColumnRange>* hubs,
+                                cudaStream_t s);
 // Exclusive scan in place; scratch: scan_scratch(n) words.
 long scan_scratch(long n);
 cudaError_t exclusive_scan(unsigned* a, long n, unsigned* scratch, cudaStream_t s);

@@ -16,6 +16,7 @@
 // per-warp counts in shared memory give every key its place after the
 // earlier warps and rounds of its tile.
 #include <algorithm>
+#include <vector>
 
 #include "common.cuh"
 #include "kernels.hpp"
@@ -222,20 +223,23 @@ __global__ void k_column_starts(const unsigned* __restrict__ keys, long n, int n
 }
 
 // w[c] = sum of column c's values, added one by one in entry order from 0 (the
-// order of a loop over the entries, so the same bits).  A lane per column; a
-// column of more than kLaneColumn entries by its whole warp: 32 values loaded
-// at once, added in order by shuffles.
+// order of a loop over the entries, so the same bits).  A lane per column here;
+// columns of more than kLaneColumn entries go to list (lens[0]: how many,
+// lens[1]: the longest's entries), 0 for now.
 constexpr int kLaneColumn = 64;
 template <class V>
-__global__ void __launch_bounds__(RT) k_column_sums_ordered(const V* __restrict__ vals, const int* __restrict__ perm,
-                                                           const int* __restrict__ start, int n_col,
-                                                           double* __restrict__ w) {
+__global__ void __launch_bounds__(RT) k_column_sums_short(const V* __restrict__ vals, const int* __restrict__ perm,
+                                                         const int* __restrict__ start, int n_col,
+                                                         double* __restrict__ w, int* __restrict__ list,
+                                                         int* __restrict__ lens) {
   const int lane = threadIdx.x & 31;
+  int most = 0;
   for (long c0 = (blockIdx.x * (long)RT + threadIdx.x) / kWarp * kWarp; c0 < n_col; c0 += (long)gridDim.x * RT) {
     const long c = c0 + lane;
     const int a = c < n_col ? start[c] : 0, e = c < n_col ? start[c + 1] : 0;
+    const bool is_long = e - a > kLaneColumn;
     double sum = 0.0;
-    if (e - a <= kLaneColumn) {
+    if (!is_long) {
       int t = a;
       for (; t + 4 <= e; t += 4) {
         double v[4];
@@ -245,27 +249,111 @@ __global__ void __launch_bounds__(RT) k_column_sums_ordered(const V* __restrict_
         for (int u = 0; u < 4; u++) sum = add_rn(sum, v[u]);
       }
       for (; t < e; t++) sum = add_rn(sum, widen(vals[perm[t]]));
-    }
-    for (unsigned left = __ballot_sync(FULL, e - a > kLaneColumn); left; left &= left - 1) {
-      const int src = __ffs(left) - 1;
-      const int la = __shfl_sync(FULL, a, src), le = __shfl_sync(FULL, e, src);
-      double s = 0.0, v = la + lane < le ? widen(vals[perm[la + lane]]) : 0.0;
-      for (int t = la; t < le; t += kWarp) {
-        const int next = t + kWarp + lane;
-        const double vn = next < le ? widen(vals[perm[next]]) : 0.0;
-        const int m = min(kWarp, le - t);
-        if (m == kWarp) {
-#pragma unroll
-          for (int u = 0; u < kWarp; u++) s = add_rn(s, __shfl_sync(FULL, v, u));
-        } else {
-          for (int u = 0; u < m; u++) s = add_rn(s, __shfl_sync(FULL, v, u));
-        }
-        v = vn;
-      }
-      if (lane == src) sum = s;
+    } else {
+      list[atomicAdd(lens, 1)] = (int)c;
+      most = max(most, e - a);
     }
     if (c < n_col) w[c] = sum;
   }
+  most = __reduce_max_sync(FULL, most);
+  if (lane == 0 && most > 0) atomicMax(lens + 1, most);
+}
+
+// The listed columns of at most `most` entries, a warp each (columns of a list,
+// not of the matrix: neighbours in the numbering may all be long): 32 values
+// loaded at once, added in order by shuffles.
+template <class V>
+__global__ void __launch_bounds__(RT) k_column_sums_long(const V* __restrict__ vals, const int* __restrict__ perm,
+                                                        const int* __restrict__ start, const int* __restrict__ list,
+                                                        int count, int most, double* __restrict__ w) {
+  const int lane = threadIdx.x & 31;
+  for (int k = (blockIdx.x * RT + threadIdx.x) / kWarp; k < count; k += gridDim.x * (RT / kWarp)) {
+    const int c = list[k], la = start[c], le = start[c + 1];
+    if (le - la > most) continue;
+    double s = 0.0, v = la + lane < le ? widen(vals[perm[la + lane]]) : 0.0;
+    for (int t = la; t < le; t += kWarp) {
+      const int next = t + kWarp + lane;
+      const double vn = next < le ? widen(vals[perm[next]]) : 0.0;
+      const int m = min(kWarp, le - t);
+      if (m == kWarp) {
+#pragma unroll
+        for (int u = 0; u < kWarp; u++) s = add_rn(s, __shfl_sync(FULL, v, u));
+      } else {
+        for (int u = 0; u < m; u++) s = add_rn(s, __shfl_sync(FULL, v, u));
+      }
+      v = vn;
+    }
+    if (lane == 0) w[c] = s;
+  }
+}
+
+// The listed columns of more than `over` entries: found[0] of them, then
+// (column, first sorted entry, entries) each, the first kMostHubs of them.
+constexpr int kMostHubs = 256;
+__global__ void k_long_columns(const int* __restrict__ start, const int* __restrict__ list, int count, int over,
+                               int* __restrict__ found) {
+  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < count; k += gridDim.x * blockDim.x) {
+    const int c = list[k], a = start[c], len = start[c + 1] - a;
+    if (len <= over) continue;
+    const int at = atomicAdd(found, 1);
+    if (at >= kMostHubs) continue;
+    found[1 + 3 * at] = c;
+    found[2 + 3 * at] = a;
+    found[3 + 3 * at] = len;
+  }
+}
+
+// Columns that the caller adds up on the host, longest first.  On the device a
+// column is a chain of dependent FP64 additions, 46 ns an entry, on the host 1
+// to 3; the device's columns run side by side, the host's one after another.  So
+// the longest ones go to the host as long as all that it takes so far costs it
+// less than the shortest of them costs the device (2^20 nodes, 200,000 entries
+// and one column of 10^6: first solve 47.7 -> 2.2 ms more than the next; 32
+// neighbouring columns of 100,000, on one warp before the list: 152 -> 9.0).  More than kMostHubs columns within the
+// ratio of the longest are work enough for the device's many warps.
+constexpr int kHubMin = 4096, kHubRatio = 12;
+cudaError_t choose_hubs(const int* start, const int* list, int count, int longest, int* found,
+                        std::vector<ColumnRange>* hubs, cudaStream_t s) {
+  hubs->clear();
+  if (longest <= kHubMin) return cudaSuccess;
+  std::vector<int> h(1 + 3 * kMostHubs);
+  cudaError_t e = cudaMemsetAsync(found, 0, sizeof(int), s);
+  if (e != cudaSuccess) return e;
+  k_long_columns<<<grid_for(count), RT, 0, s>>>(start, list, count, std::max(kHubMin, longest / kHubRatio), found);
+  e = cudaGetLastError();
+  if (e == cudaSuccess) e = cudaMemcpyAsync(h.data(), found, h.size() * sizeof(int), cudaMemcpyDeviceToHost, s);
+  const cudaError_t w = cudaStreamSynchronize(s);
+  if (e == cudaSuccess) e = w;
+  if (e != cudaSuccess || h[0] > kMostHubs) return e;
+  for (int k = 0; k < h[0]; k++) hubs->push_back({h[1 + 3 * k], h[2 + 3 * k], h[3 + 3 * k]});
+  std::sort(hubs->begin(), hubs->end(), [](const ColumnRange& a, const ColumnRange& b) {
+    return a.len != b.len ? a.len > b.len : a.col < b.col;
+  });
+  long taken = 0;
+  size_t k = 0;
+  while (k < hubs->size() && taken + (*hubs)[k].len < (long)kHubRatio * (*hubs)[k].len) taken += (*hubs)[k++].len;
+  while (k > 0 && k < hubs->size() && (*hubs)[k].len == (*hubs)[k - 1].len) k--;  // the device skips by length
+  hubs->resize(k);
+  return cudaSuccess;
+}
+
+template <class V>
+cudaError_t column_sums(const V* vals, const int* perm, const int* start, int n_col, int* list, int* found, double* w,
+                        std::vector<ColumnRange>* hubs, cudaStream_t s) {
+  cudaError_t e = cudaMemsetAsync(found, 0, 2 * sizeof(int), s);
+  if (e != cudaSuccess) return e;
+  k_column_sums_short<<<grid_for(n_col), RT, 0, s>>>(vals, perm, start, n_col, w, list, found);
+  e = cudaGetLastError();
+  int lens[2] = {0, 0};
+  if (e == cudaSuccess) e = cudaMemcpyAsync(lens, found, sizeof lens, cudaMemcpyDeviceToHost, s);
+  const cudaError_t done = cudaStreamSynchronize(s);
+  if (e == cudaSuccess) e = done;
+  if (e != cudaSuccess || lens[0] == 0) return e;
+  e = choose_hubs(start, list, lens[0], lens[1], found, hubs, s);
+  if (e != cudaSuccess) return e;
+  const int most = hubs->empty() ? lens[1] : hubs->back().len - 1;
+  k_column_sums_long<<<grid_for((long)lens[0] * kWarp), RT, 0, s>>>(vals, perm, start, list, lens[0], most, w);
+  return cudaGetLastError();
 }
 }  // namespace
 
@@ -274,36 +362,35 @@ cudaError_t radix_sort_pairs(uint64_t* keys, uint64_t* keys_alt, int* vals, int*
   return sort_pairs(keys, keys_alt, vals, vals_alt, n, bits, scratch, result_in_alt, s);
 }
 
-long column_sums_scratch(long n, int n_col) { return 4 * n + n_col + 1 + radix_scratch(n); }
+long column_sums_scratch(long n, int n_col) {
+  return 4 * n + n_col + 1 + radix_scratch(n) + n / kLaneColumn + 1 + 1 + 3 * kMostHubs;
+}
 
 cudaError_t column_sums_ordered(const void* vals, int prec, const int* colidx, long n, int f_col, int n_col,
-                                unsigned* scratch, double* w, cudaStream_t s) {
+                                unsigned* scratch, double* w, const int** sorted, std::vector<ColumnRange>* hubs,
+                                cudaStream_t s) {
+  hubs->clear();
   if (n_col <= 0) return cudaSuccess;
   unsigned *keys = scratch, *alt = keys + n;
   int *perm = reinterpret_cast<int*>(alt + n), *perm_alt = perm + n, *start = perm_alt + n;
+  unsigned* radix = reinterpret_cast<unsigned*>(start + n_col + 1);
+  int* list = reinterpret_cast<int*>(radix + radix_scratch(n));
+  int* found = list + n / kLaneColumn + 1;
   int bits = 0, in_alt = 0;
   while (bits < 31 && (1L << bits) < (long)n_col) bits++;
   if (n > 0) k_column_keys<<<grid_for(n), RT, 0, s>>>(colidx, n, f_col, keys, perm);
   cudaError_t e = cudaGetLastError();
-  if (e == cudaSuccess)
-    e = sort_pairs(keys, alt, perm, perm_alt, n, bits, reinterpret_cast<unsigned*>(start + n_col + 1), &in_alt, s);
+  if (e == cudaSuccess) e = sort_pairs(keys, alt, perm, perm_alt, n, bits, radix, &in_alt, s);
   if (e != cudaSuccess) return e;
   const int* p = in_alt ? perm_alt : perm;
+  *sorted = p;
   k_column_starts<<<grid_for((long)n_col + 1), RT, 0, s>>>(in_alt ? alt : keys, n, n_col, start);
-  const int grid = grid_for(n_col);
   switch (prec) {
-    case kF64:
-      k_column_sums_ordered<<<grid, RT, 0, s>>>(static_cast<const double*>(vals), p, start, n_col, w);
-      break;
-    case kF32:
-      k_column_sums_ordered<<<grid, RT, 0, s>>>(static_cast<const float*>(vals), p, start, n_col, w);
-      break;
-    case kBF16:
-      k_column_sums_ordered<<<grid, RT, 0, s>>>(static_cast<const __nv_bfloat16*>(vals), p, start, n_col, w);
-      break;
-    default: return cudaErrorInvalidValue;
+    case kF64: return column_sums(static_cast<const double*>(vals), p, start, n_col, list, found, w, hubs, s);
+    case kF32: return column_sums(static_cast<const float*>(vals), p, start, n_col, list, found, w, hubs, s);
+    case kBF16: return column_sums(static_cast<const __nv_bfloat16*>(vals), p, start, n_col, list, found, w, hubs, s);
   }
-  return cudaGetLastError();
+  return cudaErrorInvalidValue;
 }
 
 // COO -> DENSE (MatrixDENSE.cpp:15-37): the entries in (row, column) order,

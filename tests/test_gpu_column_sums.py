@@ -58,3 +58,27 @@ def test_empty_columns(gpu, used):
     x, *_ = m.page_rank(beta=0.85, epsilon=1e-13, max_iterations=60)
     ref = oracle.pagerank(rp, col, v, beta=0.85, epsilon=1e-13, max_iterations=60)
     assert np.abs(x - ref[0]).sum() <= 1e-12
+
+
+@pytest.mark.parametrize("prec", ["f64", "f32", "bf16"])
+@pytest.mark.parametrize("lengths", [[4096], [4097], [200_000], [60_000, 40_000, 40_000, 5000, 4096],
+                                     [9000] * 14, [30_000] * 3 + [4097] * 300])
+def test_hub_columns(gpu, lengths, prec):
+    """Columns next to each other long enough for the host to add some of them
+    (4097 entries and more, up to eleven equal ones) or, being many, none."""
+    T = gpu
+    n, extra = 9000, 150_000
+    rng = np.random.default_rng(len(lengths) + lengths[0])
+    col = np.concatenate([rng.integers(2000, n, extra)] + [np.full(k, 700 + i) for i, k in enumerate(lengths)])
+    row = rng.integers(0, n, len(col))
+    order = np.argsort(row, kind="stable")
+    col, row = col[order].astype(np.int32), row[order]
+    rp = np.concatenate(([0], np.cumsum(np.bincount(row, minlength=n)))).astype(np.int32)
+    v = rng.uniform(0.5, 1.0, len(col)) * 2.0 ** -rng.integers(0, 12, len(col))
+    v /= np.bincount(col, v, minlength=n)[col] * rng.uniform(1.0, 2.0, n)[col]
+    m = T.MatrixCSR.from_arrays(n, n, rp, col, v)
+    m.set_precision({"f64": T.F64, "f32": T.F32, "bf16": T.BF16}[prec])
+    w = v if prec == "f64" else v.astype(np.float32).astype(np.float64) if prec == "f32" else oracle.bf16_round(v)
+    x, *_ = m.page_rank(beta=0.85, epsilon=1e-13, max_iterations=60)
+    ref = oracle.pagerank(rp, col, w, beta=0.85, epsilon=1e-13, max_iterations=60)
+    assert np.abs(x - ref[0]).sum() <= 1e-12
