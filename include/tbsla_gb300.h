@@ -248,11 +248,14 @@ typedef struct {
   int tile;       /* ROWBLOCK entries per block */
   double ms;      /* mean device time of one Ax, CUDA events, L2 warm */
 } tbsla_tuning;
-/* Autotuner (CSR): times every candidate configuration -- the sliced-ELL
+/* Autotuner (CSR): times every candidate configuration -- the automatic one
+ * first (named by the kernel it takes, with thresholds 0), the sliced-ELL
  * kernel over its layout thresholds, column blocks and steps in flight, the
- * merge-path kernel and the row-block kernel -- on this matrix (`reps` Ax
- * each after one warm-up, x = 1), leaves the handle set to the fastest and
- * writes it to *best.  trials (optional): the first max_trials timings in
+ * merge-path kernel and the row-block kernel -- on this matrix (`reps` Ax or
+ * more each after one warm-up, x = 1), leaves the handle set to the fastest and
+ * writes it to *best.  Where the automatic one is the fastest the handle stays
+ * TBSLA_CSR_AUTO; where another one is, PageRank still takes the layout that it
+ * has under TBSLA_CSR_AUTO.  trials (optional): the first max_trials timings in
  * candidate order, their count in *ntrials.  The device copy is rebuilt for
  * every layout tried. */
 int tbsla_matrix_autotune(tbsla_matrix* m, int reps, tbsla_tuning* best, tbsla_tuning* trials, int max_trials,

@@ -107,6 +107,10 @@ def csr_key(m, precision: int) -> str:
 
 
 def apply_csr(m, cfg: dict) -> None:
+    if cfg.get("automatic"):  # its thresholds and PageRank's layout are no explicit setting's
+        m.set_algorithm(m.AUTO)
+        m.set_sell_params(0, 0, 16384, 0)
+        return
     algo = {"sell": m.SELL, "merge": m.MERGE, "rowblock": m.ROWBLOCK}[cfg["algo"]]
     if cfg["algo"] == "rowblock":
         m.set_tile(cfg["tile"])
@@ -127,8 +131,8 @@ def tune_csr(m, precision: int, reps: int = 3, path: str | None = None, force: b
     names = {m.SELL: "sell", m.MERGE: "merge", m.ROWBLOCK: "rowblock"}
     cfg = {"algo": names[best["algorithm"]], "items": int(best["items"]), "tile": int(best["tile"]),
            "short_thr": int(best["short_thr"]), "long_thr": int(best["long_thr"]), "sigma": int(best["sigma"]),
-           "col_block": int(best["col_block"])}
-    apply_csr(m, cfg)
+           "col_block": int(best["col_block"]),
+           "automatic": best == trials[0]}  # the first candidate; the handle is set already
     entry = {"settings": cfg, "trials": len(trials), "best_ms": float(best.get("ms", 0.0))}
     store(k, entry, path)
     return dict(entry, cached=False, key=k)

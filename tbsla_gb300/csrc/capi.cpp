@@ -344,6 +344,7 @@ int tbsla_matrix_set_csr_algorithm(tbsla_matrix* m, int algorithm, int items) tr
       (algorithm != TBSLA_CSR_ROWBLOCK && items != 0 && items != 4 && items != 8 && items != 16))
     return TBSLA_ERR_INVALID_ARG;
   if (algorithm == TBSLA_CSR_MERGE && items == 0) items = 8;
+  m->csr_tuned = false;
   if (algorithm == TBSLA_CSR_SELL) m->sell_unroll = items;  // a launch parameter only; 0 = automatic
   if (m->csr_algo != algorithm || (algorithm == TBSLA_CSR_MERGE && m->merge_items != items)) {
     m->invalidate();

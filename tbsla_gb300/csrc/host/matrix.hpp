@@ -67,6 +67,7 @@ struct tbsla_matrix {
   int precision = TBSLA_F64;
   int csr_tile = 0;        // row-block budget (entries per block; 0: 1024 under the automatic kernel, else 2048)
   int csr_algo = -1;       // -1: automatic (default), 0: merge path, 1: row blocks, 2: sliced ELL
+  bool csr_tuned = false;  // csr_algo is the autotuner's choice for SpMV, not the caller's
   int merge_items = 8;     // merge path: items per thread
   int sell_short = 0;      // sliced ELL: rows up to this length, one lane each, sorted per window
                            // (0: by size: 16 .. 64, several column blocks 64 or 128)

@@ -87,3 +87,39 @@ def test_triplets_with_a_long_row(gpu, longest, fmt, prec):
     assert oracle.rel_err_normalized(m.spmv(x), oracle.coo_ax(n, row, col, w, x), scale) <= TOL
     entry = 12 if prec == "f64" else 8
     assert (m.device_bytes() > entry * len(row) + 4.3 * n) == (longest > 10_240)
+
+
+@pytest.mark.parametrize("n,mean", [(1000, 10), (50_000, 10), (100_000, 16)])
+def test_autotuned_handle(gpu, n, mean, tmp_path):
+    """The automatic setting is the first candidate; whichever wins, PageRank
+    keeps the layout that an untouched handle gives it, and the cache brings a
+    second handle to the same setting."""
+    from tbsla_gb300 import autotune as A
+
+    T = gpu
+    rng = np.random.default_rng(n)
+    rp = np.concatenate(([0], np.cumsum(rng.integers(1, 2 * mean, n)))).astype(np.int32)
+    ci = rng.integers(0, n, rp[-1]).astype(np.int32)
+    v = 1.0 / np.bincount(ci, minlength=n)[ci]
+    make = lambda: T.MatrixCSR.from_arrays(n, n, rp, ci, v)
+    m, fresh = make(), make()
+    best, trials = m.autotune(reps=3)
+    assert trials[0]["algorithm"] == m.ROWBLOCK and trials[0]["tile"] == 1024
+    assert best in trials and best["ms"] == min(t["ms"] for t in trials)
+    assert {(t["short_thr"], t["long_thr"]) for t in trials if t["algorithm"] == m.SELL} >= {(16, 16), (64, 64)}
+    sizes = []
+    for h in (m, fresh):
+        h.upload()
+        before = h.device_bytes()
+        x, it, _, ok = h.page_rank(0.85, 1e-10, 500)
+        assert ok and np.abs(x - oracle.pagerank(rp, ci, v, 0.85, 1e-10, it, stop_early=False)[0]).sum() <= 1e-10
+        sizes.append(h.device_bytes() - before)
+    assert sizes[1] > 0 and (sizes[0] == sizes[1] or best["algorithm"] == m.SELL)
+    path = str(tmp_path / "tune.json")
+    first, second = make(), make()
+    e = A.tune_csr(first, T.F64, path=path)
+    f = A.tune_csr(second, T.F64, path=path)
+    assert f["cached"] and e["settings"] == f["settings"]
+    first.upload()
+    second.upload()
+    assert first.device_bytes() == second.device_bytes()
