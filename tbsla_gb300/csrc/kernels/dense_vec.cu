@@ -131,7 +131,8 @@ __global__ void __launch_bounds__(NT) k_dense_rows_f64x2(const double* __restric
 // [2^-80, 2^80], sums of up to 2^31 of them finite, error terms normal): the
 // values are checked once at upload, x by the split kernel on every call,
 // whose CTAs leave a flag each; a launch that reads a set flag runs every row
-// in FP64, in the same kernel (no host round trip).
+// in FP64 instead, in the same kernel (no host round trip).  Bound there: the FP64 pipe for FP32 and BF16 values, HBM
+// and the pipe for FP64 ones.
 constexpr float kDfLo = 9.094947017729282e-13f;  // 2^-40
 constexpr float kDfHi = 1.099511627776e12f;      // 2^40
 
@@ -206,6 +207,7 @@ struct Step<double, VEC> {
       for (int k = 0; k < NV; k++) v[k] = ld_stream(p + min(c + 32 * k, last), pol);
     }
   }
+  __device__ __forceinline__ double value(int k) const { return v[k]; }
   // a = h + l: Dot2 on h (x as xh + xl), then l * xh into the error term
   // (l * xl is below 2^-48 of the product)
   __device__ __forceinline__ void add(float& s, float& c, int k, float xh, float xl) const {
@@ -228,6 +230,7 @@ struct Step<float, VEC> {
       for (int k = 0; k < NV; k++) v[k] = ld_stream(p + min(c + 32 * k, last), pol);
     }
   }
+  __device__ __forceinline__ double value(int k) const { return widen(v[k]); }
   __device__ __forceinline__ void add(float& s, float& c, int k, float xh, float xl) const {
     dot2_step(s, c, v[k], DF{xh, xl});
   }
@@ -248,11 +251,13 @@ struct Step<__nv_bfloat16, VEC> {  // a bfloat16 is the high half of its float; 
       }
     }
   }
+  __device__ __forceinline__ unsigned word(int k) const {
+    if constexpr (!VEC) return v[k] << 16;
+    return k & 1 ? v[k >> 1] & 0xffff0000u : v[k >> 1] << 16;
+  }
+  __device__ __forceinline__ double value(int k) const { return widen_bits(word(k)); }
   __device__ __forceinline__ void add(float& s, float& c, int k, float xh, float xl) const {
-    unsigned w;
-    if constexpr (!VEC) w = v[k] << 16;
-    else w = k & 1 ? v[k >> 1] & 0xffff0000u : v[k >> 1] << 16;
-    dot2_step(s, c, __uint_as_float(w), DF{xh, xl});
+    dot2_step(s, c, __uint_as_float(word(k)), DF{xh, xl});
   }
 };
 
@@ -277,6 +282,75 @@ __device__ __forceinline__ DF warp_sum_rows(DF (&t)[R]) {
   return t[0];
 }
 
+// The sum of row lane / (32 / R) of the warp's R rows from row0 on, of this
+// warp's columns, into y (y += sum; fresh: y = sum).
+template <int R>
+__device__ __forceinline__ void store_rows(double mine, long row0, int ln_row, int log2s, double* y, int fresh,
+                                           double (*s_part)[R]) {
+  constexpr int NW = NT / kWarp;
+  const int lane = threadIdx.x % kWarp, warp = threadIdx.x / kWarp, S = 1 << log2s;
+  const int r = lane / (kWarp / R);
+  const bool head = lane % (kWarp / R) == 0;
+  if (S == 1) {
+    if (head && row0 + r < ln_row) y[row0 + r] = add_rn(fresh ? 0.0 : y[row0 + r], mine);
+    return;
+  }
+  if (head) s_part[warp][r] = mine;
+  __syncthreads();
+  if (threadIdx.x < (NW >> log2s) * R) {
+    const int g = threadIdx.x / R, q = threadIdx.x % R;
+    const long row = ((long)blockIdx.x * (NW >> log2s) + g) * R + q;
+    double t = 0;
+    for (int k = 0; k < S; k++) t = add_rn(t, s_part[g * S + k][q]);
+    if (row < ln_row) y[row] = add_rn(fresh ? 0.0 : y[row], t);
+  }
+}
+
+// The same rows and columns in FP64 (x out of the range): a row at a time, eight
+// sums a lane, as short as those of 256 threads a row, so that the multiply-adds
+// do not wait for one another.  A function of its own that nothing comes after,
+// so that the double-float loop keeps its registers.
+template <class V, int R, bool VEC>
+__device__ __noinline__ void rows_f64(const V* a0, int rows, long row0, int ln_row, int ln_col, int log2s,
+                                      const double* x, double* y, int fresh, double (*s_part)[R]) {
+  constexpr int NV = Step<V, VEC>::NV, SC = 32 * NV;
+  const int lane = threadIdx.x % kWarp, S = 1 << log2s, part = threadIdx.x / kWarp & (S - 1);
+  const int nsteps = (ln_col + SC - 1) / SC;
+  const int last = ln_col - (VEC ? NV : 1), c0 = VEC ? NV * lane : lane;
+  const uint64_t pol = policy_evict_first();
+  double mine = 0;
+  for (int r = 0; r < rows; r++) {
+    const V* a = a0 + (size_t)r * ln_col;
+    double acc[8];
+#pragma unroll
+    for (int k = 0; k < 8; k++) acc[k] = 0;
+    auto add = [&](const Step<V, VEC>& f, int c, int to) {
+#pragma unroll
+      for (int k = 0; k < NV; k++) {
+        const int cc = VEC ? c + k : c + 32 * k;
+        const double xv = cc < ln_col ? x[cc] : 0.0;
+        acc[to + k] = fma_rn(f.value(k), xv, acc[to + k]);
+      }
+    };
+    for (int st = part; st < nsteps; st += 2 * S) {
+      Step<V, VEC> f0, f1;
+      const bool two = st + S < nsteps;
+      f0.load(a, st * SC + c0, last, pol);
+      f1.load(a, (two ? st + S : st) * SC + c0, last, pol);
+      add(f0, st * SC + c0, 0);
+      if (two) add(f1, (st + S) * SC + c0, 8 - NV);
+    }
+#pragma unroll
+    for (int o = 4; o > 0; o /= 2) {
+#pragma unroll
+      for (int k = 0; k < o; k++) acc[k] = add_rn(acc[k], acc[k + o]);
+    }
+    const double sum = warp_sum(acc[0]);
+    if (lane / (kWarp / R) == r) mine = sum;
+  }
+  store_rows<R>(mine, row0, ln_row, log2s, y, fresh, s_part);
+}
+
 // y += A x (fresh: y = A x).  The CTA's eight warps are 8 / S groups of R rows
 // times S = 1 << log2s parts of the columns (steps part, part + S, ...).  The
 // values of two steps are loaded, then used: 32 warps on an SM (64 registers)
@@ -298,8 +372,20 @@ __global__ void __launch_bounds__(NT, 4) k_dense_df(const V* __restrict__ A, int
   const V* const a0 = A + (size_t)min(row0, (long)ln_row - 1) * ln_col;
   const int rows = (int)min((long)R, max(1L, ln_row - row0));
   auto row_at = [&](int r) { return a0 + (size_t)min(r, rows - 1) * ln_col; };
-  int out = 0;  // x out of the range somewhere (looked at when the flags are there: after the sums)
+  const int last = ln_col - (VEC ? NV : 1), c0 = VEC ? NV * lane : lane;
+  // the first values on their way to L2 under the flags (24576 x 8192 BF16: 107.9
+  // -> 104 us)
+#pragma unroll
+  for (int r = 0; r < R; r++) {
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(row_at(r) + min(part * SC + c0, last)));
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(row_at(r) + min((part + S) * SC + c0, last)));
+  }
+  int out = 0;  // x out of the range somewhere: the same in every CTA
   for (int k = lane; k < nbad; k += kWarp) out |= bad[k];
+  if (__any_sync(0xffffffffu, out)) {
+    rows_f64<V, R, VEC>(a0, rows, row0, ln_row, ln_col, log2s, x, y, fresh, s_part);
+    return;
+  }
   // (sh, sc): the Dot2 sum of one step (FP32) or two of a lane, then folded
   // into (th, tl): the rounding of the carried errors grows with the entries
   // of one sum
@@ -320,7 +406,6 @@ __global__ void __launch_bounds__(NT, 4) k_dense_df(const V* __restrict__ A, int
       sh[r] = sc[r] = 0.f;
     }
   };
-  const int last = ln_col - (VEC ? NV : 1), c0 = VEC ? NV * lane : lane;
   auto load = [&](Step<V, VEC>(&f)[R], int st) {
 #pragma unroll
     for (int r = 0; r < R; r++) f[r].load(row_at(r), st * SC + c0, last, pol);
@@ -375,33 +460,7 @@ __global__ void __launch_bounds__(NT, 4) k_dense_df(const V* __restrict__ A, int
   DF t[R];
 #pragma unroll
   for (int r = 0; r < R; r++) t[r] = two_sum(th[r], tl[r]);
-  double mine = df_val(warp_sum_rows<R>(t));  // the sum of row lane / (32 / R)
-  if (__any_sync(0xffffffffu, out)) {
-#pragma unroll
-    for (int r = 0; r < R; r++) {
-      double acc = 0;
-      for (int st = part; st < nsteps; st += S)
-        for (int j = st * SC + lane; j < min(st * SC + SC, ln_col); j += kWarp)
-          acc = fma_rn(widen(ld_stream(row_at(r) + j, pol)), x[j], acc);
-      acc = warp_sum(acc);
-      if (lane / (kWarp / R) == r) mine = acc;
-    }
-  }
-  const int r = lane / (kWarp / R);
-  const bool head = lane % (kWarp / R) == 0;
-  if (S == 1) {
-    if (head && row0 + r < ln_row) y[row0 + r] = add_rn(fresh ? 0.0 : y[row0 + r], mine);
-    return;
-  }
-  if (head) s_part[warp][r] = mine;
-  __syncthreads();
-  if (threadIdx.x < (NW >> log2s) * R) {
-    const int g = threadIdx.x / R, q = threadIdx.x % R;
-    const long row = ((long)blockIdx.x * (NW >> log2s) + g) * R + q;
-    double t = 0;
-    for (int k = 0; k < S; k++) t = add_rn(t, s_part[g * S + k][q]);
-    if (row < ln_row) y[row] = add_rn(fresh ? 0.0 : y[row], t);
-  }
+  store_rows<R>(df_val(warp_sum_rows<R>(t)), row0, ln_row, log2s, y, fresh, s_part);
 }
 
 // FP64 rows with 16-byte aligned starts (ln_col even): 16-byte loads.
