@@ -118,21 +118,22 @@ __global__ void __launch_bounds__(NT) k_dense_rows_f64x2(const double* __restric
 //    rows are aligned for it) and their xh / xl, which serve all R rows, and
 //    adds them with compensated Dot2 steps (the product's and the sum's
 //    rounding errors carried exactly into a second float);
-//  * the lanes' pairs are summed across the warp in double-float (TwoSum-
-//    based additions), the R rows at once (each half of the warp goes on with
-//    half of the rows), and the column parts in FP64, in a fixed order.
-// Bound: HBM for FP64 and FP32 values (16384 x 8192: 161 and 97 us, 6.7 and
-// 5.5 TB/s with the launches), instruction issue (about 15 per entry) for BF16
-// (24576 x 8192: 104 us).  With a CTA per row, one row's x loads, its warp
-// reductions and a barrier came to more instructions than the entries
-// themselves: 177, 122 and 164 us, and 65 us for 9000 x 600 FP32, now 7.8.
+//  * the lanes' pairs are summed across the warp in FP64, the R rows at once
+//    (each half of the warp goes on with half of the rows), and so are the
+//    column parts, in a fixed order.
+// Bound: HBM for FP64 and FP32 values (16384 x 8192: 159 and 89 us, 6.8 and
+// 6.0 TB/s with the launches), instruction issue (about 15 per entry, 17 to 20
+// on short rows, see Sums) for BF16 (24576 x 8192: 103 us).  With a CTA per row,
+// one row's x loads, its warp reductions and a barrier came to more
+// instructions than the entries themselves: 178, 122 and 164 us, and 65 us for
+// 9000 x 600 FP32, now 8.3.
 // The float arithmetic is exact only inside the float exponent range, so the
 // path needs every nonzero |x| and |a| in [2^-40, 2^40] (products within
 // [2^-80, 2^80], sums of up to 2^31 of them finite, error terms normal): the
 // values are checked once at upload, x by the split kernel on every call,
 // whose CTAs leave a flag each; a launch that reads a set flag runs every row
-// in FP64 instead, in the same kernel (no host round trip).  Bound there: the FP64 pipe for FP32 and BF16 values, HBM
-// and the pipe for FP64 ones.
+// in FP64 instead, in the same kernel (no host round trip).  Bound there: the
+// FP64 pipe, and HBM for FP64 values.
 constexpr float kDfLo = 9.094947017729282e-13f;  // 2^-40
 constexpr float kDfHi = 1.099511627776e12f;      // 2^40
 
@@ -184,6 +185,19 @@ __device__ __forceinline__ void split_f64(double a, float& h, float& l) {
   l = __fmul_rn(__int2float_rn((int)(lo << 3) >> 3), scale);
 }
 
+// One term a (xh + xl) of a Dot2 sum: the rounding errors of product and sum are
+// carried into c with the small products, all of the term's before they meet c,
+// which then is rounded once a term (dot2_step: twice).  L: l * xh too.
+template <bool L = false>
+__device__ __forceinline__ void dense_step(float& s, float& c, float a, float xh, float xl, float l = 0.f) {
+  const float pr = __fmul_rn(a, xh);
+  float e = __fmaf_rn(a, xl, __fmaf_rn(a, xh, -pr));
+  if constexpr (L) e = __fmaf_rn(l, xh, e);
+  const DF t = two_sum(s, pr);
+  s = t.h;
+  c = __fadd_rn(c, __fadd_rn(e, t.l));
+}
+
 // A step is 32 * NV columns; one lane's NV values of a row's step, as loaded:
 // 16 bytes (FP64: 32).  VEC: columns c .. c + NV - 1, the row aligned for it;
 // else columns c, c + 32, ...  A column past the row's last one (`last`: its
@@ -208,13 +222,12 @@ struct Step<double, VEC> {
     }
   }
   __device__ __forceinline__ double value(int k) const { return v[k]; }
-  // a = h + l: Dot2 on h (x as xh + xl), then l * xh into the error term
+  // a = h + l: Dot2 on h (x as xh + xl), with l * xh among the small terms
   // (l * xl is below 2^-48 of the product)
   __device__ __forceinline__ void add(float& s, float& c, int k, float xh, float xl) const {
     float h, l;
     split_f64(v[k], h, l);
-    dot2_step(s, c, h, DF{xh, xl});
-    c = __fmaf_rn(l, xh, c);
+    dense_step<true>(s, c, h, xh, xl, l);
   }
 };
 template <bool VEC>
@@ -232,7 +245,7 @@ struct Step<float, VEC> {
   }
   __device__ __forceinline__ double value(int k) const { return widen(v[k]); }
   __device__ __forceinline__ void add(float& s, float& c, int k, float xh, float xl) const {
-    dot2_step(s, c, v[k], DF{xh, xl});
+    dense_step(s, c, v[k], xh, xl);
   }
 };
 template <bool VEC>
@@ -257,29 +270,51 @@ struct Step<__nv_bfloat16, VEC> {  // a bfloat16 is the high half of its float; 
   }
   __device__ __forceinline__ double value(int k) const { return widen_bits(word(k)); }
   __device__ __forceinline__ void add(float& s, float& c, int k, float xh, float xl) const {
-    dot2_step(s, c, __uint_as_float(word(k)), DF{xh, xl});
+    dense_step(s, c, __uint_as_float(word(k)), xh, xl);
   }
 };
 
 // The warp's sums of R values per lane: the halves of the warp go on with half
-// of the values each until one is left, which the remaining lanes add up.
-// Lanes [r * 32 / R, (r + 1) * 32 / R) get value r.
+// of the values each until one is left, which the remaining lanes add up.  Lanes
+// [r * 32 / R, (r + 1) * 32 / R) get value r.  In FP64: a double-float addition
+// rounds as much as some columns' terms do, and costs more.  With `brief`, the
+// halves in double-float (short rows, which have the error to spare and for
+// which the FP64 pipe would be the bound: 40,000 x 200 BF16 15.2 us, not 19.6).
 template <int R>
-__device__ __forceinline__ DF warp_sum_rows(DF (&t)[R]) {
-  int o = 16;
+__device__ __forceinline__ double warp_sum_rows(DF (&t)[R], bool brief) {
+  constexpr unsigned full = 0xffffffffu;
+  double sum;
+  if (R > 1 && brief) {
+    int o = 16;
 #pragma unroll
-  for (int n = R; n > 1; n /= 2, o /= 2) {
-    const bool up = threadIdx.x & o;
+    for (int n = R; n > 1; n /= 2, o /= 2) {
+      const bool up = threadIdx.x & o;
 #pragma unroll
-    for (int i = 0; i < n / 2; i++) {
-      const DF keep = up ? t[i + n / 2] : t[i], give = up ? t[i] : t[i + n / 2];
-      t[i] = df_add(keep, DF{__shfl_xor_sync(0xffffffffu, give.h, o), __shfl_xor_sync(0xffffffffu, give.l, o)});
+      for (int i = 0; i < n / 2; i++) {
+        const DF keep = up ? t[i + n / 2] : t[i], give = up ? t[i] : t[i + n / 2];
+        t[i] = df_add(keep, DF{__shfl_xor_sync(full, give.h, o), __shfl_xor_sync(full, give.l, o)});
+      }
     }
+    sum = add_rn(widen(t[0].h), widen(t[0].l));
+  } else {
+    double d[R];
+#pragma unroll
+    for (int r = 0; r < R; r++) d[r] = add_rn(widen(t[r].h), widen(t[r].l));
+    int o = 16;
+#pragma unroll
+    for (int n = R; n > 1; n /= 2, o /= 2) {
+      const bool up = threadIdx.x & o;
+#pragma unroll
+      for (int i = 0; i < n / 2; i++) {
+        const double keep = up ? d[i + n / 2] : d[i], give = up ? d[i] : d[i + n / 2];
+        d[i] = add_rn(keep, __shfl_xor_sync(full, give, o));
+      }
+    }
+    sum = d[0];
   }
 #pragma unroll
-  for (; o > 0; o /= 2)
-    t[0] = df_add(t[0], DF{__shfl_xor_sync(0xffffffffu, t[0].h, o), __shfl_xor_sync(0xffffffffu, t[0].l, o)});
-  return t[0];
+  for (int o = 16 / R; o > 0; o /= 2) sum = add_rn(sum, __shfl_xor_sync(full, sum, o));
+  return sum;
 }
 
 // The sum of row lane / (32 / R) of the warp's R rows from row0 on, of this
@@ -351,12 +386,27 @@ __device__ __noinline__ void rows_f64(const V* a0, int rows, long row0, int ln_r
   store_rows<R>(mine, row0, ln_row, log2s, y, fresh, s_part);
 }
 
+constexpr int kBriefColumns = 512;
+
+// How a lane's Dot2 sums are kept: their error grows with the entries of one sum
+// and with the folds of such sums into one pair, and a lane adds up to eight
+// times the entries that a thread of a CTA per row (the kernel before this one)
+// did.  Each is used where its error against 64 bits is no larger than that
+// kernel's, which holds 2.7e-15 of the 2-norm at 513 columns, 3.3e-15 (FP32 and
+// BF16) to 5e-15 (FP64) at 600 to 1000, twice that at 4096:
+enum Sums {
+  kLong,    // a step or two folded into one pair: error 3.4e-15 (FP32, 1544 to 4608 columns) to 6.8e-15
+  kFours,   // four entries, two or four pairs: 2.6 to 3.9e-15 (kLong 6.4 to 7.4e-15 at 600 to 1000 columns)
+  kPairs,   // two entries, four pairs: 2.2 to 3.3e-15; only for unaligned rows, which had the least error
+  kEights,  // eight entries, two pairs (BF16): 4.2 to 4.4e-15
+};
+
 // y += A x (fresh: y = A x).  The CTA's eight warps are 8 / S groups of R rows
 // times S = 1 << log2s parts of the columns (steps part, part + S, ...).  The
 // values of two steps are loaded, then used: 32 warps on an SM (64 registers)
 // keep as many loads in flight as 24 that load a step ahead (80 registers: BF16
 // 117, FP32 98, FP64 193 us where 109, 101 and 185 were taken then).
-template <class V, int R, bool VEC>
+template <class V, int R, bool VEC, Sums SUMS>
 __global__ void __launch_bounds__(NT, 4) k_dense_df(const V* __restrict__ A, int ln_row, int ln_col, int log2s,
                                                    const float* xs, const double* x, const int* bad, int nbad,
                                                    double* y, int fresh) {
@@ -386,22 +436,28 @@ __global__ void __launch_bounds__(NT, 4) k_dense_df(const V* __restrict__ A, int
     rows_f64<V, R, VEC>(a0, rows, row0, ln_row, ln_col, log2s, x, y, fresh, s_part);
     return;
   }
-  // (sh, sc): the Dot2 sum of one step (FP32) or two of a lane, then folded
-  // into (th, tl): the rounding of the carried errors grows with the entries
-  // of one sum
-  float sh[R], sc[R], th[R], tl[R];
+  // (sh, sc): the Dot2 sum of P entries of a lane (kLong: of one step, FP32, or
+  // two), then folded into one of the sums (th, tl) in turn
+  constexpr bool LONG = SUMS == kLong;
+  constexpr int P = SUMS == kEights ? 8 : SUMS == kPairs ? 2 : 4;
+  constexpr int CH = LONG ? 1 : SUMS == kEights || (SUMS == kFours && NV == 4) ? 2 : 4;
+  float sh[R], sc[R], th[CH][R], tl[CH][R];
 #pragma unroll
-  for (int r = 0; r < R; r++) sh[r] = sc[r] = th[r] = tl[r] = 0.f;
-  auto fold = [&]() {
+  for (int r = 0; r < R; r++) {
+    sh[r] = sc[r] = 0.f;
+#pragma unroll
+    for (int q = 0; q < CH; q++) th[q][r] = tl[q][r] = 0.f;
+  }
+  auto fold = [&](int q) {
 #pragma unroll
     for (int r = 0; r < R; r++) {
-      const DF t = two_sum(th[r], sh[r]);
-      th[r] = t.h;
-      tl[r] = __fadd_rn(tl[r], __fadd_rn(t.l, sc[r]));
-      if constexpr (sizeof(V) != 8) {  // keeps tl small against th
-        const DF u = fast_two_sum(th[r], tl[r]);
-        th[r] = u.h;
-        tl[r] = u.l;
+      const DF t = two_sum(th[q][r], sh[r]);
+      th[q][r] = t.h;
+      tl[q][r] = __fadd_rn(tl[q][r], __fadd_rn(t.l, sc[r]));
+      if constexpr (!LONG || sizeof(V) != 8) {  // keeps tl small against th
+        const DF u = fast_two_sum(th[q][r], tl[q][r]);
+        th[q][r] = u.h;
+        tl[q][r] = u.l;
       }
       sh[r] = sc[r] = 0.f;
     }
@@ -410,7 +466,7 @@ __global__ void __launch_bounds__(NT, 4) k_dense_df(const V* __restrict__ A, int
 #pragma unroll
     for (int r = 0; r < R; r++) f[r].load(row_at(r), st * SC + c0, last, pol);
   };
-  auto add = [&](const Step<V, VEC>(&f)[R], int st) {
+  auto add = [&](const Step<V, VEC>(&f)[R], int st, int half) {
     const int c = st * SC + c0;
 #pragma unroll
     for (int k0 = 0; k0 < NV; k0 += 4) {
@@ -438,6 +494,7 @@ __global__ void __launch_bounds__(NT, 4) k_dense_df(const V* __restrict__ A, int
       for (int k = 0; k < 4; k++) {
 #pragma unroll
         for (int r = 0; r < R; r++) f[r].add(sh[r], sc[r], k0 + k, xh[k], xl[k]);
+        if (!LONG && (k0 + k + 1) % P == 0) fold(((k0 + k) / P + half * (NV / P)) % CH);
       }
     }
   };
@@ -446,21 +503,25 @@ __global__ void __launch_bounds__(NT, 4) k_dense_df(const V* __restrict__ A, int
     Step<V, VEC> f0[R], f1[R];
     load(f0, st);
     load(f1, st + S);
-    add(f0, st);
-    if constexpr (sizeof(V) == 4) fold();
-    add(f1, st + S);
-    fold();
+    add(f0, st, 0);
+    if constexpr (LONG && sizeof(V) == 4) fold(0);
+    add(f1, st + S, 1);
+    if constexpr (LONG) fold(0);
   }
   if (st < nsteps) {
     Step<V, VEC> f0[R];
     load(f0, st);
-    add(f0, st);
+    add(f0, st, 0);
+    if constexpr (LONG) fold(0);
   }
-  fold();
   DF t[R];
 #pragma unroll
-  for (int r = 0; r < R; r++) t[r] = two_sum(th[r], tl[r]);
-  store_rows<R>(df_val(warp_sum_rows<R>(t)), row0, ln_row, log2s, y, fresh, s_part);
+  for (int r = 0; r < R; r++) {
+    t[r] = DF{th[0][r], tl[0][r]};
+#pragma unroll
+    for (int q = 1; q < CH; q++) t[r] = df_add(t[r], DF{th[q][r], tl[q][r]});
+  }
+  store_rows<R>(warp_sum_rows<R>(t, VEC && ln_col <= kBriefColumns), row0, ln_row, log2s, y, fresh, s_part);
 }
 
 // FP64 rows with 16-byte aligned starts (ln_col even): 16-byte loads.
@@ -625,17 +686,17 @@ cudaError_t dense_values_df_range(const void* vals, int prec, size_t n, int* fla
 }
 
 namespace {
-template <class V, int R, bool VEC>
+template <class V, int R, bool VEC, Sums SUMS>
 cudaError_t launch_dense_df(const V* a, int ln_row, int ln_col, int log2s, const float* xs, const double* x, const int* bad,
                      int nbad, double* y, int fresh, cudaStream_t s) {
   const long warps = (((long)ln_row + R - 1) / R) << log2s;
   const unsigned grid = (unsigned)((warps + NT / kWarp - 1) / (NT / kWarp));
-  return launch_early(k_dense_df<V, R, VEC>, grid, NT, 0, s, a, ln_row, ln_col, log2s, xs, x, bad, nbad, y, fresh);
+  return launch_early(k_dense_df<V, R, VEC, SUMS>, grid, NT, 0, s, a, ln_row, ln_col, log2s, xs, x, bad, nbad, y, fresh);
 }
 
-// Rows per warp: 4 (FP32) or 2 (the others, whose rows cost more registers a
-// step: with 4, BF16 24576 x 8192 takes 120 us where 2 take 109, FP64 20000 x
-// 8192 238 and 204), fewer where the GPU would not get half a warp's work for
+// Rows per warp: 4 (FP32) or 2 (the others and kPairs, whose rows cost more
+// registers a step: with 4, BF16 24576 x 8192 takes 120 us where 2 take 109, FP64
+// 20000 x 8192 238 and 204), fewer where the GPU would not get half a warp's work for
 // each resident warp.  Column parts: until there are four for each resident
 // warp (FP32 16384 x 8192 with 1 / 2 / 4 / 8 parts: 106 / 104 / 102 / 100 us;
 // BF16 24576 x 8192: 106 / 105 / 111 / 128), while a part keeps four steps (FP64
@@ -644,10 +705,10 @@ cudaError_t launch_dense_df(const V* a, int ln_row, int ln_col, int log2s, const
 // reads long pieces of few rows, and HBM gives more for fewer streams (20000
 // rows, 2 / 4 / 8 parts: 5120 columns 133 / 132 / 144 us, 16384 columns 396 /
 // 381 / 384).
-template <class V, bool VEC>
+template <class V, bool VEC, Sums SUMS>
 cudaError_t dense_df_shape(const V* a, int ln_row, int ln_col, const float* xs, const double* x, const int* bad, int nbad,
                     double* y, int fresh, cudaStream_t s) {
-  constexpr int kMost = sizeof(V) == 4 ? 4 : 2;
+  constexpr int kMost = sizeof(V) == 4 && SUMS != kPairs ? 4 : 2;
   constexpr long kWarps = 152L * 32;
   constexpr int SC = 32 * Step<V, VEC>::NV;
   const int nsteps = (ln_col + SC - 1) / SC;
@@ -658,10 +719,24 @@ cudaError_t dense_df_shape(const V* a, int ln_row, int ln_col, const float* xs, 
   int log2s = 0;
   while (log2s < most && (((long)ln_row + r - 1) / r << log2s) < 4 * kWarps) log2s++;
   if (sizeof(V) == 8 && VEC && nsteps >= 40) log2s = std::max(log2s, 2);
-  if (r == 1) return launch_dense_df<V, 1, VEC>(a, ln_row, ln_col, log2s, xs, x, bad, nbad, y, fresh, s);
+  if (r == 1) return launch_dense_df<V, 1, VEC, SUMS>(a, ln_row, ln_col, log2s, xs, x, bad, nbad, y, fresh, s);
   if constexpr (kMost >= 4)
-    if (r == 4) return launch_dense_df<V, 4, VEC>(a, ln_row, ln_col, log2s, xs, x, bad, nbad, y, fresh, s);
-  return launch_dense_df<V, 2, VEC>(a, ln_row, ln_col, log2s, xs, x, bad, nbad, y, fresh, s);
+    if (r == 4) return launch_dense_df<V, 4, VEC, SUMS>(a, ln_row, ln_col, log2s, xs, x, bad, nbad, y, fresh, s);
+  return launch_dense_df<V, 2, VEC, SUMS>(a, ln_row, ln_col, log2s, xs, x, bad, nbad, y, fresh, s);
+}
+
+// The sums by the columns (see Sums; us of 24,000 rows, against kLong): BF16
+// fours to 2304 columns (1104: 23.5, 19.9; 2048, 20,000 rows: 33.6, 28.2), eights to
+// 4608 (2312: 41.2, 40.7), FP32 fours to 1536 (1504: 36.2, 33.2), FP64, bound by HBM,
+// fours to 4608 (2312: 77.8, 76.6).
+template <class V, bool VEC>
+cudaError_t dense_df_sums(const V* a, int ln_row, int ln_col, const float* xs, const double* x, const int* bad, int nbad,
+                          double* y, int fresh, cudaStream_t s) {
+  constexpr int fours = sizeof(V) == 4 ? 1536 : sizeof(V) == 2 ? 2304 : 4608;
+  if (ln_col <= fours) return dense_df_shape<V, VEC, kFours>(a, ln_row, ln_col, xs, x, bad, nbad, y, fresh, s);
+  if constexpr (sizeof(V) == 2)
+    if (ln_col <= 4608) return dense_df_shape<V, VEC, kEights>(a, ln_row, ln_col, xs, x, bad, nbad, y, fresh, s);
+  return dense_df_shape<V, VEC, kLong>(a, ln_row, ln_col, xs, x, bad, nbad, y, fresh, s);
 }
 
 template <class V>
@@ -672,8 +747,9 @@ cudaError_t dense_df_vec(const void* vals, int ln_row, int ln_col, const float* 
   // and holds whole vectors (xs from cudaMalloc)
   constexpr int NV = Step<V, true>::NV;
   if ((uintptr_t)vals % 16 == 0 && (uintptr_t)xs % 16 == 0 && ln_col % NV == 0)
-    return dense_df_shape<V, true>(a, ln_row, ln_col, xs, x, bad, nbad, y, fresh, s);
-  return dense_df_shape<V, false>(a, ln_row, ln_col, xs, x, bad, nbad, y, fresh, s);
+    return dense_df_sums<V, true>(a, ln_row, ln_col, xs, x, bad, nbad, y, fresh, s);
+  if (ln_col <= 1100) return dense_df_shape<V, false, kPairs>(a, ln_row, ln_col, xs, x, bad, nbad, y, fresh, s);
+  return dense_df_sums<V, false>(a, ln_row, ln_col, xs, x, bad, nbad, y, fresh, s);
 }
 }  // namespace
 
