@@ -43,6 +43,7 @@
 #include "host/matrix.hpp"
 #include "kernels/common.cuh"
 #include "kernels/kernels.hpp"
+#include "probe_rows.hpp"
 #include "tbsla_gb300.h"
 
 namespace {
@@ -453,11 +454,12 @@ __global__ void __launch_bounds__(NT) k_head(int n, const int* __restrict__ lrow
 constexpr int PMAX = 16;
 
 // Y = A X on A's pattern (FP32 values).
+template <bool WIDE>
 __global__ void k_spmm_a(int n, int P, const int* __restrict__ rowptr, const int* __restrict__ colidx,
                          const float* __restrict__ a, const float* __restrict__ X, float* __restrict__ Y) {
   const long len = (long)n * P;
   for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < len; t += (long)gridDim.x * blockDim.x) {
-    const int i = (int)((unsigned)t / (unsigned)P), p = (int)(t - (long)i * P);
+    const int i = (int)tbsla_gpu::probe_row<WIDE>(t, P), p = (int)(t - (long)i * P);
     float acc = 0.f;
     for (int k = rowptr[i]; k < rowptr[i + 1]; k++) acc += a[k] * X[(long)colidx[k] * P + p];
     Y[t] = acc;
@@ -465,12 +467,13 @@ __global__ void k_spmm_a(int n, int P, const int* __restrict__ rowptr, const int
 }
 
 // Y = L X (rows of L) or Y = L^T X (columns of L, through the L^T index).
+template <bool WIDE>
 __global__ void k_spmm_l(int n, int P, const int* __restrict__ ptr, const int* __restrict__ idx,
                          const int* __restrict__ other, const float* __restrict__ lval, int transpose,
                          const float* __restrict__ X, float* __restrict__ Y) {
   const long len = (long)n * P;
   for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < len; t += (long)gridDim.x * blockDim.x) {
-    const int i = (int)((unsigned)t / (unsigned)P), p = (int)(t - (long)i * P);
+    const int i = (int)tbsla_gpu::probe_row<WIDE>(t, P), p = (int)(t - (long)i * P);
     float acc = 0.f;
     for (int k = ptr[i]; k < ptr[i + 1]; k++) {
       const int q = transpose ? idx[k] : k;  // L entry; its column (L) or row (L^T):
@@ -1143,12 +1146,15 @@ int backward(const float* wq, Work& w, double* dloss, float* grad, cudaStream_t 
   const int n = w.n, P = w.P, gw = warp_grid(n), gq = warp_grid(((long)n + NB - 1) / NB);
   const long len = (long)n * P;
   const int gp = row_grid(len);
-  k_spmm_a<<<gp, NT, 0, s>>>(n, P, w.rowptr.p, w.colidx.p, w.aval.p, w.Z.p, w.U.p);
-  k_spmm_l<<<gp, NT, 0, s>>>(n, P, w.trowptr.p, w.tidx.p, w.lrow.p, w.lval.p, 1, w.U.p, w.V.p);
-  k_spmm_l<<<gp, NT, 0, s>>>(n, P, w.lrowptr.p, nullptr, w.lcol.p, w.lval.p, 0, w.V.p, w.W.p);
+  const bool wide = tbsla_gpu::probe_rows_wide(len);
+  const auto spmm_a = wide ? k_spmm_a<true> : k_spmm_a<false>;
+  const auto spmm_l = wide ? k_spmm_l<true> : k_spmm_l<false>;
+  spmm_a<<<gp, NT, 0, s>>>(n, P, w.rowptr.p, w.colidx.p, w.aval.p, w.Z.p, w.U.p);
+  spmm_l<<<gp, NT, 0, s>>>(n, P, w.trowptr.p, w.tidx.p, w.lrow.p, w.lval.p, 1, w.U.p, w.V.p);
+  spmm_l<<<gp, NT, 0, s>>>(n, P, w.lrowptr.p, nullptr, w.lcol.p, w.lval.p, 0, w.V.p, w.W.p);
   MCK(cudaMemsetAsync(dloss, 0, sizeof(double), s));
   k_residual<<<std::min(gp, 152 * 2), NT, 0, s>>>(len, 1.f / (float)len, w.W.p, w.Z.p, w.G.p, dloss);
-  k_spmm_l<<<gp, NT, 0, s>>>(n, P, w.trowptr.p, w.tidx.p, w.lrow.p, w.lval.p, 1, w.G.p, w.GV.p);
+  spmm_l<<<gp, NT, 0, s>>>(n, P, w.trowptr.p, w.tidx.p, w.lrow.p, w.lval.p, 1, w.G.p, w.GV.p);
   k_dl<<<row_grid(w.nl), NT, 0, s>>>(w.nl, P, w.lrow.p, w.lcol.p, w.G.p, w.V.p, w.U.p, w.GV.p, w.dl.p);
   MCK(cudaMemsetAsync(grad, 0, NPARAMS * sizeof(float), s));
   k_head_bwd<<<std::min(gq, 152 * 6), NT, 0, s>>>(n, w.lrowptr.p, w.lcol.p, w.lsrc.p, w.trowptr.p, w.tidx.p,
