@@ -68,8 +68,9 @@ cudaError_t csr_merge_spmv_noalloc(const double* vals, const int* rowptr, const 
 // most short_thr entries take one lane each and are sorted by length within
 // windows of `sigma` consecutive rows; longer rows take the fewest lanes (up
 // to 32) that keep their slice at most long_thr steps wide and are sorted by
-// length over the whole block.  A row that 32 lanes cannot hold in long_thr
-// steps is cut into pieces of at most 32 * long_thr consecutive entries, a
+// length over the whole block.  A row that 32 lanes cannot hold in `piece`
+// steps (long_thr; twice that for FP64 values from 2^22 entries on, automatic
+// thresholds) is cut into pieces of at most 32 * piece consecutive entries, a
 // slice each; the warp that finishes a row's last piece adds the pieces'
 // sums in piece order.  One warp per slice, fetched dynamically, widest
 // slices first; lanes past their row's end issue no loads, so padding costs

@@ -123,3 +123,58 @@ def test_autotuned_handle(gpu, n, mean, tmp_path):
     first.upload()
     second.upload()
     assert first.device_bytes() == second.device_bytes()
+
+
+@pytest.mark.parametrize("count", [(1 << 19) - 1, 1 << 19, (3 << 20) - 1, 3 << 20])
+@pytest.mark.parametrize("longest", [64, 65])
+def test_automatic_kernel_by_size(gpu, count, longest):
+    """Row blocks up to 2^19 entries, up to 3 2^20 where no row is longer than
+    64, sliced ELL from there on: told by the bytes (the sliced-ELL copy holds
+    the entries twice)."""
+    T = gpu
+    n = 100_000
+    lens = np.full(n, count // n)
+    lens[n // 2] = longest
+    rest = count - lens.sum()
+    others = np.delete(np.arange(n), n // 2)
+    lens[others[: abs(rest)]] += np.sign(rest)
+    assert lens.sum() == count and lens.max() == longest and lens[n // 2] == longest
+    m, x, ref, scale = csr(T, n, lens, count + longest)
+    y = m.spmv(x)
+    assert oracle.rel_err_normalized(y, ref, scale) <= TOL
+    sell = count >= 3 << 20 or (count >= 1 << 19 and longest > 64)
+    assert (m.device_bytes() > 24 * count) == sell
+    m.set_algorithm(m.SELL if sell else m.ROWBLOCK)
+    if not sell:
+        m.set_tile(1024)
+    assert np.array_equal(m.spmv(x), y)
+
+
+@pytest.mark.parametrize("prec", ["f64", "f32"])
+@pytest.mark.parametrize("params,steps", [((0, 0, 16384, 0), 16), ((64, 64, 16384, 0), 64), ((8, 32, 16384, 0), 32)])
+def test_cuts_at_the_threshold(gpu, params, steps, prec):
+    """One column block, rows around one, two and three pieces of 32 lanes x
+    `steps` entries (16: the automatic threshold below 2^22 entries).  The
+    pieces of a cut row are told by the bytes: 8 a piece for its place, 8 for
+    its sum, and a slice of its own."""
+    T = gpu
+    n, cut = 40_000, 32 * steps
+    around = [cut - 1, cut, cut + 1, 2 * cut - 1, 2 * cut, 2 * cut + 1, 3 * cut, 3 * cut + 1]
+    size = {}
+    for which in ("cut", "one shorter"):
+        lens = np.full(n, 6)
+        lens[500 * (1 + np.arange(len(around)))] = np.array(around) - (which == "one shorter")
+        m, x, _, _ = csr(T, n, lens, steps)
+        m.set_precision({"f64": T.F64, "f32": T.F32}[prec])
+        m.set_algorithm(m.SELL)
+        m.set_sell_params(*params)
+        a = m.arrays()
+        v = a["values"] if prec == "f64" else a["values"].astype(np.float32).astype(np.float64)
+        ref = oracle.csr_ax(a["rowptr"], a["colidx"], v, x)
+        scale = oracle.csr_absrow(a["rowptr"], a["colidx"], v, x)
+        y = m.spmv(x)
+        assert oracle.rel_err_normalized(y, ref, scale) <= TOL
+        assert np.array_equal(m.spmv(x), y)
+        size[which] = m.device_bytes()
+    # lengths one shorter: cut + 1 -> cut, 2 cut + 1 -> 2 cut, 3 cut + 1 -> 3 cut: three pieces and one cut row fewer
+    assert size["cut"] - size["one shorter"] > 3 * (8 + 8 + 16 + 8 * 32)
