@@ -244,8 +244,8 @@ namespace {
 
 // Stable counting sort of COO/SCOO triplets by row (device copy order).
 // ends[i]: one past the last triplet of row rmin + i.
-void sort_by_row(const tbsla_matrix* m, long nnz, int rmin, int rmax, std::vector<int>& rows,
-                 std::vector<int>& cols, std::vector<double>& vals, std::vector<long>& ends) {
+void sort_by_row(const tbsla_matrix* m, long nnz, int rmin, int rmax, std::vector<int>& cols,
+                 std::vector<double>& vals, std::vector<long>& ends) {
   const int* r = m->idx0.data();
   const int* c = m->idx1.data();
   const double* v = m->values.data();
@@ -253,12 +253,10 @@ void sort_by_row(const tbsla_matrix* m, long nnz, int rmin, int rmax, std::vecto
   std::vector<long> pos(span + 1, 0);
   for (long k = 0; k < nnz; k++) pos[r[k] - rmin + 1]++;
   for (size_t i = 0; i < span; i++) pos[i + 1] += pos[i];
-  rows.resize(nnz);
   cols.resize(nnz);
   vals.resize(nnz);
   for (long k = 0; k < nnz; k++) {
     long p = pos[r[k] - rmin]++;
-    rows[p] = r[k];
     cols[p] = c[k];
     vals[p] = v[k];
   }
@@ -382,7 +380,9 @@ int build_sell(const tbsla_matrix* m, DeviceMatrix* d, int n, int nc, int f_col,
   const int W = (int)(((long)nc + P - 1) / P);
   std::vector<int> lens((size_t)P * n, 0);
   if (P == 1) {
-    for (int i = 0; i < n; i++) lens[i] = rp[i + 1] - rp[i];
+    parallel_for(n, [&](long b, long e) {
+      for (long i = b; i < e; i++) lens[i] = rp[i + 1] - rp[i];
+    });
   } else {
     parallel_for(n, [&](long b, long e) {
       for (long i = b; i < e; i++)
@@ -511,17 +511,23 @@ int build_coo_rows(const tbsla_matrix* m, DeviceMatrix* d, const std::vector<lon
                    const std::vector<int>& cols, const std::vector<double>& vals) {
   const tbsla_info& I = m->info;
   const bool scoo = m->format == TBSLA_SCOO;
-  std::vector<int> rp(1, 0);
-  rp.insert(rp.end(), ends.begin(), ends.end());
-  const int n = (int)rp.size() - 1;
+  const int n = (int)ends.size();
+  std::vector<int> rp((size_t)n + 1, 0);
+  for (int i = 0; i < n; i++) rp[i + 1] = (int)ends[i];
+  struct Settle {  // rp, cols and vals outlive their copies on every way out
+    DeviceMatrix* d;
+    ~Settle() { cudaStreamSynchronize(d->stream); }
+  } settle{d};
   int st = upload_ints(d, &d->idx0, rp.data(), rp.size());
   if (!st) st = upload_ints(d, &d->idx1, cols.data(), cols.size());
   if (!st) st = upload_values(d, vals.data(), vals.size());
-  st = settled(d, st);
   if (st) return st;
-  int longest = 0;
-  for (int i = 0; i < n; i++) longest = std::max(longest, rp[i + 1] - rp[i]);
-  if (row_blocks_first(rp.data(), n) && longest <= kCooRowBlockMost) {
+  auto longest = [&]() {
+    int l = 0;
+    for (int i = 0; i < n; i++) l = std::max(l, rp[i + 1] - rp[i]);
+    return l;
+  };
+  if (row_blocks_first(rp.data(), n) && longest() <= kCooRowBlockMost) {
     d->algo = TBSLA_CSR_ROWBLOCK;
     d->items = 4;
     int* blocks = nullptr;
@@ -624,16 +630,19 @@ int build(const tbsla_matrix* m, DeviceMatrix* d) {
       }
       d->min_row = rmin;
       d->max_row = rmax;
-      std::vector<int> rows, cols;
+      std::vector<int> cols;
       std::vector<double> vals;
       std::vector<long> ends;
-      sort_by_row(m, nnz, rmin, rmax, rows, cols, vals, ends);
+      sort_by_row(m, nnz, rmin, rmax, cols, vals, ends);
       int st = TBSLA_OK;
       if (nnz < INT_MAX && (long)rmax - rmin < nnz) {
         st = build_coo_rows(m, d, ends, cols, vals);
         if (st != TBSLA_ERR_ALLOC) return st;
         d->free_rows();  // no room for the copies: the triplets alone take less
       }
+      std::vector<int> rows(nnz);
+      for (size_t i = 0; i < ends.size(); i++)
+        std::fill(rows.begin() + (i ? ends[i - 1] : 0), rows.begin() + ends[i], rmin + (int)i);
       st = upload_ints(d, &d->idx0, rows.data(), nnz);
       if (!st) st = upload_ints(d, &d->idx1, cols.data(), nnz);
       if (!st) st = upload_values(d, vals.data(), nnz);
