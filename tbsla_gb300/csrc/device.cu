@@ -497,7 +497,7 @@ int build_sell(const tbsla_matrix* m, DeviceMatrix* d, int n, int nc, int f_col,
 // layout is filled (12 bytes an entry, FP64, where the triplets take 16).  Only
 // where a row of the range has a triplet on average: else the arrays over the
 // rows outgrow the triplets.
-// Bound: the gathers of x, as for CSR.  FP64, 2^22 rows x 10: 251 -> 183 us (with
+// Bound: the gathers of x, as for CSR.  FP64, 2^22 rows x 10: 250 -> 174 us (with
 // triplet chunks: 142 us of gathers, key compares and the carry pass on top);
 // 10,000 x 14: 14.5 -> 6.2; power-law rows, 10^6 x 14: 87 -> 69.
 // A row longer than kCooRowBlockMost triplets goes to sliced ELL at every size,

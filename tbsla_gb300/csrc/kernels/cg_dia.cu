@@ -45,8 +45,8 @@
 // Per-system scalars are kept in shared memory by every CTA and updated
 // redundantly from the same global sums after each barrier, so no CTA waits
 // for another to publish them.  The sums rotate through three accumulator
-// slots: CTA 0 clears the slot two phases ahead, which no CTA reads or
-// writes at that time.
+// slots: CTA 0 clears the next phase's slot, which no CTA reads or writes
+// during this one.
 //
 // Every grid-wide wait is bounded (`wait_ns`, globaltimer): a CTA whose wait
 // runs out sets the error word and returns, and every other CTA returns at
@@ -392,9 +392,8 @@ __global__ void __launch_bounds__(PNT, 3) k_cg_persistent(DiaCg c) {
   int g = 0;   // iteration parity of the R / P buffers
   bool init = true;
   auto slot = [&](int p) { return c.acc + (size_t)(p % 3) * 4 * ns; };
-  // CTA 0 clears the slot and the claim counters two phases ahead (read at
-  // the start of the previous phase by every CTA, written next in the
-  // following phase)
+  // CTA 0 clears the next phase's slot and claim counters (last read before
+  // this phase began by every CTA, written next in the following phase)
   auto clear_ahead = [&]() {
     if (blockIdx.x == 0) {
       double* a = slot(ph + 1);

@@ -204,8 +204,8 @@ struct BatchPlan {
 // wave is a small part of the step, at least 64 (below that the start of an
 // item, three dependent loads, is most of it) and at most 1024.  32 vectors,
 // FP32 values, us a step with items of 64 / 256 / 512 / 1024 / 2048 entries:
-// 1,220 / 911 / 796 / 785 / 791 at 2^20 nodes (14.8 M entries), 66 / 65 / 96 /
-// 141 / 241 at 20,000; this rule: 780 and 66.
+// 1,162 / 853 / 740 / 727 / 734 at 2^20 nodes (14.8 M entries), 60 / 59 / 75 /
+// 94 / 171 at 20,000; this rule: 723 and 59.
 int batch_plan_budget(long nnz, int n, int warps);
 void batch_plan_build(const int* rowptr, int n, int budget, std::vector<int4>* items, std::vector<int>* piece_cut,
                       std::vector<int>* cut_first);

@@ -354,18 +354,18 @@ struct StreamF64 {
 // stream, GB X-row gathers in flight whatever the row boundaries, finishing
 // each row (the same epilogue) where its last entry is added.  Each row's
 // products are added in entry order with the same steps, so Y is the same
-// bit for bit as with a warp per row; only the order in which rows enter the
-// norms' partial sums differs.  Rows of a few entries (most rows of a
+// bit for bit as with a warp per row, cut rows apart (below), and the order in
+// which rows enter the norms' partial sums differs.  Rows of a few entries (most rows of a
 // power-law graph) then share one gather latency instead of paying one each,
 // and a row's epilogue operands (T, X, w) are loaded when the previous row
 // finishes.
 //
 // A row longer than an item is cut into pieces, an item each and the first
 // ones claimed: one warp walking a hub row was the critical path of the step
-// (2^20 nodes, 14.8 M
-// entries, the longest row 35,187, 32 vectors, FP32 values: 3.95 -> 0.77 ms a
-// step; FP64 values 6.2 -> 1.4 ms).  The warp that finishes a row's last piece adds the pieces'
-// sums in entry order, in FP64, and runs the row's epilogue.
+// (2^20 nodes, 14.8 M entries, the longest row 35,187, 32 vectors, FP32 values:
+// 3.95 -> 0.72 ms a step; FP64 values 6.2 -> 1.4 ms).  The warp that finishes a
+// row's last piece adds the pieces' sums in entry order, in FP64, and runs the
+// row's epilogue.
 //
 // The kernel is bound by instruction issue and by how many warps hide the
 // gathers (FP64 values: by the FP64 pipe), so the per-entry work is kept
