@@ -1179,7 +1179,8 @@ double stored_value(double v, int prec) {
 bool column_weights_device(const tbsla_matrix* m, DeviceMatrix* d, std::vector<double>& w, int* st) {
   const tbsla_info& I = m->info;
   const long n = d->nnz - m->idx0[0];
-  if (n < kColumnSumsMin || n >= INT_MAX) return false;
+  // (the kernels' 32-bit indexes run a few warps past an end)
+  if (n < kColumnSumsMin || n > INT_MAX - 256) return false;
   unsigned* scratch = nullptr;
   if (dalloc(&scratch, (size_t)column_sums_scratch(n, I.ln_col)) != TBSLA_OK) return false;
   struct Free {
