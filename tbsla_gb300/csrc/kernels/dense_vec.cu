@@ -121,8 +121,8 @@ __global__ void __launch_bounds__(NT) k_dense_rows_f64x2(const double* __restric
 //  * the lanes' pairs are summed across the warp in FP64, the R rows at once
 //    (each half of the warp goes on with half of the rows), and so are the
 //    column parts, in a fixed order.
-// Bound: HBM for FP64 and FP32 values (16384 x 8192: 159 and 89 us, 6.8 and
-// 6.0 TB/s with the launches), instruction issue (about 15 per entry, 17 to 20
+// Bound: HBM for FP64 and FP32 values (16384 x 8192: 160 and 89 us, 6.7 and
+// 6.0 TB/s with the launches), instruction issue (about 15 per entry, 16 to 18
 // on short rows, see Sums) for BF16 (24576 x 8192: 103 us).  With a CTA per row,
 // one row's x loads, its warp reductions and a barrier came to more
 // instructions than the entries themselves: 178, 122 and 164 us, and 65 us for
@@ -395,10 +395,10 @@ constexpr int kBriefColumns = 512;
 // kernel's, which holds 2.7e-15 of the 2-norm at 513 columns, 3.3e-15 (FP32 and
 // BF16) to 5e-15 (FP64) at 600 to 1000, twice that at 4096:
 enum Sums {
-  kLong,    // a step or two folded into one pair: error 3.4e-15 (FP32, 1544 to 4608 columns) to 6.8e-15
-  kFours,   // four entries, two or four pairs: 2.6 to 3.9e-15 (kLong 6.4 to 7.4e-15 at 600 to 1000 columns)
+  kLong,    // a step or two folded into one pair: error 3.4 to 5.2e-15 (FP32, FP64), 6.8e-15 (BF16)
+  kFours,   // four entries, two or four pairs: 2.6 to 3.9e-15
   kPairs,   // two entries, four pairs: 2.2 to 3.3e-15; only for unaligned rows, which had the least error
-  kEights,  // eight entries, two pairs (BF16): 4.2 to 4.4e-15
+  kEights,  // eight entries, two pairs (BF16): 4.1 to 4.4e-15
 };
 
 // y += A x (fresh: y = A x).  The CTA's eight warps are 8 / S groups of R rows
@@ -454,11 +454,9 @@ __global__ void __launch_bounds__(NT, 4) k_dense_df(const V* __restrict__ A, int
       const DF t = two_sum(th[q][r], sh[r]);
       th[q][r] = t.h;
       tl[q][r] = __fadd_rn(tl[q][r], __fadd_rn(t.l, sc[r]));
-      if constexpr (!LONG || sizeof(V) != 8) {  // keeps tl small against th
-        const DF u = fast_two_sum(th[q][r], tl[q][r]);
-        th[q][r] = u.h;
-        tl[q][r] = u.l;
-      }
+      const DF u = fast_two_sum(th[q][r], tl[q][r]);  // keeps tl small against th
+      th[q][r] = u.h;
+      tl[q][r] = u.l;
       sh[r] = sc[r] = 0.f;
     }
   };
@@ -726,13 +724,13 @@ cudaError_t dense_df_shape(const V* a, int ln_row, int ln_col, const float* xs, 
 }
 
 // The sums by the columns (see Sums; us of 24,000 rows, against kLong): BF16
-// fours to 2304 columns (1104: 23.5, 19.9; 2048, 20,000 rows: 33.6, 28.2), eights to
-// 4608 (2312: 41.2, 40.7), FP32 fours to 1536 (1504: 36.2, 33.2), FP64, bound by HBM,
-// fours to 4608 (2312: 77.8, 76.6).
+// fours to 1792 columns (1104: 23.5, 19.9), eights to 4608 (1800: 34.6, 32.7;
+// 2312: 41.3, 40.9), FP32 fours to 1536 (1104: 28.4, 26.2; 1504: 36.2, 33.2), FP64
+// too (1104: 43.1, 42.9; 1504: 53.2, 52.8; HBM bounds it).
 template <class V, bool VEC>
 cudaError_t dense_df_sums(const V* a, int ln_row, int ln_col, const float* xs, const double* x, const int* bad, int nbad,
                           double* y, int fresh, cudaStream_t s) {
-  constexpr int fours = sizeof(V) == 4 ? 1536 : sizeof(V) == 2 ? 2304 : 4608;
+  constexpr int fours = sizeof(V) == 2 ? 1792 : 1536;
   if (ln_col <= fours) return dense_df_shape<V, VEC, kFours>(a, ln_row, ln_col, xs, x, bad, nbad, y, fresh, s);
   if constexpr (sizeof(V) == 2)
     if (ln_col <= 4608) return dense_df_shape<V, VEC, kEights>(a, ln_row, ln_col, xs, x, bad, nbad, y, fresh, s);
@@ -748,7 +746,7 @@ cudaError_t dense_df_vec(const void* vals, int ln_row, int ln_col, const float* 
   constexpr int NV = Step<V, true>::NV;
   if ((uintptr_t)vals % 16 == 0 && (uintptr_t)xs % 16 == 0 && ln_col % NV == 0)
     return dense_df_sums<V, true>(a, ln_row, ln_col, xs, x, bad, nbad, y, fresh, s);
-  if (ln_col <= 1100) return dense_df_shape<V, false, kPairs>(a, ln_row, ln_col, xs, x, bad, nbad, y, fresh, s);
+  if (ln_col <= (sizeof(V) == 8 ? 512 : 1100)) return dense_df_shape<V, false, kPairs>(a, ln_row, ln_col, xs, x, bad, nbad, y, fresh, s);
   return dense_df_sums<V, false>(a, ln_row, ln_col, xs, x, bad, nbad, y, fresh, s);
 }
 }  // namespace

@@ -62,7 +62,7 @@ def row_sums_256(a, x, fp64):
 
 
 @pytest.mark.parametrize("prec", ["f64", "f32", "bf16"])
-@pytest.mark.parametrize("nc", [200, 512, 513, 600, 1000, 1003, 1104, 1301, 1544, 2000, 2312, 4099, 4104])
+@pytest.mark.parametrize("nc", [200, 401, 512, 513, 600, 800, 1000, 1003, 1104, 1301, 1544, 1801, 2000, 2312, 4099, 4104])
 def test_error(gpu, nc, prec):
     T = gpu
     nr = min(4000, 5_000_000 // nc)
