@@ -322,6 +322,12 @@ int settled(DeviceMatrix* d, int st) {
   return st ? st : e;
 }
 
+// The same on every way out of a scope, exceptions included.
+struct Settle {
+  DeviceMatrix* d;
+  ~Settle() { cudaStreamSynchronize(d->stream); }
+};
+
 SellArgs sell_args(const tbsla_matrix* m, const DeviceMatrix* d) {
   SellArgs a;
   a.vals = d->vals;
@@ -380,9 +386,7 @@ int build_sell(const tbsla_matrix* m, DeviceMatrix* d, int n, int nc, int f_col,
   const int W = (int)(((long)nc + P - 1) / P);
   std::vector<int> lens((size_t)P * n, 0);
   if (P == 1) {
-    parallel_for(n, [&](long b, long e) {
-      for (long i = b; i < e; i++) lens[i] = rp[i + 1] - rp[i];
-    });
+    for (int i = 0; i < n; i++) lens[i] = rp[i + 1] - rp[i];
   } else {
     parallel_for(n, [&](long b, long e) {
       for (long i = b; i < e; i++)
@@ -433,7 +437,9 @@ int build_sell(const tbsla_matrix* m, DeviceMatrix* d, int n, int nc, int f_col,
       std::copy(L + r0, L + r1, part.begin() + r0);
       L = part.data();
     }
-    SellPlan hp;
+    struct HostPlan : SellPlan {
+      ~HostPlan() { sell_plan_free(this); }
+    } hp;
     sell_plan_build(L, n, sthr, lthr, piece, m->sell_sigma, blk > 0, steps, &hp);
     hp.col_lo = blk * W;
     hp.col_hi = blk == P - 1 ? INT_MAX : (blk + 1) * W;
@@ -457,7 +463,6 @@ int build_sell(const tbsla_matrix* m, DeviceMatrix* d, int n, int nc, int f_col,
       d->bytes += (size_t)hp.npieces * 8 + (size_t)hp.ncut * 28;
     }
     st = settled(d, st);  // host plan arrays are freed next
-    sell_plan_free(&hp);
     steps += dp.sell_len / 32;
   }
   d->sell_parts = R;
@@ -514,10 +519,7 @@ int build_coo_rows(const tbsla_matrix* m, DeviceMatrix* d, const std::vector<lon
   const int n = (int)ends.size();
   std::vector<int> rp((size_t)n + 1, 0);
   for (int i = 0; i < n; i++) rp[i + 1] = (int)ends[i];
-  struct Settle {  // rp, cols and vals outlive their copies on every way out
-    DeviceMatrix* d;
-    ~Settle() { cudaStreamSynchronize(d->stream); }
-  } settle{d};
+  const Settle settle{d};  // before rp, cols and vals go
   int st = upload_ints(d, &d->idx0, rp.data(), rp.size());
   if (!st) st = upload_ints(d, &d->idx1, cols.data(), cols.size());
   if (!st) st = upload_values(d, vals.data(), vals.size());
@@ -577,8 +579,9 @@ int build(const tbsla_matrix* m, DeviceMatrix* d) {
       d->items = tile <= 1024 ? 4 : tile <= 2048 ? 8 : 16;
       int* blocks = nullptr;
       csr_partition(rp, I.ln_row, 256 * d->items, d->algo == TBSLA_CSR_ROWBLOCK ? kCsrMaxSteps : 0, &blocks, &d->nblocks);
-      st = settled(d, upload_ints(d, &d->blocks, blocks, (size_t)d->nblocks + 1));
-      delete[] blocks;
+      const std::unique_ptr<int[]> keep(blocks);
+      const Settle settle{d};  // before the blocks go; the plans are made under the copies
+      st = upload_ints(d, &d->blocks, blocks, (size_t)d->nblocks + 1);
       if (st) return st;
       d->merge_items = m->merge_items;
       d->ntiles = merge_tiles(I.ln_row, enz, d->merge_items);

@@ -495,32 +495,28 @@ void sell_plan_build(const int* L, int n, int sthr, int lthr, int piece, int sig
     long first;  // index into wide_rows of its first row
     int piece;   // of a cut row (-1: whole rows)
   };
-  std::vector<int4> desc;
-  std::vector<int> meta, meta_len;
-  std::vector<std::pair<int, int>> order;  // (width, slice) of the wide slices
   std::vector<Slice> wide;
   std::vector<int> wide_rows;
   std::vector<int> piece_cut, piece_at, piece_len, cut_first;
-  auto by_len = [&](int a, int b) { return len(a) > len(b); };
-  // longest first, equal lengths in row order: counted where the lengths are
-  // close together (60,000 rows: 0.3 ms, compared 6 ms)
-  auto sort_wide = [&](std::vector<int>& v) {
+  // v by key, largest first, equal keys in v's order: counted where the keys
+  // are close together (60,000 rows by length: 0.3 ms, compared 6 ms)
+  auto sort_down = [](std::vector<int>& v, auto key) {
     int lo = INT_MAX, hi = 0;
-    for (int i : v) lo = std::min(lo, len(i)), hi = std::max(hi, len(i));
+    for (int i : v) lo = std::min(lo, key(i)), hi = std::max(hi, key(i));
     if (v.empty() || (size_t)(hi - lo) > 8 * v.size() + 65536) {
-      std::stable_sort(v.begin(), v.end(), by_len);
+      std::stable_sort(v.begin(), v.end(), [&](int a, int b) { return key(a) > key(b); });
       return;
     }
     std::vector<size_t> at((size_t)(hi - lo) + 2, 0);
-    for (int i : v) at[(size_t)(hi - len(i)) + 1]++;
+    for (int i : v) at[(size_t)(hi - key(i)) + 1]++;
     for (size_t k = 1; k < at.size(); k++) at[k] += at[k - 1];
     std::vector<int> out(v.size());
-    for (int i : v) out[at[(size_t)(hi - len(i))]++] = i;
+    for (int i : v) out[at[(size_t)(hi - key(i))]++] = i;
     v.swap(out);
   };
   for (int g = 0; g <= 5; g++) {
     auto& v = lng[g];
-    sort_wide(v);
+    sort_down(v, len);
     const int per = 32 >> g;
     // a row past 32 * piece entries: equal pieces, whole steps each
     size_t q0 = 0;
@@ -534,29 +530,18 @@ void sell_plan_build(const int* L, int n, int sthr, int lthr, int piece, int sig
         piece_at.push_back(at);
         piece_len.push_back(std::min(size, l - at));
         wide_rows.push_back(v[q0]);
-        order.push_back({s.width, (int)wide.size()});
         wide.push_back(s);
       }
     }
     for (size_t q = q0; q < v.size(); q += per) {
       Slice s{(len(v[q]) + (1 << g) - 1) >> g, g, (long)wide_rows.size(), -1};
       for (int r = 0; r < per; r++) wide_rows.push_back(q + r < v.size() ? v[q + r] : -1);
-      order.push_back({s.width, (int)wide.size()});
       wide.push_back(s);
     }
   }
-  std::stable_sort(order.begin(), order.end(), [](auto& a, auto& b) { return a.first > b.first; });
-  long off = step0;  // in steps of 32 entries
-  for (auto& o : order) {
-    const Slice& s = wide[o.second];
-    desc.push_back(make_int4((int)off, s.width, s.g, s.piece >= 0 ? -2 - s.piece : -1));
-    for (int l = 0; l < 32; l++) {
-      const int row = wide_rows[s.first + (l >> s.g)];
-      meta.push_back(row);
-      meta_len.push_back(s.piece >= 0 ? piece_len[s.piece] : row >= 0 ? len(row) : 0);
-    }
-    off += s.width;
-  }
+  std::vector<int> order(wide.size());  // the wide slices, widest first
+  std::iota(order.begin(), order.end(), 0);
+  sort_down(order, [&](int k) { return wide[k].width; });
   // Short rows: one lane each, sorted by length within windows.
   const int nwin = (n + sigma - 1) / sigma;
   std::vector<std::vector<int>> win(nwin);
@@ -566,15 +551,35 @@ void sell_plan_build(const int* L, int n, int sthr, int lthr, int piece, int sig
       auto& v = win[w];
       for (int i = r0; i < r1; i++)
         if (len(i) <= sthr && (len(i) > 0 || !skip_empty)) v.push_back(i);
-      std::stable_sort(v.begin(), v.end(), by_len);
+      sort_down(v, len);
     }
   });
   std::vector<long> first(nwin + 1, 0);
   for (int w = 0; w < nwin; w++) first[w + 1] = first[w] + (long)((win[w].size() + 31) / 32);
-  const long nwide = (long)desc.size();
-  const long nshort = first[nwin];
-  desc.resize(nwide + nshort);
-  meta.resize(32 * (nwide + nshort));
+  const long nwide = (long)wide.size(), nshort = first[nwin], nslices = nwide + nshort;
+  // the arrays, filled where they stay
+  p->slice = new int4[std::max<long>(nslices, 1)];
+  p->lane = new int[std::max<long>(32 * nslices, 1)];
+  p->lane_len = new int[std::max<long>(32 * nwide, 1)];
+  int4* const desc = p->slice;
+  int *const meta = p->lane, *const meta_len = p->lane_len;
+  long off = step0;  // in steps of 32 entries
+  for (long k = 0; k < nwide; k++) {
+    const Slice& s = wide[order[k]];
+    desc[k] = make_int4((int)off, s.width, s.g, s.piece >= 0 ? -2 - s.piece : -1);
+    off += s.width;
+  }
+  constexpr long kChunk = 1024;  // wide slices a thread takes at a time
+  parallel_for_items((nwide + kChunk - 1) / kChunk, [&](long b, long e) {
+    for (long k = b * kChunk; k < std::min(e * kChunk, nwide); k++) {
+      const Slice& s = wide[order[k]];
+      for (int l = 0; l < 32; l++) {
+        const int row = wide_rows[s.first + (l >> s.g)];
+        meta[32 * k + l] = row;
+        meta_len[32 * k + l] = s.piece >= 0 ? piece_len[s.piece] : row >= 0 ? len(row) : 0;
+      }
+    }
+  });
   parallel_for_items(nwin, [&](long b, long e) {
     for (long w = b; w < e; w++) {
       const auto& v = win[w];
@@ -594,19 +599,13 @@ void sell_plan_build(const int* L, int n, int sthr, int lthr, int piece, int sig
       }
     }
   });
-  for (long k = nwide; k < nwide + nshort; k++) {
+  for (long k = nwide; k < nslices; k++) {
     desc[k].x = (int)off;
     off += desc[k].y;
   }
   p->nwide = (int)nwide;
-  p->nslices = (int)(nwide + nshort);
+  p->nslices = (int)nslices;
   p->sell_len = (off - step0) * 32;
-  p->slice = new int4[std::max<size_t>(desc.size(), 1)];
-  std::copy(desc.begin(), desc.end(), p->slice);
-  p->lane = new int[std::max<size_t>(meta.size(), 1)];
-  std::copy(meta.begin(), meta.end(), p->lane);
-  p->lane_len = new int[std::max<size_t>(meta_len.size(), 1)];
-  std::copy(meta_len.begin(), meta_len.end(), p->lane_len);
   p->npieces = (int)piece_at.size();
   p->ncut = (int)cut_first.size();
   cut_first.push_back(p->npieces);
